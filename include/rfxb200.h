@@ -327,31 +327,29 @@ int rfxb_plan_box_flux(RfxbPlan* plan, const int* box, double* flux_dev, void* s
 int64_t rfxb_plan_device_bytes(const RfxbPlan* plan);
 
 /* Which forward step kernel the launches of a plan (or batch) use: 0 the
- * generic one (cp.async staging, CPML psi read from global memory), 1 TMA
- * staging without CPML, 2 TMA staging with the CPML psi staged by TMA one
- * plane ahead; -1 for a null handle.  A diagnostic of this implementation,
- * no counterpart in the reference. */
+ * generic one (cp.async staging, one cell per thread, CPML psi read from global
+ * memory), 1 TMA staging and four cells per thread without CPML, 2 the same
+ * with the CPML psi prefetched one plane ahead; -1 for a null handle.  A
+ * diagnostic of this implementation, no counterpart in the reference. */
 int rfxb_plan_forward_variant(const RfxbPlan* plan);
 int rfxb_batch_forward_variant(const RfxbBatch* batch);
 
 /* Which reverse step kernel the adjoint launches of a plan (or batch) use:
- * 0 cp.async staging, 1 TMA staging with CPML psi read from global memory,
- * 2 TMA staging with the adjoint psi and ce staged by TMA one plane ahead,
- * 3 TMA staging without any CPML (groups without CPML); with 1 or 2, tiles
- * whose reverse step touches no slab run on 3 beside it, and with 2 the
- * CPML work of tiles that reach no y slab runs on variant 4 (variant 2
- * without the y-slab terms, four CTAs per SM) on a third stream.  -1 before
- * the first adjoint advance or for a null handle.  A diagnostic of this
- * implementation, no counterpart in the reference. */
+ * 0 cp.async staging, one cell per thread, 2 TMA staging and four cells per
+ * thread with the adjoint psi and ce prefetched one plane ahead, 3 the same
+ * without any CPML (groups without CPML); with 2, items whose reverse step
+ * touches no slab run the CPML-free code.  -1 before the first adjoint advance
+ * or for a null handle.  A diagnostic of this implementation, no counterpart
+ * in the reference. */
 int rfxb_plan_adjoint_variant(const RfxbPlan* plan);
 int rfxb_batch_adjoint_variant(const RfxbBatch* batch);
 
 /* Step-kernel launches per forward time step (*fwd: 1, or 2 with the split
  * into CPML and plain tiles; with two-step passes, fwd_depth 2, the launches
  * of one pass of two steps: the two-step tiles plus two launches of each
- * one-step list) and per reverse time step (*rev: 1, 2 with the
- * split, 3 when variant 4 takes the CPML work without a y slab; -1 before
- * the first adjoint advance), not counting DFT / flux / NTFF epilogue
+ * one-step list) and per reverse time step (*rev: 1, 2 or 3 with
+ * the split into plain tiles, CPML tiles that reach a y slab and the other CPML
+ * tiles; -1 before the first adjoint advance), not counting DFT / flux / NTFF epilogue
  * kernels.  A diagnostic of this implementation. */
 int rfxb_plan_step_launches(const RfxbPlan* plan, int* fwd, int* rev);
 int rfxb_batch_step_launches(const RfxbBatch* batch, int* fwd, int* rev);
@@ -360,16 +358,16 @@ int rfxb_batch_step_launches(const RfxbBatch* batch, int* fwd, int* rev);
  * the autotuner (rfx_b200/autotune.py) searches.  Every setting computes the
  * same steps; they differ in how the tiles are split among kernel variants
  * and streams and in which launch a captured graph hands to the SMs first.
- *   fwd_split  1: forward tiles split, the CPML-free variant 1 beside the
- *                 staged-psi variant 2 on two streams; 0: one launch
+ *   fwd_split  0: one launch over all tiles, CPML-free items on the CPML-free
+ *                 code; 1: CPML-free and CPML tiles (8 x 32) in two launches on
+ *                 two streams
  *   fwd_order  with the split, 0: plain-tile launch first, 1: CPML-tile
  *                 launch first
- *   adj_lite   1: reverse CPML work of tiles that reach no y slab on
- *                 variant 4 (third stream); 0: on variant 2
- *   adj_order  order of the reverse launches, a permutation of (variant 4,
- *                 variant 2, variant 3) by index: 0 (4,2,3), 1 (4,3,2),
- *                 2 (2,4,3), 3 (2,3,4), 4 (3,4,2), 5 (3,2,4); without
- *                 variant 4 only the relative order of 2 and 3 counts
+ *   adj_lite   0: one reverse launch over all tiles; 1: three launches on three
+ *                 streams -- CPML tiles that reach no y slab (a), those that
+ *                 reach one (b), plain tiles (c)
+ *   adj_order  order of those launches: 0 (a,b,c), 1 (a,c,b), 2 (b,a,c),
+ *                 3 (b,c,a), 4 (c,a,b), 5 (c,b,a)
  *   fwd_persist  0: the launches above; k >= 1: one persistent launch per
  *                 step over both forward lists (as many CTAs as are resident,
  *                 each pulling items from device queues), k-1 CTAs per SM

@@ -1,5 +1,7 @@
-// Fused reverse step of the adjoint: the same tiling, x-march, staged plane
-// pipeline and halo recomputation as the forward step kernel.
+// Generic fused reverse step of the adjoint (per-thread copies): the tiling, x
+// march, staged plane pipeline and halo recomputation of the generic forward
+// kernel (rfxb_fwd.cu), used with RFXB_STAGING=cpasync and by plans whose psi
+// offsets pass 32 bits; every other plan's reverse step is in rfxb_adjv.cu.
 //
 // The transpose of one forward step (see rfxb_adj.cu for the derivation)
 // has the forward's dependency shape with the roles swapped:
@@ -13,26 +15,9 @@
 // PEC/edge mask.  Adjoint fields and psi are ping-ponged like the forward
 // state, so halo cells recomputed by a neighbour CTA read step-consistent
 // values.  The eps_r gradient over the recorded region is accumulated in
-// phase A from the forward history.
-//
-// The CPML terms of each relation are evaluated once per cell: the y / z
-// relations are exchanged between neighbouring cells through shared memory,
-// the x relations are carried along the march.  Modes (template MODE):
-//   0  cp.async staging (4 planes), psi and ce read from global memory;
-//   1  TMA staging (4 planes), psi and ce read from global memory;
-//   2  TMA staging (3 planes) plus a two-slot ring that brings, one plane
-//      ahead, every adjoint psi and ce value the plane's CPML terms read, so
-//      no slab cell waits on a global load.  The host selects it when no
-//      tile reaches both slabs of an axis;
-//   3  TMA staging (4 planes) with the CPML code compiled out, for the
-//      tiles and x ranges whose reverse step touches no slab (the host runs
-//      them beside variant 2 or 1 on a second stream);
-//   4  variant 2 for tiles that reach no y slab: the y relations and the
-//      edge-mask staging compiled out and the ring without its y-slab
-//      arrays (57 KB of shared memory; three CTAs per SM at 80 registers,
-//      measured faster than four at 64 with spills; a third stream).
-#include <algorithm>
-
+// phase A from the forward history.  The y / z CPML relations are evaluated
+// once per cell and exchanged through shared memory; the x relations are
+// carried along the march.
 #include "rfxb_common.cuh"
 
 namespace rfxb {
@@ -56,9 +41,7 @@ struct AdjDims {
   static constexpr unsigned BYTES = 4u * (NE + NB + NH + NC);
 };
 
-// One plane stage; EMS: with the tile's PEC edge-mask bits (staged only when
-// the plan has a mask; variant 4 has no room for them).
-template <int TY, bool EMS>
+template <int TY>
 struct __align__(128) AdjStage {
   float ae[3][TY + 2][RFXB_AEW];   // masked adjoint E, rows y0-1 .. y0+TY, z from z0-4
   float p0[AdjDims<TY>::P0];
@@ -67,69 +50,25 @@ struct __align__(128) AdjStage {
   float ah[3][TY + 1][RFXB_AHW];   // adjoint H, rows y0-1 .. y0+TY-1, z from z0-4
   float p2[AdjDims<TY>::P2];
   float ca[TY][RFXB_TZ];           // ca of the tile
-  unsigned char em[TY][RFXB_TZ];   // PEC edge-mask bits of the tile
-};
-template <int TY>
-struct __align__(128) AdjStage<TY, false> {
-  float ae[3][TY + 2][RFXB_AEW];
-  float p0[AdjDims<TY>::P0];
-  float cbp[TY + 2][RFXB_AEW];
-  float p1[AdjDims<TY>::P1];
-  float ah[3][TY + 1][RFXB_AHW];
-  float p2[AdjDims<TY>::P2];
-  float ca[TY][RFXB_TZ];
 };
 
-// The plane stages come last so that a kernel using fewer of them (modes 2
-// and 4) allocates only those, followed by its psi ring (modes 2, 4) or the
-// exchange array of the CPML terms (modes 0, 1): r_E / r_H of the y and z
-// relations (y q0, y q1, z q0, z q1) at rows y0-1 .. y0+TY, columns
-// z0-1 .. z0+32.
+// The exchange array of the CPML terms: r_E / r_H of the y and z relations
+// (y q0, y q1, z q0, z q1) at rows y0-1 .. y0+TY, columns z0-1 .. z0+32.
 template <int TY>
 using AdjExchange = float[4][TY + 2][RFXB_TZ + 2];
 
-template <int TY, bool EMS>
+template <int TY>
 struct AdjSmem {
   float p[3][TY + 1][RFXB_TZ + 1];   // ch * aH1 of plane i, [y - y0 + 1][z - z0 + 1]
   RfxbInst P;
   AdjInst A;
-  unsigned long long mbar[RFXB_ANSTAGE];
-  unsigned long long pbar[2];        // psi ring (modes 2, 4)
-  AdjStage<TY, EMS> st[RFXB_ANSTAGE];
+  AdjStage<TY> st[RFXB_ANSTAGE];
+  AdjExchange<TY> rx;
 };
 
 // Plane p lives in stage (p + 1) mod NST.
 template <int NST>
 __device__ __forceinline__ int astage_of(int p) { return (p + 1) % NST; }
-// Planes are loaded in order xa-1, xa, ...; a stage completes its k-th fill on
-// mbarrier phase k.
-template <int NST>
-__device__ __forceinline__ uint32_t astage_parity(int p, int xa) { return (uint32_t)(((p - xa + 1) / NST) & 1); }
-
-// One slot of the mode-2 psi ring: everything the CPML terms of plane p read
-// (floats, 128-byte aligned sub-arrays; zp = the launch's largest z-psi row):
-//   EY  [q][TY+2][40]  adjoint E-side psi of the y slab, rows y0-1.., z from z0-4
-//   HY  [q][TY+1][36]  adjoint H-side psi of the y slab, rows y0-1.., z from z0-4
-//   EXN [q][TY+1][36]  adjoint E-side psi of the x slab at plane p+1
-//   HX  [q][TY][32]    adjoint H-side psi of the x slab on the tile
-//   CE  [TY+2][40]     ce of plane p on the E footprint
-//   CEN [TY+1][36]     ce of plane p+1 on the H footprint
-//   EZ  [q][TY+2][n4]  adjoint E-side psi of the z slab, layer s
-//   HZ  [q][TY+1][n4]  adjoint H-side psi of the z slab
-// (YS false, variant 4: no EY / HY arrays.)
-template <int TY, bool YS>
-struct APsiSlot {
-  static constexpr int EY = 0;
-  static constexpr int HY = EY + (YS ? up32(2 * (TY + 2) * RFXB_AEW) : 0);
-  static constexpr int EXN = HY + (YS ? up32(2 * (TY + 1) * RFXB_AHW) : 0);
-  static constexpr int HX = EXN + up32(2 * (TY + 1) * RFXB_AHW);
-  static constexpr int CE = HX + up32(2 * TY * RFXB_TZ);
-  static constexpr int CEN = CE + up32((TY + 2) * RFXB_AEW);
-  static constexpr int EZ = CEN + up32((TY + 1) * RFXB_AHW);
-  __host__ __device__ static constexpr int HZ(int zp) { return EZ + up32(2 * (TY + 2) * zp); }
-  __host__ __device__ static constexpr int FLOATS(int zp) { return HZ(zp) + up32(2 * (TY + 1) * zp); }
-};
-
 struct AdjCtx {
   int nx, ny, nz, zs, ncp, par, apar;
   long long ps, off0, cs;
@@ -290,105 +229,15 @@ __device__ __forceinline__ void adj_load_stage(SM& S, const AdjCtx& C, const flo
   }
 }
 
-// TMA boxes of plane ip (one thread): adjoint E and H of parity apar, cb with
-// the E footprint, ca of the tile.
-template <int TY, int NST, bool EMS>
-__device__ __forceinline__ void adj_tma_stage(AdjSmem<TY, EMS>& S, const CUtensorMap* tm, int apar, int y0, int z0,
-                                              int ip) {
-  const int s = astage_of<NST>(ip);
-  const uint32_t mb = smem_u32(&S.mbar[s]);
-  const bool em = EMS && S.P.emask != nullptr;
-  mbar_expect_tx(mb, AdjDims<TY>::BYTES + (em ? (unsigned)(TY * RFXB_TZ) : 0u));
-  if constexpr (EMS) {
-    if (em) tma_load_4d(smem_u32(&S.st[s].em[0][0]), tm + RFXB_MAP_EMASK, z0, y0 + 1, ip + 1, 0, mb);
-  }
-  tma_load_4d(smem_u32(&S.st[s].ae[0][0][0]), tm + 5 + apar, z0 - 4, y0, ip + 1, 0, mb);
-  tma_load_4d(smem_u32(&S.st[s].cbp[0][0]), tm + 9, z0 - 4, y0, ip + 1, 1, mb);
-  tma_load_4d(smem_u32(&S.st[s].ah[0][0][0]), tm + 7 + apar, z0 - 4, y0, ip + 1, 3, mb);
-  tma_load_4d(smem_u32(&S.st[s].ca[0][0]), tm + 10, z0, y0 + 1, ip + 1, 0, mb);
-}
-
-// r_E / r_H of one relation from a given old psi (modes 2, 4: staged); the new
-// psi goes to the other parity at index qi.
-__device__ __forceinline__ float re_core(const AdjInst& A, const AdjCtx& C, int axis, const float4& cf, long long qi,
-                                         float psi, float sgn, float ce, float at, bool write) {
-  const float nu = psi + sgn * ce * at;
-  if (write) A.aPsiE[C.par ^ 1][axis][qi] = cf.x * nu;
-  return cf.y * nu + sgn * ce * (cf.z * at);
-}
-__device__ __forceinline__ float rh_core(const AdjInst& A, const AdjCtx& C, int axis, const float4& cf, long long qi,
-                                         float psi, float sgn, float pt, bool write) {
-  const float nu = psi + sgn * pt;
-  if (write) A.aPsiH[C.par ^ 1][axis][qi] = cf.x * nu;
-  return cf.y * nu + sgn * (cf.z * pt);
-}
-
-// Which CPML slab of an axis the cells lo..hi of a CTA reach: side or -1
-// (modes 2 and 4 guarantee at most one side per axis).
-__device__ __forceinline__ int atile_side(int lo, int hi, int n, int ncp) {
-  if (lo < ncp) return 0;
-  if (hi >= n - ncp) return 1;
-  return -1;
-}
-
-// Issue the mode-2 ring boxes of plane p (one thread).
-template <int TY, bool YS>
-__device__ __forceinline__ void apsi_issue(float* slot, uint32_t mb, const CUtensorMap* tm, const AdjCtx& C, int zp4,
-                                           int y0, int z0, int p, bool yz_tile, int ysd, int zsd, int n4) {
-  using L = APsiSlot<TY, YS>;
-  const int par = C.par;
-  int sx = 0, sn = 0;
-  const int xsd = C.cpx ? cpml_side(p, C.nx, C.ncp, sx) : -1;
-  const int xnd = (C.cpx && p + 1 < C.nx) ? cpml_side(p + 1, C.nx, C.ncp, sn) : -1;
-  unsigned bytes = 0;
-  if (yz_tile) bytes += 4u * (TY + 2) * RFXB_AEW;
-  if (ysd >= 0) bytes += 4u * 2 * (TY + 2) * RFXB_AEW + 4u * 2 * (TY + 1) * RFXB_AHW;
-  if (zsd >= 0) bytes += 4u * 2 * (TY + 2) * n4 + 4u * 2 * (TY + 1) * n4;
-  if (xnd >= 0) bytes += 4u * 2 * (TY + 1) * RFXB_AHW + 4u * (TY + 1) * RFXB_AHW;
-  if (xsd >= 0) bytes += 4u * 2 * TY * RFXB_TZ;
-  mbar_expect_tx(mb, bytes);
-  if (yz_tile) tma_load_4d(smem_u32(slot + L::CE), tm + 9, z0 - 4, y0, p + 1, 2, mb);
-  if (ysd >= 0) {
-    const int jb = ysd ? C.ny - C.ncp : 0;
-    tma_load_4d(smem_u32(slot + L::EY), tm + RFXB_MAP_APE + 2 + par, z0 - 4, y0 - 1 - jb, p, 2 * ysd, mb);
-    tma_load_4d(smem_u32(slot + L::HY), tm + RFXB_MAP_APH + 2 + par, z0 - 4, y0 - 1 - jb, p, 2 * ysd, mb);
-  }
-  if (zsd >= 0) {
-    tma_load_4d(smem_u32(slot + L::EZ), tm + RFXB_MAP_APE + 4 + par, 0, y0 - 1, p, 2 * zsd, mb);
-    tma_load_4d(smem_u32(slot + L::HZ(zp4)), tm + RFXB_MAP_APH + 4 + par, 0, y0 - 1, p, 2 * zsd, mb);
-  }
-  if (xnd >= 0) {
-    tma_load_4d(smem_u32(slot + L::EXN), tm + RFXB_MAP_APE + 0 + par, z0 - 4, y0 - 1, sn, 2 * xnd, mb);
-    tma_load_4d(smem_u32(slot + L::CEN), tm + 23, z0 - 4, y0, p + 2, 2, mb);
-  }
-  if (xsd >= 0) tma_load_4d(smem_u32(slot + L::HX), tm + RFXB_MAP_APH + 0 + par, z0, y0, sx, 2 * xsd, mb);
-}
-
-template <int MODE>
-struct AdjBounds { static constexpr int MIN_CTAS = 4; };
-template <>
-struct AdjBounds<2> { static constexpr int MIN_CTAS = 3; };
-template <>
-struct AdjBounds<4> { static constexpr int MIN_CTAS = 3; };   // 80 registers, no spills (measured 0.6 % faster than 4)
-
-// One work item of the reverse step (see the forward's fwd_item): returns
-// false when a bounded wait ran out (status set, every issued box waited
-// for); the caller must then leave.  The shared memory at `raw` holds the
-// layout of this mode; the mbarriers sit at the same offsets in every mode.
-template <int TY, int MODE>
-__device__ __forceinline__ bool adj_item(unsigned char* raw, const RfxbInst* __restrict__ insts,
-                                         const AdjInst* __restrict__ adjs, const RfxbWork w,
-                                         const CUtensorMap* __restrict__ maps, int n, int par, int apar, int zp,
-                                         StepPhases& ph, const StepFault& fault, bool first_item) {
-  constexpr bool TMA = MODE != 0;
-  constexpr bool RING = MODE == 2 || MODE == 4;       // psi ring
-  constexpr bool YS = MODE != 4;                      // y-slab relations compiled in
-  constexpr int NST = RING ? 3 : RFXB_ANSTAGE;        // plane stages
-  using L = APsiSlot<TY, YS>;
-  using SM = AdjSmem<TY, MODE != 4>;
-  SM& S = *reinterpret_cast<SM*>(raw);
-  float* ring = reinterpret_cast<float*>(&S.st[NST]);   // modes 2, 4: two psi slots after the stages
-  auto& rx = *reinterpret_cast<AdjExchange<TY>*>(&S.st[NST]);   // modes 0, 1: the exchange array
+// One launch per reverse step: CTA b runs work item b.
+__global__ void __launch_bounds__(256, 4)
+adj_step_kernel(const RfxbInst* __restrict__ insts, const AdjInst* __restrict__ adjs, const RfxbWork* __restrict__ work,
+                int n, int par, int apar) {
+  constexpr int TY = 8, NST = RFXB_ANSTAGE;
+  extern __shared__ __align__(128) unsigned char adj_smem_raw[];
+  auto& S = *reinterpret_cast<AdjSmem<TY>*>(adj_smem_raw);
+  auto& rx = S.rx;
+  const RfxbWork w = work[blockIdx.x];
   const int lane = threadIdx.x, ty = threadIdx.y;
   const int tid = ty * 32 + lane;
   load_inst(S.P, insts + w.inst, tid, 32 * TY);
@@ -399,12 +248,6 @@ __device__ __forceinline__ bool adj_item(unsigned char* raw, const RfxbInst* __r
     for (int t = tid; t < nw; t += 32 * TY) d[t] = __ldg(s + t);
   }
   __syncthreads();
-  const int wlim = fault.wait_limit;
-  // the thread that issues the TMA boxes: lane 0 of the last warp (warps 0
-  // and 1 compute the halo row and column of phase A)
-  const int producer = 32 * (TY - 1);
-  const bool skip_first = first_item && (int)blockIdx.x == fault.cta;
-  const CUtensorMap* tm = maps + (size_t)w.inst * RFXB_NMAPS;
   const RfxbInst& P = S.P;
   const AdjInst& A = S.A;
   AdjCtx C;
@@ -414,9 +257,9 @@ __device__ __forceinline__ bool adj_item(unsigned char* raw, const RfxbInst* __r
   C.ch0 = P.ch0;
   const int y0 = w.y0, z0 = w.z0;
   // the +1 neighbours of the tile (row y0+TY, column z0+32) also read CPML terms
-  C.cpx = MODE != 3 && C.ncp > 0 && (P.cpml_axes & 1u);
-  C.cpy = MODE != 3 && YS && C.ncp > 0 && (P.cpml_axes & 2u) && (y0 - 1 < C.ncp || y0 + TY >= C.ny - C.ncp);
-  C.cpz = MODE != 3 && C.ncp > 0 && (P.cpml_axes & 4u) && (z0 - 1 < C.ncp || z0 + 32 >= C.nz - C.ncp);
+  C.cpx = C.ncp > 0 && (P.cpml_axes & 1u);
+  C.cpy = C.ncp > 0 && (P.cpml_axes & 2u) && (y0 - 1 < C.ncp || y0 + TY >= C.ny - C.ncp);
+  C.cpz = C.ncp > 0 && (P.cpml_axes & 4u) && (z0 - 1 < C.ncp || z0 + 32 >= C.nz - C.ncp);
   const float* aF0 = A.aF[apar][0];
   float* aFo = A.aF[apar ^ 1][0];
   const int j = y0 + ty, k = z0 + lane;
@@ -453,70 +296,16 @@ __device__ __forceinline__ bool adj_item(unsigned char* raw, const RfxbInst* __r
   const int xa = w.xa, xb = w.xb;
   const float* ca = P.ca;
   const float* cb = P.cb;
-  // mode-2 psi ring: the slab side this tile reaches per axis, and the
-  // bookkeeping of the two slots (identical in every thread)
   const bool yz_tile = C.cpy || C.cpz;
-  const int ysd = (RING && C.cpy) ? atile_side(y0 - 1, y0 + TY, C.ny, C.ncp) : -1;
-  const int zsd = (RING && C.cpz) ? atile_side(z0 - 1, z0 + 32, C.nz, C.ncp) : -1;
-  const int n4 = P.ncp4;
-  auto xslab = [&](int p) { return C.cpx && p >= 0 && p < C.nx && (p < C.ncp || p >= C.nx - C.ncp); };
-  auto psi_need = [&](int p) {
-    if (!RING || p < 0 || p >= C.nx) return false;
-    return yz_tile || xslab(p) || xslab(p + 1);
-  };
-  unsigned& pph = ph.ring;
-  unsigned pout = 0u;
-  // completion parity of the stage holding plane p (the k-th fill of a stage
-  // in this item is k phases past where the previous items left it)
-  auto sparity = [&](int p) -> uint32_t {
-    return ((ph.stage >> astage_of<NST>(p)) ^ (uint32_t)((p - xa + 1) / NST)) & 1u;
-  };
-  auto psi_fill = [&](int p) {
-    if (!psi_need(p)) return;
-    if (tid == producer)
-      apsi_issue<TY, YS>(ring + (p & 1) * L::FLOATS(zp), smem_u32(&S.pbar[p & 1]), tm, C, zp, y0, z0, p, yz_tile, ysd,
-                     zsd, n4);
-    pout |= 1u << (p & 1);
-  };
-  auto psi_wait = [&](int p) -> bool {
-    if (!psi_need(p)) return true;
-    const int sl = p & 1;
-    const bool ok = mbar_wait_bounded(smem_u32(&S.pbar[sl]), (pph >> sl) & 1u, wlim);
-    if (ok) {
-      pph ^= 1u << sl;
-      pout &= ~(1u << sl);
-    }
-    return ok;
-  };
-  auto bail = [&](int last_issued, int from) {
-    if (tid == 0) {
-      atomicOr(P.status, 1);
-      for (int p = from; p <= last_issued; ++p)
-        mbar_wait_bounded(smem_u32(&S.mbar[astage_of<NST>(p)]), sparity(p), wlim);
-      for (int sl = 0; sl < 2; ++sl)
-        if (pout & (1u << sl)) mbar_wait_bounded(smem_u32(&S.pbar[sl]), (pph >> sl) & 1u, wlim);
-    }
-  };
-  if (TMA) {
-    if (tid == producer)
-      for (int p = xa - 1; p <= min(xa + NST - 2, xb); ++p)
-        if (!(skip_first && p == xa)) adj_tma_stage<TY, NST>(S, tm, apar, y0, z0, p);
-    psi_fill(xa);
-    const bool ok = mbar_wait_bounded(smem_u32(&S.mbar[astage_of<NST>(xa - 1)]), sparity(xa - 1), wlim) &&
-                    mbar_wait_bounded(smem_u32(&S.mbar[astage_of<NST>(xa)]), sparity(xa), wlim);
-    if (__syncthreads_or(!ok)) { bail(min(xa + NST - 2, xb), xa - 1); return false; }
-  } else {
-    adj_load_stage<TY>(S, C, aF0, ca, cb, y0, z0, xa - 1, tid);
-    adj_load_stage<TY>(S, C, aF0, ca, cb, y0, z0, xa, tid);
-    cp_async_commit();
-    adj_load_stage<TY>(S, C, aF0, ca, cb, y0, z0, xa + 1, tid);
-    cp_async_commit();
-    if (xa + 2 <= xb) adj_load_stage<TY>(S, C, aF0, ca, cb, y0, z0, xa + 2, tid);
-    cp_async_commit();
-    cp_async_wait<2>();
-    __syncthreads();
-  }
-
+  adj_load_stage<TY>(S, C, aF0, ca, cb, y0, z0, xa - 1, tid);
+  adj_load_stage<TY>(S, C, aF0, ca, cb, y0, z0, xa, tid);
+  cp_async_commit();
+  adj_load_stage<TY>(S, C, aF0, ca, cb, y0, z0, xa + 1, tid);
+  cp_async_commit();
+  if (xa + 2 <= xb) adj_load_stage<TY>(S, C, aF0, ca, cb, y0, z0, xa + 2, tid);
+  cp_async_commit();
+  cp_async_wait<2>();
+  __syncthreads();
   // phase A of plane xa-1 at this column: p and r_H there (not stored)
   float py_prev = 0.f, pz_prev = 0.f, rhy_prev = 0.f, rhz_prev = 0.f;
   if (xa > 0 && own) {
@@ -584,108 +373,16 @@ __device__ __forceinline__ bool adj_item(unsigned char* raw, const RfxbInst* __r
       xe1_n = __ldg(xe_tab + i + 2);
       xh0_n = __ldg(xh_tab + i + 1);
     }
-    if (TMA) {
-      // plane i+1 (and plane i's psi) have landed; after the barrier plane
-      // i-1's stage takes plane i+NST-1 and its psi slot plane i+1
-      const bool ok = mbar_wait_bounded(smem_u32(&S.mbar[astage_of<NST>(i + 1)]), sparity(i + 1), wlim) && psi_wait(i);
-      if (__syncthreads_or(!ok)) { bail(min(i + NST - 2, xb), i + 1); return false; }
-      if (tid == producer && i + NST - 1 <= xb) adj_tma_stage<TY, NST>(S, tm, apar, y0, z0, i + NST - 1);
-      if (i + 1 < xb) psi_fill(i + 1);
-    } else {
-      cp_async_wait<1>();
-      __syncthreads();
-      if (i + 3 <= xb) adj_load_stage<TY>(S, C, aF0, ca, cb, y0, z0, i + 3, tid);
-      cp_async_commit();
-    }
+    cp_async_wait<1>();
+    __syncthreads();
+    if (i + 3 <= xb) adj_load_stage<TY>(S, C, aF0, ca, cb, y0, z0, i + 3, tid);
+    cp_async_commit();
     const int b0 = astage_of<NST>(i), b1 = astage_of<NST>(i + 1);
-    const float* PS = ring + (i & 1) * L::FLOATS(zp);
-    // Mode 2: r_E / r_H of the y (axes bit 1) and z (bit 2) relations at
-    // footprint position (r, c) = (jj - y0 + 1, kk - z0 + 1), evaluated from
-    // the staged plane and the psi ring; .x .y: y relations q0 q1, .z .w: z
-    // relations q0 q1; zero outside the grid and the slabs.  Each cell reads
-    // its neighbours' relations this way, so no exchange barrier is needed.
-    auto re_at = [&](int r, int c, int axes, bool write) -> float4 {
-      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      const int jj = y0 - 1 + r, kk = z0 - 1 + c;
-      if (jj < 0 || jj >= C.ny || kk < 0 || kk >= C.nz) return v;
-      int sy = 0, sz = 0;
-      const int dy = ((axes & 1) && C.cpy) ? cpml_side(jj, C.ny, C.ncp, sy) : -1;
-      const int dz = ((axes & 2) && C.cpz) ? cpml_side(kk, C.nz, C.ncp, sz) : -1;
-      if (dy < 0 && dz < 0) return v;
-      const auto& X = S.st[b0];
-      const float ce = PS[L::CE + r * RFXB_AEW + c + 3];
-      const float ax = X.ae[0][r][c + 3];
-      if (dy >= 0) {
-        const float4 cf = __ldg(P.cpt + (2 + dy) * C.ncp + sy);
-        const int o = r * RFXB_AEW + c + 3;
-        v.x = re_core(A, C, 1, cf, write ? psi_q(P, 1, dy, 0, sy, i, jj, kk) : 0, PS[L::EY + o], +1.f, ce, ax,
-                      write);                                                           // ex <- hz
-        v.y = re_core(A, C, 1, cf, write ? psi_q(P, 1, dy, 1, sy, i, jj, kk) : 0,
-                      PS[L::EY + (TY + 2) * RFXB_AEW + o], -1.f, ce, X.ae[2][r][c + 3], write);   // ez <- hx
-      }
-      if (dz >= 0) {
-        const float4 cf = __ldg(P.cpt + (4 + dz) * C.ncp + sz);
-        const int o = r * n4 + sz;
-        v.z = re_core(A, C, 2, cf, write ? psi_q(P, 2, dz, 0, sz, i, jj, kk) : 0, PS[L::EZ + o], -1.f, ce, ax,
-                      write);                                                           // ex <- hy
-        v.w = re_core(A, C, 2, cf, write ? psi_q(P, 2, dz, 1, sz, i, jj, kk) : 0, PS[L::EZ + (TY + 2) * n4 + o],
-                      +1.f, ce, X.ae[1][r][c + 3], write);                              // ey <- hx
-      }
-      return v;
-    };
-    auto rh_at = [&](int r, int c, int axes, bool write) -> float4 {
-      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      const int jj = y0 - 1 + r, kk = z0 - 1 + c;
-      if (jj < 0 || jj >= C.ny || kk < 0 || kk >= C.nz) return v;
-      int sy = 0, sz = 0;
-      const int dy = ((axes & 1) && C.cpy) ? cpml_side(jj, C.ny, C.ncp, sy) : -1;
-      const int dz = ((axes & 2) && C.cpz) ? cpml_side(kk, C.nz, C.ncp, sz) : -1;
-      if (dy < 0 && dz < 0) return v;
-      const float p0 = S.p[0][r][c];
-      if (dy >= 0) {
-        const float4 cf = __ldg(P.cpt + (2 + dy) * C.ncp + sy);
-        const int o = r * RFXB_AHW + c + 3;
-        v.x = rh_core(A, C, 1, cf, write ? psi_q(P, 1, dy, 0, sy, i, jj, kk) : 0, PS[L::HY + o], -1.f, p0,
-                      write);                                                           // hx <- ez
-        v.y = rh_core(A, C, 1, cf, write ? psi_q(P, 1, dy, 1, sy, i, jj, kk) : 0,
-                      PS[L::HY + (TY + 1) * RFXB_AHW + o], +1.f, S.p[2][r][c], write);  // hz <- ex
-      }
-      if (dz >= 0) {
-        const float4 cf = __ldg(P.cpt + (4 + dz) * C.ncp + sz);
-        const int hz = L::HZ(zp), o = r * n4 + sz;
-        v.z = rh_core(A, C, 2, cf, write ? psi_q(P, 2, dz, 0, sz, i, jj, kk) : 0, PS[hz + o], +1.f, p0,
-                      write);                                                           // hx <- ey
-        v.w = rh_core(A, C, 2, cf, write ? psi_q(P, 2, dz, 1, sz, i, jj, kk) : 0, PS[hz + (TY + 1) * n4 + o],
-                      -1.f, S.p[1][r][c], write);                                       // hy <- ex
-      }
-      return v;
-    };
     const long long e = cell_index(C, i, j, k);
 
     // x relations of plane i+1 (written by this CTA when it owns that plane)
     float nx0 = 0.f, nx1 = 0.f, nxh = 0.f;
-    if (RING && xslab(i + 1)) {   // psi and ce of plane i+1 from the ring
-      const auto& Y1 = S.st[b1];
-      const bool wr = i + 1 < xb;
-      int sx;
-      const int sd = cpml_side(i + 1, C.nx, C.ncp, sx);
-      const float4 cf = __ldg(P.cpt + sd * C.ncp + sx);
-      constexpr int RQ = (TY + 1) * RFXB_AHW;
-      auto xnext = [&](int r, int zc, int jj, int kk, float at0, float at1, bool write, float& v0, float& v1) {
-        const float ce = PS[L::CEN + r * RFXB_AHW + zc];
-        v0 = re_core(A, C, 0, cf, psi_q(P, 0, sd, 0, sx, i + 1, jj, kk), PS[L::EXN + r * RFXB_AHW + zc], -1.f, ce,
-                     at0, write);
-        v1 = re_core(A, C, 0, cf, psi_q(P, 0, sd, 1, sx, i + 1, jj, kk), PS[L::EXN + RQ + r * RFXB_AHW + zc], +1.f,
-                     ce, at1, write);
-      };
-      if (own) xnext(ly, lz, j, k, Y1.ae[1][ly][lz], Y1.ae[2][ly][lz], wr, nx0, nx1);
-      float d0 = 0.f, d1 = 0.f;
-      if (row_halo) { xnext(0, lz, y0 - 1, k, Y1.ae[1][0][lz], 0.f, false, d0, d1); nxh = d0; }
-      if (col_halo) {
-        xnext(lane + 1, 3, y0 + lane, z0 - 1, 0.f, Y1.ae[2][lane + 1][3], false, d0, d1);
-        nxh = d1;
-      }
-    } else if (!RING && C.cpx && i + 1 < C.nx) {
+    if (C.cpx && i + 1 < C.nx) {
       const auto& Y1 = S.st[b1];
       const bool wr = i + 1 < xb;
       if (own) {
@@ -701,10 +398,10 @@ __device__ __forceinline__ bool adj_item(unsigned char* raw, const RfxbInst* __r
                       P.ce[cell_index(C, i + 1, y0 + lane, z0 - 1)], false);
     }
 
-    // Modes 0 / 1: r_E of the y / z relations at the tile, its +1 row /
+    // r_E of the y / z relations at the tile, its +1 row /
     // column and the halo cells, once per cell into the exchange array (own
     // cells write their psi)
-    if (!RING && yz_tile) {
+    if (yz_tile) {
       const auto& X = S.st[b0];
       auto re_fill = [&](int r, int c, bool write) {
         const int jj = y0 - 1 + r, kk = z0 - 1 + c;
@@ -742,26 +439,11 @@ __device__ __forceinline__ bool adj_item(unsigned char* raw, const RfxbInst* __r
 
     // ---- phase A ----
     float ahx = 0.f, ahy = 0.f, ahz = 0.f;
-    float4 rown = make_float4(0.f, 0.f, 0.f, 0.f);   // mode 2: this cell's y / z r_E
     if (own) {
       adj_a_cell<TY, 7, false>(P, A, S, C, b0, b1, i, j, k, ly, lz, xe0, xe1, ye0, ye1, ze0, ze1, true, ahx, ahy,
                                ahz);
       if (C.cpx) { ahz += rx0 - nx0; ahy += rx1 - nx1; }
-      if (RING) {
-        if (yz_tile) {
-          rown = re_at(ly, lh, 3, true);
-          if (C.cpy) {
-            const float4 ry = re_at(ly + 1, lh, 1, false);
-            ahz += rown.x - ry.x;
-            ahx += rown.y - ry.y;
-          }
-          if (C.cpz) {
-            const float4 rz = re_at(ly, lh + 1, 2, false);
-            ahy += rown.z - rz.z;
-            ahx += rown.w - rz.w;
-          }
-        }
-      } else {
+      {
         if (C.cpy) {
           ahz += rx[0][ly][lh] - rx[0][ly + 1][lh];
           ahx += rx[1][ly][lh] - rx[1][ly + 1][lh];
@@ -816,14 +498,7 @@ __device__ __forceinline__ bool adj_item(unsigned char* raw, const RfxbInst* __r
         adj_a_cell<TY, 5, false>(P, A, S, C, b0, b1, i, y0 - 1, k, 0, lz, xe0, xe1, ye0_r, ye1_r, ze0_r, ze1_r,
                                  false, a1, a2, a3);
         if (C.cpx) a3 += rxh - nxh;
-        if (RING) {   // row y0 is this thread's own row: its r_E is rown
-          if (C.cpy) {
-            const float4 r0 = re_at(0, lh, 1, false);
-            a3 += r0.x - rown.x;
-            a1 += r0.y - rown.y;
-          }
-          if (C.cpz) a1 += re_at(0, lh, 2, false).w - re_at(0, lh + 1, 2, false).w;
-        } else {
+        {
           if (C.cpy) {
             a3 += rx[0][0][lh] - rx[0][1][lh];
             a1 += rx[1][0][lh] - rx[1][1][lh];
@@ -852,14 +527,7 @@ __device__ __forceinline__ bool adj_item(unsigned char* raw, const RfxbInst* __r
                                  ze0_c, ze1_c, false, a1, a2, a3);
         const int r = lane + 1;
         if (C.cpx) a2 += rxh - nxh;
-        if (RING) {
-          if (C.cpy) a1 += re_at(r, 0, 1, false).y - re_at(r + 1, 0, 1, false).y;
-          if (C.cpz) {
-            const float4 z0v = re_at(r, 0, 2, false), z1v = re_at(r, 1, 2, false);
-            a2 += z0v.z - z1v.z;
-            a1 += z0v.w - z1v.w;
-          }
-        } else {
+        {
           if (C.cpy) a1 += rx[1][r][0] - rx[1][r + 1][0];
           if (C.cpz) {
             a2 += rx[2][r][0] - rx[2][r][1];
@@ -882,10 +550,10 @@ __device__ __forceinline__ bool adj_item(unsigned char* raw, const RfxbInst* __r
     }
     __syncthreads();
 
-    // Modes 0 / 1: r_H of the y / z relations at the tile and the low halo
+    // r_H of the y / z relations at the tile and the low halo
     // row / column (rows y0-1 .. y0+TY-1, columns z0-1 .. z0+31), once per
     // cell into the exchange array
-    if (!RING && yz_tile) {
+    if (yz_tile) {
       auto rh_fill = [&](int r, int c, bool write, bool ny_, bool nz_) {
         const int jj = y0 - 1 + r, kk = z0 - 1 + c;
         float v0 = 0.f, v1 = 0.f, v2 = 0.f, v3 = 0.f;
@@ -926,37 +594,14 @@ __device__ __forceinline__ bool adj_item(unsigned char* raw, const RfxbInst* __r
       float ay = cav * X.ae[1][ly][lz] + ((xh0 * pz - xhm * pz_prev) - (zh0 * px - zhm * px_zm));
       float az = cav * X.ae[2][ly][lz] + ((yh0 * px - yhm * px_ym) - (xh0 * py - xhm * py_prev));
       if (C.cpx) {   // (hy <- ez, +1, q0), (hz <- ey, -1, q1): aE(x) += r(x-1) - r(x)
-        if (RING) {
-          if (xslab(i)) {
-            int sx;
-            const int sd = cpml_side(i, C.nx, C.ncp, sx);
-            const float4 cf = __ldg(P.cpt + sd * C.ncp + sx);
-            const int o = ty * RFXB_TZ + lane;
-            rhy = rh_core(A, C, 0, cf, psi_q(P, 0, sd, 0, sx, i, j, k), PS[L::HX + o], +1.f, py, true);
-            rhz = rh_core(A, C, 0, cf, psi_q(P, 0, sd, 1, sx, i, j, k), PS[L::HX + TY * RFXB_TZ + o], -1.f, pz, true);
-          }
-        } else {
+        {
           rhy = rh_eval(P, A, C, 0, 0, +1.f, i, j, k, py, true);
           rhz = rh_eval(P, A, C, 0, 1, -1.f, i, j, k, pz, true);
         }
         az += rhy_prev - rhy;
         ay += rhz_prev - rhz;
       }
-      if (RING) {
-        if (yz_tile) {
-          const float4 rh = rh_at(ly, lh, 3, true);
-          if (C.cpy) {   // (hx <- ez, -1, q0), (hz <- ex, +1, q1)
-            const float4 ry = rh_at(ly - 1, lh, 1, false);
-            az += ry.x - rh.x;
-            ax += ry.y - rh.y;
-          }
-          if (C.cpz) {   // (hx <- ey, +1, q0), (hy <- ex, -1, q1)
-            const float4 rz = rh_at(ly, lh - 1, 2, false);
-            ay += rz.z - rh.z;
-            ax += rz.w - rh.w;
-          }
-        }
-      } else {
+      {
         if (C.cpy) {   // (hx <- ez, -1, q0), (hz <- ex, +1, q1)
           az += rx[0][ly - 1][lh] - rx[0][ly][lh];
           ax += rx[1][ly - 1][lh] - rx[1][ly][lh];
@@ -1004,9 +649,7 @@ __device__ __forceinline__ bool adj_item(unsigned char* raw, const RfxbInst* __r
       if (pec_k0) { ax = 0.f; ay = 0.f; }
       if (pec_kz) az = 0.f;
       if (P.emask) {
-        unsigned m;
-        if constexpr (MODE == 4) m = (unsigned)P.emask[e];   // not staged on this variant
-        else m = TMA ? (unsigned)X.em[ty][lane] : (unsigned)P.emask[e];
+        const unsigned m = (unsigned)P.emask[e];
         if (m & 1u) ax = 0.f;
         if (m & 2u) ay = 0.f;
         if (m & 4u) az = 0.f;
@@ -1023,138 +666,9 @@ __device__ __forceinline__ bool adj_item(unsigned char* raw, const RfxbInst* __r
     rx1 = nx1;
     rxh = nxh;
   }
-  if (!TMA) cp_async_wait<0>();
-  if (TMA) {   // the phases this item advanced: stage s filled by planes xa-1 .. xb
-    const int T = xb - xa + 2;
-    for (int st = 0; st < NST; ++st) {
-      const int fills = T / NST + ((((st - xa) % NST + NST) % NST) < T % NST ? 1 : 0);
-      ph.stage ^= (uint32_t)(fills & 1) << st;
-    }
-  }
-  __syncthreads();   // every thread is done with the stages, P and A before the next item reuses them
-  return true;
+  cp_async_wait<0>();
 }
 
-template <int TY>
-__device__ __forceinline__ void adj_init_barriers(unsigned char* raw, int nst, bool ring, int tid) {
-  auto& S = *reinterpret_cast<AdjSmem<TY, true>*>(raw);
-  if (tid == 0) {
-    for (int q = 0; q < nst; ++q) mbar_init(smem_u32(&S.mbar[q]), 1);
-    if (ring) { mbar_init(smem_u32(&S.pbar[0]), 1); mbar_init(smem_u32(&S.pbar[1]), 1); }
-    mbar_fence_init();
-  }
-  __syncthreads();
-}
-
-// One launch per reverse step and variant: CTA b runs work item b.
-template <int TY, int MODE>
-__global__ void __launch_bounds__(32 * TY, AdjBounds<MODE>::MIN_CTAS)
-adj_step_kernel(const RfxbInst* __restrict__ insts, const AdjInst* __restrict__ adjs,
-                const RfxbWork* __restrict__ work, const CUtensorMap* __restrict__ maps, int n, int par, int apar,
-                int zp) {
-  extern __shared__ __align__(128) unsigned char adj_smem_raw[];
-  constexpr bool RING = MODE == 2 || MODE == 4;
-  if (MODE != 0) adj_init_barriers<TY>(adj_smem_raw, RING ? 3 : RFXB_ANSTAGE, RING, threadIdx.y * 32 + threadIdx.x);
-  StepPhases ph;
-  adj_item<TY, MODE>(adj_smem_raw, insts, adjs, work[blockIdx.x], maps, n, par, apar, zp, ph, StepFault{}, true);
-}
-
-__device__ __forceinline__ bool adj_work_valid(const RfxbWork& w, const RfxbInst* insts, int n_inst, int ty) {
-  if (w.inst < 0 || w.inst >= n_inst) return false;
-  const RfxbInst& I = insts[w.inst];
-  return w.y0 >= 0 && w.y0 < I.ny && w.y0 % ty == 0 && w.z0 >= 0 && w.z0 < I.nz && w.z0 % RFXB_TZ == 0 &&
-         w.xa >= 0 && w.xa < w.xb && w.xb <= I.nx;
-}
-
-// Persistent reverse step: one launch per reverse step of as many CTAs as
-// are resident.  Queue 0 holds the tiles that reach a y slab (variant 2),
-// queue 1 the other CPML work (variant 4), queue 2 the CPML-free tiles
-// (variant 3).  CTAs of role 0 (blocks [0, role_ctas), one per SM when the
-// first wave spreads) take CPML-free items first, role 1 variant-4 items,
-// role 2 variant-2 items; an emptied queue sends a CTA to the others, so the
-// latency-bound CPML work and the bandwidth-bound plain work share every SM.
-// Invalid items are skipped and flagged (status bit 2); the last CTA to
-// finish clears the fetch counters for the next launch.
-template <int TY>
-__global__ void __launch_bounds__(32 * TY, 3)
-adj_persist_kernel(const RfxbInst* __restrict__ insts, const AdjInst* __restrict__ adjs, int n_inst,
-                   RfxbAdjQueues Q, const CUtensorMap* __restrict__ maps, int n, int par, int apar) {
-  extern __shared__ __align__(128) unsigned char adj_smem_raw[];
-  __shared__ int pick[2];
-  const int tid = threadIdx.y * 32 + threadIdx.x;
-  adj_init_barriers<TY>(adj_smem_raw, RFXB_ANSTAGE, true, tid);
-  StepPhases ph;
-  StepFault fault;
-  fault.cta = Q.fault_cta;
-  fault.wait_limit = Q.wait_limit;
-  static constexpr int kOrder[3][3] = {{2, 1, 0}, {1, 0, 2}, {0, 1, 2}};
-  const int role = min(2, (int)blockIdx.x / max(1, Q.role_ctas));
-  bool first_item = true;
-  bool ok = true;
-  while (ok) {
-    if (tid == 0) {
-      pick[0] = -1;
-      for (int t = 0; t < 3; ++t) {
-        const int q = kOrder[role][t];
-        if (*(volatile int*)&Q.ctr[q] >= Q.count[q]) continue;   // drained (counters only grow): no ticket
-        const int k = atomicAdd(&Q.ctr[q], 1);
-        if (k < Q.count[q]) { pick[0] = q; pick[1] = k; break; }
-      }
-    }
-    __syncthreads();
-    const int q = pick[0], k = pick[1];
-    __syncthreads();
-    if (q < 0) break;
-    const RfxbWork w = Q.list[q][k];
-    if (!adj_work_valid(w, insts, n_inst, TY)) {
-      if (tid == 0) atomicOr(Q.status, 2);
-      continue;
-    }
-    if (q == 0) ok = adj_item<TY, 2>(adj_smem_raw, insts, adjs, w, maps, n, par, apar, Q.zp, ph, fault, first_item);
-    else if (q == 1) ok = adj_item<TY, 4>(adj_smem_raw, insts, adjs, w, maps, n, par, apar, Q.zp, ph, fault, first_item);
-    else ok = adj_item<TY, 3>(adj_smem_raw, insts, adjs, w, maps, n, par, apar, Q.zp, ph, fault, first_item);
-    first_item = false;
-  }
-  if (tid == 0) {
-    __threadfence();
-    if (atomicAdd(&Q.ctr[3], 1) == (int)gridDim.x - 1) {
-      Q.ctr[0] = 0;
-      Q.ctr[1] = 0;
-      Q.ctr[2] = 0;
-      Q.ctr[3] = 0;
-      __threadfence();
-    }
-  }
-}
-
-template __global__ void adj_step_kernel<8, 0>(const RfxbInst*, const AdjInst*, const RfxbWork*,
-                                               const CUtensorMap*, int, int, int, int);
-template __global__ void adj_step_kernel<8, 1>(const RfxbInst*, const AdjInst*, const RfxbWork*,
-                                               const CUtensorMap*, int, int, int, int);
-template __global__ void adj_step_kernel<8, 2>(const RfxbInst*, const AdjInst*, const RfxbWork*,
-                                               const CUtensorMap*, int, int, int, int);
-template __global__ void adj_step_kernel<8, 3>(const RfxbInst*, const AdjInst*, const RfxbWork*,
-                                               const CUtensorMap*, int, int, int, int);
-template __global__ void adj_step_kernel<8, 4>(const RfxbInst*, const AdjInst*, const RfxbWork*,
-                                               const CUtensorMap*, int, int, int, int);
-template __global__ void adj_persist_kernel<8>(const RfxbInst*, const AdjInst*, int, RfxbAdjQueues,
-                                               const CUtensorMap*, int, int, int);
-
-// Dynamic shared memory of a mode: the fixed part, the plane stages it uses
-// and (modes 2, 4) the two ring slots sized for z-psi rows of zp floats, or
-// (modes 0, 1) the exchange array.
-size_t adj_step_smem_bytes(int mode, int zp) {
-  if (mode == 5)   // the persistent kernel: the largest of variants 2, 3 and 4
-    return std::max(std::max(adj_step_smem_bytes(2, zp), adj_step_smem_bytes(3, zp)), adj_step_smem_bytes(4, zp));
-  using Lite = AdjSmem<8, false>;
-  using Full = AdjSmem<8, true>;
-  if (mode == 4)
-    return offsetof(Lite, st) + 3 * sizeof(AdjStage<8, false>) +
-           2 * sizeof(float) * (size_t)APsiSlot<8, false>::FLOATS(zp);
-  const size_t fixed = offsetof(Full, st);
-  if (mode == 2) return fixed + 3 * sizeof(AdjStage<8, true>) + 2 * sizeof(float) * (size_t)APsiSlot<8, true>::FLOATS(zp);
-  if (mode == 3) return fixed + RFXB_ANSTAGE * sizeof(AdjStage<8, true>);
-  return fixed + RFXB_ANSTAGE * sizeof(AdjStage<8, true>) + sizeof(AdjExchange<8>);
-}
+size_t adj_step_smem_bytes() { return sizeof(AdjSmem<8>); }
 
 }  // namespace rfxb

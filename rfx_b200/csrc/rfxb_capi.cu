@@ -24,9 +24,8 @@
 #include "rfxb_common.cuh"
 
 namespace rfxb {
-template <int TY, int MODE, bool EM>
-__global__ void fwd_step_kernel(const RfxbInst*, const RfxbWork*, const CUtensorMap*, int, int);
-size_t fwd_step_smem_bytes(int mode);
+__global__ void fwd_step_kernel(const RfxbInst*, const RfxbWork*, int, int);
+size_t fwd_step_smem_bytes();
 __global__ void dft_kernel(const RfxbInst*, const RfxbDftPlane*, int, int, int);
 __global__ void pack_kernel(float*, const float*, RfxbInst);
 __global__ void unpack_kernel(float*, const float*, RfxbInst);
@@ -43,15 +42,19 @@ __global__ void box_energy_kernel(RfxbInst, int, int, int, int, int, int, int, c
 __global__ void box_flux_kernel(RfxbInst, int, int, int, int, int, int, int, double*);
 __global__ void flux_kernel(const RfxbInst*, const RfxbFluxPlane*, int, int, int);
 __global__ void ntff_kernel(const RfxbInst*, const RfxbNtffFace*, int, int, int);
-template <int TY, int MODE>
-__global__ void adj_step_kernel(const RfxbInst*, const AdjInst*, const RfxbWork*, const CUtensorMap*, int, int, int,
-                                int);
-template <int TY, bool EM>
-__global__ void fwd_persist_kernel(const RfxbInst*, int, RfxbFwdQueues, const CUtensorMap*, int, int);
-template <int TY>
-__global__ void adj_persist_kernel(const RfxbInst*, const AdjInst*, int, RfxbAdjQueues, const CUtensorMap*, int, int,
-                                   int);
-size_t adj_step_smem_bytes(int mode, int zp);
+__global__ void adj_step_kernel(const RfxbInst*, const AdjInst*, const RfxbWork*, int, int, int);
+template <int TY, int ZQ, bool CP>
+__global__ void adjv_kernel(const RfxbInst*, const AdjInst*, const RfxbWork*, const CUtensorMap*, int, int, int, int);
+template <int TY, int ZQ>
+__global__ void adjv_persist_kernel(const RfxbInst*, const AdjInst*, int, RfxbAdjQueues, const CUtensorMap*, int, int,
+                                    int, int);
+size_t adjv_smem_bytes(int tile, bool cp);
+template <int TY, int ZQ, bool CP>
+__global__ void fwdv_kernel(const RfxbInst*, const RfxbWork*, const CUtensorMap*, int, int, int);
+template <int TY, int ZQ>
+__global__ void fwdv_persist_kernel(const RfxbInst*, int, RfxbFwdQueues, const CUtensorMap*, int, int, int);
+size_t fwdv_smem_bytes(int tile, bool cp);
+size_t adj_step_smem_bytes();
 template <int TY>
 __global__ void fwd2_step_kernel(const RfxbInst*, const RfxbWork2*, const CUtensorMap*, int, int);
 size_t fwd2_step_smem_bytes();
@@ -91,17 +94,6 @@ int sm_count() {
     int dev = 0;
     cudaGetDevice(&dev);
     if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) n = 148;
-  }
-  return n;
-}
-
-// Shared memory of one SM (228 KB on B200).
-int smem_per_sm() {
-  static int n = -1;
-  if (n < 0) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&n, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess) n = 233472;
   }
   return n;
 }
@@ -146,8 +138,6 @@ struct RfxbPlan {
   RfxbBatch* self_group = nullptr;
   // TMA descriptors (layout in rfxb_inst.h, RFXB_NMAPS)
   CUtensorMap tmaps[RFXB_NMAPS];
-  bool psi_maps_ok = false;    // the CPML psi maps encoded (staged-psi kernel usable)
-  bool adj_psi_maps_ok = false;  // the same for the adjoint psi
   int l2promo = 2;             // L2 promotion of this plan's TMA maps: 0 none, 1 64 B, 2 128 B, 3 256 B
 
   ~RfxbPlan() {
@@ -183,8 +173,12 @@ struct RfxbBatch {
   AdjInst* d_adj = nullptr;
   RfxbWork* d_work = nullptr;     // every tile (reverse steps; forward steps when not split)
   int n_work = 0;
-  // forward steps split between the CPML-free kernel (list 1) and the
-  // staged-psi kernel (list 2), launched side by side on two streams
+  // forward steps in one launch: every tile of shape vtile (rfxb_fwdv.cu)
+  int vtile = 0;
+  RfxbWork* d_wv = nullptr;
+  int n_wv = 0;
+  // forward steps split between the CPML-free tiles (list 1) and the others
+  // (list 2), launched side by side on two streams
   bool fwd_split = false;
   bool fwd_split_avail = false;   // both forward lists exist (fwd_split may be chosen)
   int fwd_order = 0;              // split forward: 0 plain-tile launch first, 1 CPML-tile launch first
@@ -192,19 +186,19 @@ struct RfxbBatch {
   int n_wf1 = 0;
   RfxbWork* d_wf2 = nullptr;
   int n_wf2 = 0;
-  // reverse steps split the same way (list 1 on the CPML-free variant 3)
-  bool adj_split = false;
+  // reverse steps in one launch (shape vtile), or split three ways on three
+  // streams (8 x 32 tiles): CPML-free tiles, tiles that reach a y slab, the
+  // other CPML work
+  RfxbWork* d_wva = nullptr;
+  int n_wva = 0;
   RfxbWork* d_wa1 = nullptr;
   int n_wa1 = 0;
-  RfxbWork* d_wa2 = nullptr;
-  int n_wa2 = 0;
   cudaStream_t side_stream = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
-  // reverse variant 4 (CPML work that reaches no y slab) on a third stream
-  bool adj_lite = false;
-  bool adj_lite_avail = false;    // the variant-4 lists exist (adj_lite may be chosen)
-  int adj_order = 0;              // permutation index of the reverse launches (rfxb200.h)
-  RfxbWork* d_wa2y = nullptr;   // variant 2 list when variant 4 takes the rest
+  bool adj_lite = false;          // the split reverse launches are chosen
+  bool adj_lite_avail = false;    // their lists exist
+  int adj_order = 0;              // permutation index of the split launches (rfxb200.h)
+  RfxbWork* d_wa2y = nullptr;
   int n_wa2y = 0;
   RfxbWork* d_wa4 = nullptr;
   int n_wa4 = 0;
@@ -250,7 +244,6 @@ struct RfxbBatch {
   int adj_persist_grid = 0;        // CTAs of the persistent reverse launch (resident at once)
   int fwd_mode = 0;                // forward step kernel variant (see rfxb_fwd.cu)
   int adj_mode = -1;               // reverse step kernel variant (see rfxb_adj_fused.cu), -1 not chosen yet
-  int adj_zp = 4;                  // z-psi row capacity of the mode-2 reverse ring
   std::vector<RfxbDftPlane> dft;
   int dft_blocks = 0;
   std::vector<void*> allocs;
@@ -320,7 +313,8 @@ struct WorkSeg {
   double c, cx;
 };
 
-void balance_segments(const std::vector<WorkSeg>& segs, int resident, double prologue, std::vector<RfxbWork>& out) {
+void balance_segments(const std::vector<WorkSeg>& segs, int resident, double prologue, std::vector<RfxbWork>& out,
+                      int min_waves = 1) {
   out.clear();
   if (segs.empty()) return;
   auto plane_cost = [](const WorkSeg& t, int i) {
@@ -385,7 +379,7 @@ void balance_segments(const std::vector<WorkSeg>& segs, int resident, double pro
   };
   std::vector<Item> best, cur;
   double best_t = 1e300;
-  for (int waves = 1; waves <= 4; ++waves) {
+  for (int waves = min_waves; waves <= min_waves + 3; ++waves) {
     cut(W / ((double)resident * waves), cur);
     const double t = makespan(cur);
     if (t < best_t * (1.0 - 0.02)) { best_t = t; best = cur; }   // more waves only for a clear gain
@@ -395,63 +389,72 @@ void balance_segments(const std::vector<WorkSeg>& segs, int resident, double pro
 
 // Whether a forward tile's cells (rows y0-1 .. y0+TY-1, columns z0-1 ..
 // z0+31) reach a y or z CPML slab.
-bool tile_reaches_yz(const RfxbPlan& p, int y0, int z0) {
+bool tile_reaches_yz(const RfxbPlan& p, int y0, int z0, int ty = kTY, int tz = 32) {
   const int n = p.inst.ncp;
   const unsigned ax = n > 0 ? p.inst.cpml_axes : 0u;
-  return ((ax & 2u) && (y0 - 1 < n || y0 + kTY - 1 >= p.ny - n)) ||
-         ((ax & 4u) && (z0 - 1 < n || z0 + 31 >= p.nz - n));
+  return ((ax & 2u) && (y0 - 1 < n || y0 + ty - 1 >= p.ny - n)) ||
+         ((ax & 4u) && (z0 - 1 < n || z0 + tz - 1 >= p.nz - n));
 }
 
-// Segments of every tile's full x line (cost model of the staged kernels).
+// Segments of every tile's full x line.
 void all_segments(const std::vector<RfxbPlan*>& plans, double slab, std::vector<WorkSeg>& segs) {
+  const int ty = kTY, tz = 32;
   for (size_t q = 0; q < plans.size(); ++q) {
     const RfxbPlan& p = *plans[q];
     const int n = p.inst.ncp;
     const unsigned ax = n > 0 ? p.inst.cpml_axes : 0u;
-    for (int y0 = 0; y0 < p.ny; y0 += kTY)
-      for (int z0 = 0; z0 < p.nz; z0 += 32) {
+    for (int y0 = 0; y0 < p.ny; y0 += ty)
+      for (int z0 = 0; z0 < p.nz; z0 += tz) {
         double c = 1.0;
-        if ((ax & 2u) && (y0 - 1 < n || y0 + kTY - 1 >= p.ny - n)) c += slab;
-        if ((ax & 4u) && (z0 - 1 < n || z0 + 31 >= p.nz - n)) c += slab;
+        if ((ax & 2u) && (y0 - 1 < n || y0 + ty - 1 >= p.ny - n)) c += slab;
+        if ((ax & 4u) && (z0 - 1 < n || z0 + tz - 1 >= p.nz - n)) c += slab;
         const int ncpx = (ax & 1u) ? n : 0;
         segs.push_back(WorkSeg{(int)q, y0, z0, 0, p.nx, p.nx, ncpx, c, (ax & 1u) ? slab : 0.0});
       }
   }
 }
 
+// Modelled cost of a tile-plane beyond a CPML-free one: cp for running the CPML
+// code at all, x / y / z for the slab it lies in.
+struct SlabCost {
+  double x, y, z, cp;
+  SlabCost(double s) : x(s), y(s), z(s), cp(0.0) {}
+  SlabCost(double sx, double sy, double sz, double c) : x(sx), y(sy), z(sz), cp(c) {}
+};
+
 // Split of the forward work between the CPML-free kernel (variant 1) and the
 // staged-psi kernel (variant 2): a tile that reaches no y/z slab runs planes
 // ncp+1 .. nx-ncp-1 (whose x-1 prologue plane is outside the x slab too) on
 // variant 1, everything else on variant 2.
-void split_segments(const std::vector<RfxbPlan*>& plans, double slab, std::vector<WorkSeg>& plain,
-                    std::vector<WorkSeg>& cpml) {
+void split_segments(const std::vector<RfxbPlan*>& plans, const SlabCost& slab, std::vector<WorkSeg>& plain,
+                    std::vector<WorkSeg>& cpml, int ty = kTY, int tz = 32) {
   for (size_t q = 0; q < plans.size(); ++q) {
     const RfxbPlan& p = *plans[q];
     const int n = p.inst.ncp;
     const unsigned ax = n > 0 ? p.inst.cpml_axes : 0u;
-    for (int y0 = 0; y0 < p.ny; y0 += kTY)
-      for (int z0 = 0; z0 < p.nz; z0 += 32) {
+    for (int y0 = 0; y0 < p.ny; y0 += ty)
+      for (int z0 = 0; z0 < p.nz; z0 += tz) {
         if (ax == 0u) {
           plain.push_back(WorkSeg{(int)q, y0, z0, 0, p.nx, p.nx, 0, 1.0, 0.0});
           continue;
         }
         const int ncpx = (ax & 1u) ? n : 0;
-        const double cx = (ax & 1u) ? slab : 0.0;
-        if (tile_reaches_yz(p, y0, z0)) {
-          double c = 1.0;
-          if ((ax & 2u) && (y0 - 1 < n || y0 + kTY - 1 >= p.ny - n)) c += slab;
-          if ((ax & 4u) && (z0 - 1 < n || z0 + 31 >= p.nz - n)) c += slab;
+        const double cx = (ax & 1u) ? slab.x : 0.0;
+        if (tile_reaches_yz(p, y0, z0, ty, tz)) {
+          double c = 1.0 + slab.cp;
+          if ((ax & 2u) && (y0 - 1 < n || y0 + ty - 1 >= p.ny - n)) c += slab.y;
+          if ((ax & 4u) && (z0 - 1 < n || z0 + tz - 1 >= p.nz - n)) c += slab.z;
           cpml.push_back(WorkSeg{(int)q, y0, z0, 0, p.nx, p.nx, ncpx, c, cx});
           continue;
         }
         const int lo = ncpx > 0 ? ncpx + 1 : 0, hi = ncpx > 0 ? p.nx - ncpx : p.nx;
         if (hi - lo < 4) {
-          cpml.push_back(WorkSeg{(int)q, y0, z0, 0, p.nx, p.nx, ncpx, 1.0, cx});
+          cpml.push_back(WorkSeg{(int)q, y0, z0, 0, p.nx, p.nx, ncpx, 1.0 + slab.cp, cx});
           continue;
         }
         plain.push_back(WorkSeg{(int)q, y0, z0, lo, hi, p.nx, 0, 1.0, 0.0});
-        if (lo > 0) cpml.push_back(WorkSeg{(int)q, y0, z0, 0, lo, p.nx, ncpx, 1.0, cx});
-        if (hi < p.nx) cpml.push_back(WorkSeg{(int)q, y0, z0, hi, p.nx, p.nx, ncpx, 1.0, cx});
+        if (lo > 0) cpml.push_back(WorkSeg{(int)q, y0, z0, 0, lo, p.nx, ncpx, 1.0 + slab.cp, cx});
+        if (hi < p.nx) cpml.push_back(WorkSeg{(int)q, y0, z0, hi, p.nx, p.nx, ncpx, 1.0 + slab.cp, cx});
       }
   }
 }
@@ -459,40 +462,41 @@ void split_segments(const std::vector<RfxbPlan*>& plans, double slab, std::vecto
 // The reverse step's split: its CPML terms reach rows y0-1 .. y0+TY, columns
 // z0-1 .. z0+32 and planes xa-1 .. xb, so the CPML-free range of a tile that
 // reaches no y/z slab is ncp+1 .. nx-ncp-2.
-void split_adj_segments(const std::vector<RfxbPlan*>& plans, double slab, std::vector<WorkSeg>& plain,
-                        std::vector<WorkSeg>& cpml, std::vector<WorkSeg>* cpml_noy = nullptr) {
+void split_adj_segments(const std::vector<RfxbPlan*>& plans, const SlabCost& slab, std::vector<WorkSeg>& plain,
+                        std::vector<WorkSeg>& cpml, std::vector<WorkSeg>* cpml_noy = nullptr, int ty = kTY,
+                        int tz = 32) {
   for (size_t q = 0; q < plans.size(); ++q) {
     const RfxbPlan& p = *plans[q];
     const int n = p.inst.ncp;
     const unsigned ax = n > 0 ? p.inst.cpml_axes : 0u;
-    for (int y0 = 0; y0 < p.ny; y0 += kTY)
-      for (int z0 = 0; z0 < p.nz; z0 += 32) {
+    for (int y0 = 0; y0 < p.ny; y0 += ty)
+      for (int z0 = 0; z0 < p.nz; z0 += tz) {
         if (ax == 0u) {
           plain.push_back(WorkSeg{(int)q, y0, z0, 0, p.nx, p.nx, 0, 1.0, 0.0});
           continue;
         }
         const int ncpx = (ax & 1u) ? n : 0;
-        const double cx = (ax & 1u) ? slab : 0.0;
-        const bool yz = ((ax & 2u) && (y0 - 1 < n || y0 + kTY >= p.ny - n)) ||
-                        ((ax & 4u) && (z0 - 1 < n || z0 + 32 >= p.nz - n));
-        const bool ys = (ax & 2u) && (y0 - 1 < n || y0 + kTY >= p.ny - n);
+        const double cx = (ax & 1u) ? slab.x : 0.0;
+        const bool yz = ((ax & 2u) && (y0 - 1 < n || y0 + ty >= p.ny - n)) ||
+                        ((ax & 4u) && (z0 - 1 < n || z0 + tz >= p.nz - n));
+        const bool ys = (ax & 2u) && (y0 - 1 < n || y0 + ty >= p.ny - n);
         // CPML work whose tile reaches no y slab goes to cpml_noy when given
         std::vector<WorkSeg>& dst = (cpml_noy && !ys) ? *cpml_noy : cpml;
         if (yz) {
-          double c = 1.0;
-          if (ys) c += slab;
-          if ((ax & 4u) && (z0 - 1 < n || z0 + 32 >= p.nz - n)) c += slab;
+          double c = 1.0 + slab.cp;
+          if (ys) c += slab.y;
+          if ((ax & 4u) && (z0 - 1 < n || z0 + tz >= p.nz - n)) c += slab.z;
           dst.push_back(WorkSeg{(int)q, y0, z0, 0, p.nx, p.nx, ncpx, c, cx});
           continue;
         }
         const int lo = ncpx > 0 ? ncpx + 1 : 0, hi = ncpx > 0 ? p.nx - ncpx - 1 : p.nx;
         if (hi - lo < 4) {
-          dst.push_back(WorkSeg{(int)q, y0, z0, 0, p.nx, p.nx, ncpx, 1.0, cx});
+          dst.push_back(WorkSeg{(int)q, y0, z0, 0, p.nx, p.nx, ncpx, 1.0 + slab.cp, cx});
           continue;
         }
         plain.push_back(WorkSeg{(int)q, y0, z0, lo, hi, p.nx, 0, 1.0, 0.0});
-        if (lo > 0) dst.push_back(WorkSeg{(int)q, y0, z0, 0, lo, p.nx, ncpx, 1.0, cx});
-        if (hi < p.nx) dst.push_back(WorkSeg{(int)q, y0, z0, hi, p.nx, p.nx, ncpx, 1.0, cx});
+        if (lo > 0) dst.push_back(WorkSeg{(int)q, y0, z0, 0, lo, p.nx, ncpx, 1.0 + slab.cp, cx});
+        if (hi < p.nx) dst.push_back(WorkSeg{(int)q, y0, z0, hi, p.nx, p.nx, ncpx, 1.0 + slab.cp, cx});
       }
   }
 }
@@ -648,23 +652,34 @@ double slab_weight() {
   return v;
 }
 
-// RFXB_FWD_SPLIT=0 runs all forward tiles of a staged-psi group on one kernel.
+// RFXB_FWD_SPLIT=1 starts groups with CPML on the two-launch forward step.
 bool fwd_split_enabled() {
   static int v = -1;
   if (v < 0) {
     const char* e = getenv("RFXB_FWD_SPLIT");
-    v = (e && std::string(e) == "0") ? 0 : 1;
+    v = (e && std::string(e) == "1") ? 1 : 0;
   }
   return v == 1;
 }
 
-// RFXB_ADJ_LITE=0 keeps the reverse CPML work of tiles without a y slab on
-// variant 2 instead of variant 4.
+// The single-launch lists, from launches of one kind of tile alone on the 277^3
+// grid (24 x 32 tiles, ns per tile-plane): CPML-free code 8.9, CPML code clear of
+// the slabs 11.8, in a y slab 12.2, in a z slab 19.4, in both 22.4, in an x slab
+// 20 in short pieces.  The reverse kernel's y and z slabs cost about alike.
+const SlabCost kFwdCost(0.4, 0.1, 0.7, 0.15), kAdjCost(0.3, 0.3, 0.3, 0.1);
+// Start-up of an item in plane costs and the fewest waves an x line is cut for.
+// Forward: little start-up, so many short pieces (step of the 277^3 grid 327 us
+// at one wave, 317 at four; of the 221x141x69 grid 94 and 78).  Reverse: the
+// start-up evaluates two planes of fluxes (100 us at one wave, 113 at three).
+constexpr double kFwdPrologue = 0.3, kAdjPrologue = 3.0;
+constexpr int kFwdWaves = 4, kAdjWaves = 1;
+
+// RFXB_ADJ_LITE=1 starts groups with CPML on the split reverse launches.
 bool adj_lite_enabled() {
   static int v = -1;
   if (v < 0) {
     const char* e = getenv("RFXB_ADJ_LITE");
-    v = (e && std::string(e) == "0") ? 0 : 1;
+    v = (e && std::string(e) == "1") ? 1 : 0;
   }
   return v == 1;
 }
@@ -724,15 +739,42 @@ void allow_smem(const void* kernel, size_t bytes) {
     cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
 }
 
-// Forward step kernel of a mode with its dynamic shared memory enabled.
-using FwdKernel = void (*)(const RfxbInst*, const RfxbWork*, const CUtensorMap*, int, int);
-FwdKernel fwd_kernel(int mode, bool em = false) {
-  em = em && mode != 0;
-  FwdKernel k = mode == 2 ? (em ? fwd_step_kernel<kTY, 2, true> : fwd_step_kernel<kTY, 2, false>)
-                : mode == 1 ? (em ? fwd_step_kernel<kTY, 1, true> : fwd_step_kernel<kTY, 1, false>)
-                            : fwd_step_kernel<kTY, 0, false>;
-  allow_smem(reinterpret_cast<const void*>(k), fwd_step_smem_bytes(mode));
+// Tile shapes of the forward step kernel (rfxb_fwdv.cu): rows, columns and
+// threads of a CTA.  Shape 1 is the 8 x 32 tile of the lists the two-step and
+// reverse kernels share.
+struct FwdTile { int ty, tz, threads; };
+constexpr FwdTile kFwdTile[2] = {{24, 32, 224}, {8, 32, 96}};
+
+using FwdKernel = void (*)(const RfxbInst*, const RfxbWork*, const CUtensorMap*, int, int, int);
+FwdKernel fwd_kernel(int tile, bool cp) {
+  FwdKernel k = tile == 0 ? (cp ? fwdv_kernel<24, 8, true> : fwdv_kernel<24, 8, false>)
+                          : (cp ? fwdv_kernel<8, 8, true> : fwdv_kernel<8, 8, false>);
+  allow_smem(reinterpret_cast<const void*>(k), fwdv_smem_bytes(tile, cp));
   return k;
+}
+
+void launch_fwd(int tile, bool cp, const RfxbBatch* g, const RfxbWork* list, int count, int n, int sel, cudaStream_t st) {
+  fwd_kernel(tile, cp)<<<count, kFwdTile[tile].threads, fwdv_smem_bytes(tile, cp), st>>>(
+      g->d_inst, list, g->d_maps, RFXB_MAP_V0 + 7 * tile, n, sel);
+}
+
+// The generic per-thread-copy forward kernel (RFXB_STAGING=cpasync, and plans
+// whose psi offsets pass 32 bits).
+void launch_fwd_generic(const RfxbBatch* g, int n, int sel, cudaStream_t st) {
+  allow_smem(reinterpret_cast<const void*>(fwd_step_kernel), fwd_step_smem_bytes());
+  fwd_step_kernel<<<g->n_work, dim3(32, kTY), fwd_step_smem_bytes(), st>>>(g->d_inst, g->d_work, n, sel);
+}
+
+// Tile shape of a group: 24 rows reread less halo and use larger CTAs, but a
+// grid needs enough of them; the line lies where eight-plane pieces still give
+// every SM its two CTAs.  Below it (97x83x109, 24 rows / 8 rows): forward 35 / 32
+// us, reverse 45 / 43; above it (the 221x141x69 grid) forward 78 / 90, reverse
+// 100 / 133, (64 grids of 64-160 a side) forward 1005 / 1207, reverse 1375 / 1839.
+int pick_fwd_tile(const RfxbBatch* g) {
+  long long items = 0;
+  for (const RfxbPlan* p : g->plans)
+    items += (long long)((p->ny + 23) / 24) * ((p->nz + 31) / 32) * (p->nx / 8);
+  return items >= 2LL * sm_count() ? 0 : 1;
 }
 
 // The two-step kernel with its dynamic shared memory enabled.
@@ -775,25 +817,20 @@ int fwd_depth_default(const RfxbBatch* g) {
   return cells >= (1LL << 24) ? 2 : 1;
 }
 
-using FwdPersistKernel = void (*)(const RfxbInst*, int, RfxbFwdQueues, const CUtensorMap*, int, int);
-FwdPersistKernel fwd_persist_kernel_for(bool em) {
-  FwdPersistKernel k = em ? fwd_persist_kernel<kTY, true> : fwd_persist_kernel<kTY, false>;
-  allow_smem(reinterpret_cast<const void*>(k), fwd_step_smem_bytes(2));
-  return k;
-}
-
 // CTAs of a persistent forward launch: as many as are resident at once.
-int fwd_persist_grid(bool em) {
-  static int r[2] = {-1, -1};
-  if (r[em] < 0) {
+int fwd_persist_grid() {
+  static int r = -1;
+  if (r < 0) {
+    const auto k = fwdv_persist_kernel<8, 8>;
+    allow_smem(reinterpret_cast<const void*>(k), fwdv_smem_bytes(1, true));
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fwd_persist_kernel_for(em), 32 * kTY,
-                                                      fwd_step_smem_bytes(2)) != cudaSuccess ||
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kFwdTile[1].threads, fwdv_smem_bytes(1, true)) !=
+            cudaSuccess ||
         per_sm < 1)
       per_sm = 1;
-    r[em] = per_sm * sm_count();
+    r = per_sm * sm_count();
   }
-  return r[em];
+  return r;
 }
 
 // Default of the persistent forward launch (RFXB_PERSIST=0 turns it off,
@@ -808,17 +845,18 @@ int fwd_persist_default() {
 // y-slab tiles, variant 4 on the other CPML work, variant 3 on plain tiles).
 bool adj_persist_avail(const RfxbBatch* g);
 
-int resident_ctas(int mode) {
-  static int r[3] = {-1, -1, -1};
-  if (r[mode] < 0) {
+// CTAs of a forward tile shape resident at once.
+int resident_ctas(int tile, bool cp) {
+  static int r[2][2] = {{-1, -1}, {-1, -1}};
+  if (r[tile][cp] < 0) {
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fwd_kernel(mode), 32 * kTY,
-                                                      fwd_step_smem_bytes(mode)) != cudaSuccess ||
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fwd_kernel(tile, cp), kFwdTile[tile].threads,
+                                                      fwdv_smem_bytes(tile, cp)) != cudaSuccess ||
         per_sm < 1)
-      per_sm = mode == 2 ? 3 : 4;
-    r[mode] = per_sm * sm_count();
+      per_sm = tile == 0 ? 2 : 5;
+    r[tile][cp] = per_sm * sm_count();
   }
-  return r[mode];
+  return r[tile][cp];
 }
 
 // TMA staging is the default; RFXB_STAGING=cpasync selects per-thread 16-byte
@@ -889,227 +927,85 @@ int encode_block_map(CUtensorMap* m, const RfxbPlan& p, float* block, int ncomp,
   return 0;
 }
 
-// Map over the padded PEC edge-mask bytes: dims (zs, ny+2, nx+2, 1) with the
-// origin at cell (-1, -1, 0), the tile box (32, TY, 1, 1).
-int encode_emask_map(RfxbPlan* p) {
-  auto fn = tensor_map_encoder();
-  if (!fn) return fail(RFXB_E_LAUNCH, "cuTensorMapEncodeTiled is not available from the driver");
-  const RfxbInst& I = p->inst;
-  void* addr = p->emask + (I.off0 - I.ps - I.zs);
-  cuuint64_t dims[4] = {(cuuint64_t)I.zs, (cuuint64_t)(p->ny + 2), (cuuint64_t)(p->nx + 2), 1};
-  cuuint64_t strides[3] = {(cuuint64_t)I.zs, (cuuint64_t)I.ps, (cuuint64_t)I.ps * (cuuint64_t)(p->nx + 2)};
-  cuuint32_t box[4] = {32, (cuuint32_t)kTY, 1, 1};
-  cuuint32_t estr[4] = {1, 1, 1, 1};
-  const CUresult r = fn(&p->tmaps[RFXB_MAP_EMASK], CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, addr, dims, strides, box, estr,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, l2_promotion(p->l2promo),
-                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return fail(RFXB_E_LAUNCH, "cuTensorMapEncodeTiled (edge mask) failed (" + std::to_string((int)r) + ")");
-  return 0;
-}
-
-// 4-D map over one CPML psi array: dims (d0, d1, d2, 4 = side*2 + q), rows of
-// d0 floats, box (b0, b1, 1, 2).
-int encode_psi_map(CUtensorMap* m, float* base, long long d0, long long d1, long long d2, unsigned b0, unsigned b1,
-                   int promo) {
-  auto fn = tensor_map_encoder();
-  if (!fn) return fail(RFXB_E_LAUNCH, "cuTensorMapEncodeTiled is not available from the driver");
-  cuuint64_t dims[4] = {(cuuint64_t)d0, (cuuint64_t)d1, (cuuint64_t)d2, 4};
-  cuuint64_t strides[3] = {(cuuint64_t)(d0 * 4), (cuuint64_t)(d0 * d1 * 4), (cuuint64_t)(d0 * d1 * d2 * 4)};
-  cuuint32_t box[4] = {b0, b1, 1, 2};
-  cuuint32_t estr[4] = {1, 1, 1, 1};
-  const CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, base, dims, strides, box, estr,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, l2_promotion(promo),
-                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return fail(RFXB_E_LAUNCH, "cuTensorMapEncodeTiled (psi) failed (" + std::to_string((int)r) + ")");
-  return 0;
-}
-
-int encode_psi_maps(RfxbPlan* p);
-
 int encode_forward_maps(RfxbPlan* p) {
   const unsigned ty = kTY;
-  for (int s = 0; s < 2; ++s) {
-    if (int rc = encode_block_map(&p->tmaps[s], *p, p->inst.F[s][0], 6, 40, ty + 2, 3)) return rc;
-    if (int rc = encode_block_map(&p->tmaps[2 + s], *p, p->inst.F[s][0], 6, 36, ty + 1, 3)) return rc;
+  for (int t = 0; t < 2; ++t) {
+    const unsigned tz = kFwdTile[t].tz, tyt = kFwdTile[t].ty;
+    CUtensorMap* m = &p->tmaps[RFXB_MAP_V0 + 7 * t];
+    for (int b = 0; b < 3; ++b) {
+      if (b == 2 && !p->mid) continue;
+      if (int rc = encode_block_map(m + b, *p, p->inst.F[b][0], 6, tz + 8, tyt + 2, 3)) return rc;
+      if (int rc = encode_block_map(m + 3 + b, *p, p->inst.F[b][0], 6, tz, tyt + 1, 3)) return rc;
+    }
+    if (int rc = encode_block_map(m + 6, *p, p->ca, 3, tz, tyt, 2)) return rc;
   }
-  if (int rc = encode_block_map(&p->tmaps[4], *p, p->ca, 3, 32, ty, 2)) return rc;
-  if (int rc = encode_block_map(&p->tmaps[10], *p, p->ca, 3, 32, ty, 1)) return rc;
-  // the two-step kernel's boxes (two-cell halo) and the intermediate state
+  // the two-step kernel's boxes (two-cell halo)
   for (int s = 0; s < 2; ++s) {
     if (int rc = encode_block_map(&p->tmaps[RFXB_MAP_E2 + s], *p, p->inst.F[s][0], 6, 40, ty + 4, 3)) return rc;
     if (int rc = encode_block_map(&p->tmaps[RFXB_MAP_H2 + s], *p, p->inst.F[s][0], 6, 40, ty + 3, 3)) return rc;
   }
   if (int rc = encode_block_map(&p->tmaps[RFXB_MAP_C2], *p, p->ca, 3, 40, ty + 2, 2)) return rc;
-  if (p->mid) {
-    if (int rc = encode_block_map(&p->tmaps[RFXB_MAP_MIDE], *p, p->mid, 6, 40, ty + 2, 3)) return rc;
-    if (int rc = encode_block_map(&p->tmaps[RFXB_MAP_MIDH], *p, p->mid, 6, 36, ty + 1, 3)) return rc;
-  }
-  const RfxbInst& I = p->inst;
-  p->psi_maps_ok = false;
-  if (I.ncp > 0) {
-    // a psi map the driver refuses only rules out the staged-psi kernel
-    const int rc = encode_psi_maps(p);
-    p->psi_maps_ok = rc == 0;
-  }
   return 0;
 }
 
-int encode_psi_maps(RfxbPlan* p) {
-  const unsigned ty = kTY;
-  const RfxbInst& I = p->inst;
-  {
-    const long long n = I.ncp, n4 = I.ncp4;
-    for (int s = 0; s < 2; ++s) {
-      if (I.cpml_axes & 1u) {
-        if (int rc = encode_psi_map(&p->tmaps[RFXB_MAP_PSH + s], I.psH[s][0], I.zs, p->ny, n, 36, ty + 1, p->l2promo)) return rc;
-        if (int rc = encode_psi_map(&p->tmaps[RFXB_MAP_PSE + s], I.psE[s][0], I.zs, p->ny, n, 32, ty, p->l2promo)) return rc;
-      }
-      if (I.cpml_axes & 2u) {
-        if (int rc = encode_psi_map(&p->tmaps[RFXB_MAP_PSH + 2 + s], I.psH[s][1], I.zs, n, p->nx, 36, ty + 1, p->l2promo)) return rc;
-        if (int rc = encode_psi_map(&p->tmaps[RFXB_MAP_PSE + 2 + s], I.psE[s][1], I.zs, n, p->nx, 32, ty, p->l2promo)) return rc;
-      }
-      if (I.cpml_axes & 4u) {
-        if (int rc = encode_psi_map(&p->tmaps[RFXB_MAP_PSH + 4 + s], I.psH[s][2], n4, p->ny, p->nx, (unsigned)n4, ty + 1, p->l2promo))
-          return rc;
-        if (int rc = encode_psi_map(&p->tmaps[RFXB_MAP_PSE + 4 + s], I.psE[s][2], n4, p->ny, p->nx, (unsigned)n4, ty, p->l2promo))
-          return rc;
-      }
-    }
-  }
-  return 0;
-}
-
-// Whether mode 2 (TMA-staged psi) can run a plan: the z-psi rows fit the
-// ring, no tile reaches both slabs of an axis (its rows y0-1..y0+TY-1 or
-// columns z0-1..z0+31), and psi offsets fit 32-bit arithmetic.
-bool psi_staging_ok(const RfxbPlan& p) {
-  const RfxbInst& I = p.inst;
-  if (I.ncp == 0) return true;
-  if (!p.psi_maps_ok || I.ncp4 > 16) return false;
+// Whether the four-cells-per-thread step kernels can run a plan: its psi offsets
+// fit 32-bit arithmetic, and no four columns reach both z slabs.
+bool vec_kernels_ok(const RfxbPlan& p) {
   for (int a = 0; a < 3; ++a)
     if (p.psi_elems[a] >= (1LL << 31)) return false;
-  const int n = I.ncp;
-  if (I.cpml_axes & 2u)
-    for (int y0 = 0; y0 < p.ny; y0 += kTY)
-      if (y0 - 1 < n && y0 + kTY - 1 >= p.ny - n) return false;
-  if (I.cpml_axes & 4u)
-    for (int z0 = 0; z0 < p.nz; z0 += 32)
-      if (z0 - 1 < n && z0 + 31 >= p.nz - n) return false;
-  return true;
+  return !(p.inst.ncp > 0 && (p.inst.cpml_axes & 4u) && p.nz - 2 * p.inst.ncp < 3);
 }
 
 // Forward kernel variant of a group: 0 with RFXB_STAGING=cpasync or when a
-// plan cannot stage its psi, 1 without any CPML, else 2.
-// RFXB_FWD_MODE=2 runs CPML-free groups on the staged-psi variant too (a
-// diagnostic of that variant's own cost).
+// plan does not suit the four-cells-per-thread kernels, 1 without any CPML, else 2.
 int group_fwd_mode(const RfxbBatch* g) {
   if (!use_tma()) return 0;
   bool any_cpml = false;
   for (auto* p : g->plans) {
     if (p->inst.ncp > 0) any_cpml = true;
-    if (!psi_staging_ok(*p)) return 0;
+    if (!vec_kernels_ok(*p)) return 0;
   }
-  const char* e = getenv("RFXB_FWD_MODE");
-  if (e && std::string(e) == "2") return 2;
   return any_cpml ? 2 : 1;
 }
 
 int encode_adjoint_maps(RfxbPlan* p) {
-  const unsigned ty = kTY;
-  for (int s = 0; s < 2; ++s) {
-    if (int rc = encode_block_map(&p->tmaps[5 + s], *p, p->adj.aF[s][0], 6, 40, ty + 2, 3)) return rc;
-    if (int rc = encode_block_map(&p->tmaps[7 + s], *p, p->adj.aF[s][0], 6, 36, ty + 1, 3)) return rc;
-  }
-  if (int rc = encode_block_map(&p->tmaps[9], *p, p->ca, 3, 40, ty + 2, 1)) return rc;
-  if (int rc = encode_block_map(&p->tmaps[10], *p, p->ca, 3, 32, ty, 1)) return rc;
-  if (int rc = encode_block_map(&p->tmaps[23], *p, p->ca, 3, 36, ty + 1, 1)) return rc;
-  p->adj_psi_maps_ok = false;
-  const RfxbInst& I = p->inst;
-  if (I.ncp > 0) {
-    // a psi map the driver refuses only rules out the staged-psi reverse kernel
-    auto enc = [&]() -> int {
-      const long long n = I.ncp, n4 = I.ncp4;
-      for (int s = 0; s < 2; ++s) {
-        if (I.cpml_axes & 1u) {
-          if (int rc = encode_psi_map(&p->tmaps[RFXB_MAP_APE + s], p->adj.aPsiE[s][0], I.zs, p->ny, n, 36, ty + 1, p->l2promo))
-            return rc;
-          if (int rc = encode_psi_map(&p->tmaps[RFXB_MAP_APH + s], p->adj.aPsiH[s][0], I.zs, p->ny, n, 32, ty, p->l2promo))
-            return rc;
-        }
-        if (I.cpml_axes & 2u) {
-          if (int rc = encode_psi_map(&p->tmaps[RFXB_MAP_APE + 2 + s], p->adj.aPsiE[s][1], I.zs, n, p->nx, 40, ty + 2, p->l2promo))
-            return rc;
-          if (int rc = encode_psi_map(&p->tmaps[RFXB_MAP_APH + 2 + s], p->adj.aPsiH[s][1], I.zs, n, p->nx, 36, ty + 1, p->l2promo))
-            return rc;
-        }
-        if (I.cpml_axes & 4u) {
-          if (int rc = encode_psi_map(&p->tmaps[RFXB_MAP_APE + 4 + s], p->adj.aPsiE[s][2], n4, p->ny, p->nx,
-                                      (unsigned)n4, ty + 2, p->l2promo))
-            return rc;
-          if (int rc = encode_psi_map(&p->tmaps[RFXB_MAP_APH + 4 + s], p->adj.aPsiH[s][2], n4, p->ny, p->nx,
-                                      (unsigned)n4, ty + 1, p->l2promo))
-            return rc;
-        }
-      }
-      return 0;
-    };
-    p->adj_psi_maps_ok = enc() == 0;
+  for (int t = 0; t < 2; ++t) {
+    const unsigned tz = kFwdTile[t].tz, ty = kFwdTile[t].ty;
+    CUtensorMap* m = &p->tmaps[RFXB_MAP_AV0 + 6 * t];
+    for (int b = 0; b < 2; ++b) {
+      if (int rc = encode_block_map(m + b, *p, p->adj.aF[b][0], 6, tz + 8, ty + 2, 3)) return rc;
+      if (int rc = encode_block_map(m + 3 + b, *p, p->adj.aF[b][0], 6, tz, ty + 1, 3)) return rc;
+    }
+    if (int rc = encode_block_map(m + 2, *p, p->ca, 3, tz + 8, ty + 2, 1)) return rc;
+    if (int rc = encode_block_map(m + 5, *p, p->ca, 3, tz, ty, 1)) return rc;
   }
   return 0;
 }
 
-// Whether the staged-psi reverse kernel can run a plan: like the forward's
-// test, over the cells its CPML terms touch (rows y0-1 .. y0+TY, columns
-// z0-1 .. z0+32).
-bool adj_psi_staging_ok(const RfxbPlan& p) {
-  const RfxbInst& I = p.inst;
-  if (I.ncp == 0) return true;
-  if (!p.adj_psi_maps_ok || I.ncp4 > 16) return false;
-  for (int a = 0; a < 3; ++a)
-    if (p.psi_elems[a] >= (1LL << 31)) return false;
-  const int n = I.ncp;
-  if (I.cpml_axes & 2u)
-    for (int y0 = 0; y0 < p.ny; y0 += kTY)
-      if (y0 - 1 < n && y0 + kTY >= p.ny - n) return false;
-  if (I.cpml_axes & 4u)
-    for (int z0 = 0; z0 < p.nz; z0 += 32)
-      if (z0 - 1 < n && z0 + 32 >= p.nz - n) return false;
-  return true;
-}
-
-// Reverse kernel variant of a group: 0 with RFXB_STAGING=cpasync, 3 without
-// any CPML, 2 when every plan can stage its psi, else 1; and the ring's
-// z-row capacity.
+// Reverse kernel variant of a group: 0 with RFXB_STAGING=cpasync or when a
+// plan does not suit the four-cells-per-thread kernels, 3 without any CPML, else 2.
 void group_adj_mode(RfxbBatch* g) {
-  g->adj_zp = 4;
-  if (!use_tma()) { g->adj_mode = 0; return; }
-  int mode = 2;
-  bool any_cpml = false;
-  for (auto* p : g->plans) {
-    if (!adj_psi_staging_ok(*p)) mode = 1;
-    if (p->inst.ncp > 0) any_cpml = true;
-    g->adj_zp = std::max(g->adj_zp, p->inst.ncp4);
-  }
-  g->adj_mode = any_cpml ? mode : 3;   // no CPML anywhere: the lean variant
+  g->adj_mode = g->fwd_mode == 0 ? 0 : g->fwd_mode == 1 ? 3 : 2;
 }
 
 using AdjKernel = void (*)(const RfxbInst*, const AdjInst*, const RfxbWork*, const CUtensorMap*, int, int, int, int);
-AdjKernel adj_kernel(int mode) {
-  AdjKernel k = mode == 4   ? adj_step_kernel<kTY, 4>
-                : mode == 3 ? adj_step_kernel<kTY, 3>
-                : mode == 2 ? adj_step_kernel<kTY, 2>
-                : mode == 1 ? adj_step_kernel<kTY, 1>
-                            : adj_step_kernel<kTY, 0>;
-  allow_smem(reinterpret_cast<const void*>(k), adj_step_smem_bytes(mode, 16));
+AdjKernel adj_kernel(int tile, bool cp) {
+  AdjKernel k = tile == 0 ? (cp ? adjv_kernel<24, 8, true> : adjv_kernel<24, 8, false>)
+                          : (cp ? adjv_kernel<8, 8, true> : adjv_kernel<8, 8, false>);
+  allow_smem(reinterpret_cast<const void*>(k), adjv_smem_bytes(tile, cp));
   return k;
+}
+
+void launch_adj(int tile, bool cp, const RfxbBatch* g, const RfxbWork* list, int count, int n, int par, int fpar,
+                cudaStream_t st) {
+  adj_kernel(tile, cp)<<<count, kFwdTile[tile].threads, adjv_smem_bytes(tile, cp), st>>>(
+      g->d_inst, g->d_adj, list, g->d_maps, RFXB_MAP_AV0 + 6 * tile, n, par, fpar);
 }
 
 // Re-encode every TMA map a plan holds with its current L2 promotion (the
 // maps are copied to the device before each launch sequence).
 int reencode_maps(RfxbPlan* p) {
   if (int rc = encode_forward_maps(p)) return rc;
-  if (p->emask)
-    if (int rc = encode_emask_map(p)) return rc;
   if (p->adj_alloc)
     if (int rc = encode_adjoint_maps(p)) return rc;
   return 0;
@@ -1148,11 +1044,11 @@ int build_group(RfxbBatch* g) {
   }
   g->fwd_mode = group_fwd_mode(g);
   if (work_mode() == 1) {
-    make_balanced_work(g->plans, resident_ctas(g->fwd_mode), g->fwd_mode == 2 ? slab_weight() : 1.0, 3.0, work);
+    make_balanced_work(g->plans, 4 * sm_count(), slab_weight(), 3.0, work);
   } else if (work_mode() == 2) {
     make_stream_work(g->plans, stream_planes(), work);
   } else {
-    const int chunks = pick_chunks(tiles, min_nx, resident_ctas(g->fwd_mode));
+    const int chunks = pick_chunks(tiles, min_nx, 4 * sm_count());
     for (size_t q = 0; q < g->plans.size(); ++q) make_work(*g->plans[q], (int)q, chunks, work);
   }
   g->n_work = (int)work.size();
@@ -1162,15 +1058,40 @@ int build_group(RfxbBatch* g) {
     g->allocs.push_back(*ptr);
     return 0;
   };
-  // forward split (variant 2 groups, balanced lists; RFXB_FWD_SPLIT=0 starts
-  // with the single list, which stays available as a launch configuration)
+  // the single-launch forward list
+  if (g->fwd_mode >= 1) {
+    g->vtile = pick_fwd_tile(g);
+    const FwdTile& T = kFwdTile[g->vtile];
+    std::vector<WorkSeg> segs, cpml;
+    split_segments(g->plans, kFwdCost, segs, cpml, T.ty, T.tz);
+    auto merge = [&]() {
+      for (WorkSeg& s : segs) s.inst |= RFXB_WORK_PLAIN;
+      segs.insert(segs.end(), cpml.begin(), cpml.end());
+    };
+    merge();
+    std::vector<RfxbWork> wv;
+    balance_segments(segs, resident_ctas(g->vtile, g->fwd_mode == 2), kFwdPrologue, wv, kFwdWaves);
+    if (int rc = galloc((void**)&g->d_wv, sizeof(RfxbWork) * wv.size())) return rc;
+    RFXB_CUDA(cudaMemcpy(g->d_wv, wv.data(), sizeof(RfxbWork) * wv.size(), cudaMemcpyHostToDevice));
+    g->n_wv = (int)wv.size();
+    segs.clear();
+    cpml.clear();
+    split_adj_segments(g->plans, kAdjCost, segs, cpml, nullptr, T.ty, T.tz);
+    merge();
+    balance_segments(segs, (g->vtile == 0 ? 2 : 5) * sm_count(), kAdjPrologue, wv, kAdjWaves);
+    if (int rc = galloc((void**)&g->d_wva, sizeof(RfxbWork) * wv.size())) return rc;
+    RFXB_CUDA(cudaMemcpy(g->d_wva, wv.data(), sizeof(RfxbWork) * wv.size(), cudaMemcpyHostToDevice));
+    g->n_wva = (int)wv.size();
+  }
+  // forward split (groups with CPML, balanced lists): a launch configuration
+  // (RFXB_FWD_SPLIT=1 starts with it)
   g->fwd_split = false;
   if (g->fwd_mode == 2 && work_mode() == 1) {
     std::vector<WorkSeg> plain, cpml;
     split_segments(g->plans, slab_weight(), plain, cpml);
     std::vector<RfxbWork> w1, w2;
-    balance_segments(plain, resident_ctas(1), 3.0, w1);
-    balance_segments(cpml, resident_ctas(2), 3.0, w2);
+    balance_segments(plain, resident_ctas(1, false), 3.0, w1);
+    balance_segments(cpml, resident_ctas(1, true), 3.0, w2);
     if (!w1.empty() && !w2.empty()) {
       if (int rc = galloc((void**)&g->d_wf1, sizeof(RfxbWork) * w1.size())) return rc;
       if (int rc = galloc((void**)&g->d_wf2, sizeof(RfxbWork) * w2.size())) return rc;
@@ -1184,53 +1105,33 @@ int build_group(RfxbBatch* g) {
       g->fwd_split_avail = true;
       g->fwd_split = fwd_split_enabled();
     }
-    // reverse split (used when the reverse kernel is variant 1 or 2); with
-    // variant 2, the CPML work of tiles that reach no y slab can go to
-    // variant 4 on a third stream
-    std::vector<WorkSeg> aplain, acpml, aplain_b, ay, anoy;
-    split_adj_segments(g->plans, slab_weight(), aplain, acpml);
-    split_adj_segments(g->plans, slab_weight(), aplain_b, ay, &anoy);
-    std::vector<RfxbWork> a1, a2;
-    balance_segments(aplain, 4 * sm_count(), 3.0, a1);
-    balance_segments(acpml, 3 * sm_count(), 3.0, a2);
-    // (a grid with no CPML-free tile, e.g. one whose every z tile reaches a z
-    // slab, still splits its CPML work between variants 2 and 4)
-    if (!a2.empty()) {
-      if (int rc = galloc((void**)&g->d_wa1, sizeof(RfxbWork) * std::max<size_t>(a1.size(), 1))) return rc;
-      if (int rc = galloc((void**)&g->d_wa2, sizeof(RfxbWork) * a2.size())) return rc;
-      if (!a1.empty())
-        RFXB_CUDA(cudaMemcpy(g->d_wa1, a1.data(), sizeof(RfxbWork) * a1.size(), cudaMemcpyHostToDevice));
-      RFXB_CUDA(cudaMemcpy(g->d_wa2, a2.data(), sizeof(RfxbWork) * a2.size(), cudaMemcpyHostToDevice));
-      g->n_wa1 = (int)a1.size();
-      g->n_wa2 = (int)a2.size();
+    // the split reverse lists
+    std::vector<WorkSeg> aplain, ay, anoy;
+    split_adj_segments(g->plans, slab_weight(), aplain, ay, &anoy);
+    std::vector<RfxbWork> a1, a2y, a4;
+    const int res = 5 * sm_count();
+    balance_segments(aplain, res, 3.0, a1);
+    balance_segments(ay, res, 3.0, a2y);
+    balance_segments(anoy, res, 3.0, a4);
+    auto upload = [&](const std::vector<RfxbWork>& v, RfxbWork** d, int* count) -> int {
+      if (int rc = galloc((void**)d, sizeof(RfxbWork) * std::max<size_t>(v.size(), 1))) return rc;
+      if (!v.empty()) RFXB_CUDA(cudaMemcpy(*d, v.data(), sizeof(RfxbWork) * v.size(), cudaMemcpyHostToDevice));
+      *count = (int)v.size();
+      return 0;
+    };
+    if (!a4.empty()) {
+      if (int rc = upload(a1, &g->d_wa1, &g->n_wa1)) return rc;
+      if (int rc = upload(a2y, &g->d_wa2y, &g->n_wa2y)) return rc;
+      if (int rc = upload(a4, &g->d_wa4, &g->n_wa4)) return rc;
       if (!g->side_stream) {
         RFXB_CUDA(cudaStreamCreateWithFlags(&g->side_stream, cudaStreamNonBlocking));
         RFXB_CUDA(cudaEventCreateWithFlags(&g->ev_fork, cudaEventDisableTiming));
         RFXB_CUDA(cudaEventCreateWithFlags(&g->ev_join, cudaEventDisableTiming));
       }
-      g->adj_split = true;
-      std::vector<RfxbWork> a2y, a4;
-      balance_segments(ay, 3 * sm_count(), 3.0, a2y);
-      int zp = 4;
-      for (auto* p : g->plans) zp = std::max(zp, p->inst.ncp4);
-      // resident CTAs of variant 4: three per SM (its launch bounds give it
-      // 80 registers)
-      const int per_sm = 3;
-      balance_segments(anoy, per_sm * sm_count(), 3.0, a4);
-      if (!a4.empty()) {
-        if (!a2y.empty()) {
-          if (int rc = galloc((void**)&g->d_wa2y, sizeof(RfxbWork) * a2y.size())) return rc;
-          RFXB_CUDA(cudaMemcpy(g->d_wa2y, a2y.data(), sizeof(RfxbWork) * a2y.size(), cudaMemcpyHostToDevice));
-        }
-        if (int rc = galloc((void**)&g->d_wa4, sizeof(RfxbWork) * a4.size())) return rc;
-        RFXB_CUDA(cudaMemcpy(g->d_wa4, a4.data(), sizeof(RfxbWork) * a4.size(), cudaMemcpyHostToDevice));
-        g->n_wa2y = (int)a2y.size();
-        g->n_wa4 = (int)a4.size();
-        RFXB_CUDA(cudaStreamCreateWithFlags(&g->side2, cudaStreamNonBlocking));
-        RFXB_CUDA(cudaEventCreateWithFlags(&g->ev_join2, cudaEventDisableTiming));
-        g->adj_lite_avail = true;
-        g->adj_lite = adj_lite_enabled();
-      }
+      RFXB_CUDA(cudaStreamCreateWithFlags(&g->side2, cudaStreamNonBlocking));
+      RFXB_CUDA(cudaEventCreateWithFlags(&g->ev_join2, cudaEventDisableTiming));
+      g->adj_lite_avail = true;
+      g->adj_lite = adj_lite_enabled();
     }
   }
   // two-step pass lists (TMA groups on balanced lists): the two-step tiles
@@ -1244,8 +1145,8 @@ int build_group(RfxbBatch* g) {
     if (!d2.empty()) {
       std::vector<RfxbWork> wd, w1, w2;
       balance_segments(d2, fwd2_resident(), 3.0, wd);
-      balance_segments(plain, resident_ctas(1), 3.0, w1);
-      balance_segments(cpml, resident_ctas(2), 3.0, w2);
+      balance_segments(plain, resident_ctas(1, false), 3.0, w1);
+      balance_segments(cpml, resident_ctas(1, true), 3.0, w2);
       std::vector<RfxbWork2> wd2;
       wd2.reserve(wd.size());
       for (const RfxbWork& w : wd)
@@ -1489,17 +1390,14 @@ void end_parities(const RfxbBatch* g, int n_steps, int& par, int& ppar) {
 // the two-step tiles (F[par] -> F[par^1], intermediate state to F[2] where
 // one-step work reads it), then the one-step work of step n+1
 // (F[2] -> F[par^1], psi pp^1 -> pp).
-int launch_pass(RfxbBatch* g, int n, int par, int pp, bool em, cudaStream_t st) {
+int launch_pass(RfxbBatch* g, int n, int par, int pp, cudaStream_t st) {
   RFXB_CUDA(cudaEventRecord(g->ev_fork, st));
   RFXB_CUDA(cudaStreamWaitEvent(g->side_stream, g->ev_fork, 0));
   RFXB_CUDA(cudaStreamWaitEvent(g->side2, g->ev_fork, 0));
   fwd2_kernel()<<<g->n_wd, dim3(32, kTY), fwd2_step_smem_bytes(), g->side2>>>(g->d_inst, g->d_wd, g->d_maps, n, par);
   if (g->n_wd1 > 0)
-    fwd_kernel(1, em)<<<g->n_wd1, dim3(32, kTY), fwd_step_smem_bytes(1), g->side_stream>>>(
-        g->d_inst, g->d_wd1, g->d_maps, n, step_sel(par, 2, pp));
-  if (g->n_wd2 > 0)
-    fwd_kernel(2, em)<<<g->n_wd2, dim3(32, kTY), fwd_step_smem_bytes(2), st>>>(g->d_inst, g->d_wd2, g->d_maps, n,
-                                                                            step_sel(par, 2, pp));
+    launch_fwd(1, false, g, g->d_wd1, g->n_wd1, n, step_sel(par, 2, pp), g->side_stream);
+  if (g->n_wd2 > 0) launch_fwd(1, true, g, g->d_wd2, g->n_wd2, n, step_sel(par, 2, pp), st);
   RFXB_CUDA(cudaEventRecord(g->ev_join, g->side_stream));
   RFXB_CUDA(cudaEventRecord(g->ev_join2, g->side2));
   RFXB_CUDA(cudaStreamWaitEvent(st, g->ev_join, 0));
@@ -1507,12 +1405,9 @@ int launch_pass(RfxbBatch* g, int n, int par, int pp, bool em, cudaStream_t st) 
   if (g->n_wd1 > 0) {
     RFXB_CUDA(cudaEventRecord(g->ev_fork, st));
     RFXB_CUDA(cudaStreamWaitEvent(g->side_stream, g->ev_fork, 0));
-    fwd_kernel(1, em)<<<g->n_wd1, dim3(32, kTY), fwd_step_smem_bytes(1), g->side_stream>>>(
-        g->d_inst, g->d_wd1, g->d_maps, n + 1, step_sel(2, par ^ 1, pp ^ 1));
+    launch_fwd(1, false, g, g->d_wd1, g->n_wd1, n + 1, step_sel(2, par ^ 1, pp ^ 1), g->side_stream);
   }
-  if (g->n_wd2 > 0)
-    fwd_kernel(2, em)<<<g->n_wd2, dim3(32, kTY), fwd_step_smem_bytes(2), st>>>(g->d_inst, g->d_wd2, g->d_maps, n + 1,
-                                                                            step_sel(2, par ^ 1, pp ^ 1));
+  if (g->n_wd2 > 0) launch_fwd(1, true, g, g->d_wd2, g->n_wd2, n + 1, step_sel(2, par ^ 1, pp ^ 1), st);
   if (g->n_wd1 > 0) {
     RFXB_CUDA(cudaEventRecord(g->ev_join, g->side_stream));
     RFXB_CUDA(cudaStreamWaitEvent(st, g->ev_join, 0));
@@ -1523,8 +1418,6 @@ int launch_pass(RfxbBatch* g, int n, int par, int pp, bool em, cudaStream_t st) 
 int launch_steps(RfxbBatch* g, int step0, int n_steps, int par0, int ppar0, bool has_dft, bool has_flux,
                  bool has_ntff, cudaStream_t st) {
   int par = par0, pp = ppar0;
-  bool em = false;   // stage the PEC edge masks when a plan of the group has one
-  for (auto* p : g->plans) em = em || p->inst.emask != nullptr;
   // per-step observers of the state after step n, held in buffer b
   auto observe = [&](int n, int b) {
     if (has_dft) dft_kernel<<<g->dft_blocks, 256, 0, st>>>(g->d_inst, g->d_dft, (int)g->dft.size(), n, b);
@@ -1537,7 +1430,7 @@ int launch_steps(RfxbBatch* g, int step0, int n_steps, int par0, int ppar0, bool
   for (int s = 0; s < n_steps;) {
     const int n = step0 + s;
     if (two_step(g) && s + 2 <= n_steps) {
-      if (int rc = launch_pass(g, n, par, pp, em, st)) return rc;
+      if (int rc = launch_pass(g, n, par, pp, st)) return rc;
       observe(n, 2);
       observe(n + 1, par ^ 1);
       par ^= 1;
@@ -1556,30 +1449,22 @@ int launch_steps(RfxbBatch* g, int step0, int n_steps, int par0, int ppar0, bool
       Q.plain_ctas = (g->fwd_persist - 1) * sm_count();
       Q.fault_cta = g->fault_cta;
       Q.wait_limit = g->wait_limit;
-      fwd_persist_kernel_for(em)<<<fwd_persist_grid(em), dim3(32, kTY), fwd_step_smem_bytes(2), st>>>(
-          g->d_inst, (int)g->plans.size(), Q, g->d_maps, n, sel);
+      fwdv_persist_kernel<8, 8><<<fwd_persist_grid(), kFwdTile[1].threads, fwdv_smem_bytes(1, true), st>>>(
+          g->d_inst, (int)g->plans.size(), Q, g->d_maps, RFXB_MAP_V0 + 7, n, sel);
     } else if (g->fwd_split) {
-      // staged-psi tiles on the caller's stream, CPML-free tiles beside them
+      // CPML tiles on the caller's stream, CPML-free tiles beside them, in the
+      // capture order fwd_order asks for
       RFXB_CUDA(cudaEventRecord(g->ev_fork, st));
       RFXB_CUDA(cudaStreamWaitEvent(g->side_stream, g->ev_fork, 0));
-      // capture order (fwd_order): by default the plain tiles first
-      // (measured 2 % faster on the sweep's forward phase than the CPML tiles
-      // first, equal on one grid)
-      auto plain = [&]() {
-        fwd_kernel(1, em)<<<g->n_wf1, dim3(32, kTY), fwd_step_smem_bytes(1), g->side_stream>>>(g->d_inst, g->d_wf1,
-                                                                                            g->d_maps, n, sel);
-      };
-      auto staged = [&]() {
-        fwd_kernel(2, em)<<<g->n_wf2, dim3(32, kTY), fwd_step_smem_bytes(2), st>>>(g->d_inst, g->d_wf2, g->d_maps,
-                                                                                n, sel);
-      };
-      if (g->fwd_order == 0) { plain(); staged(); }
-      else { staged(); plain(); }
+      if (g->fwd_order == 0) launch_fwd(1, false, g, g->d_wf1, g->n_wf1, n, sel, g->side_stream);
+      launch_fwd(1, true, g, g->d_wf2, g->n_wf2, n, sel, st);
+      if (g->fwd_order != 0) launch_fwd(1, false, g, g->d_wf1, g->n_wf1, n, sel, g->side_stream);
       RFXB_CUDA(cudaEventRecord(g->ev_join, g->side_stream));
       RFXB_CUDA(cudaStreamWaitEvent(st, g->ev_join, 0));
+    } else if (g->fwd_mode >= 1) {
+      launch_fwd(g->vtile, g->fwd_mode == 2, g, g->d_wv, g->n_wv, n, sel, st);
     } else {
-      fwd_kernel(g->fwd_mode, em)<<<g->n_work, dim3(32, kTY), fwd_step_smem_bytes(g->fwd_mode), st>>>(
-          g->d_inst, g->d_work, g->d_maps, n, sel);
+      launch_fwd_generic(g, n, sel, st);
     }
     observe(n, par ^ 1);
     par ^= 1;
@@ -1658,7 +1543,7 @@ int group_advance(RfxbBatch* g, const RfxbStepIO* ios, int step0, int n_steps, c
   // work, and their captured graphs measured slower to build and to replay
   // (1000 steps of a 513^3 grid: 0.9 s to capture, 1.58 s against 1.49 s per
   // replay)
-  if (graphs_enabled() && n_steps >= 4 && !two_step(g)) {
+if (graphs_enabled() && n_steps >= 4 && !two_step(g)) {
     const GraphKey key{0, step0, n_steps, par0, 0, (has_dft ? 1 : 0) | (has_flux ? 2 : 0) | (has_ntff ? 4 : 0),
                        ppar0};
     if (int rc = run_graph(g, key, st, [&](cudaStream_t cs) {
@@ -1678,15 +1563,6 @@ int group_advance(RfxbBatch* g, const RfxbStepIO* ios, int step0, int n_steps, c
 }
 
 bool adj_persist_avail(const RfxbBatch* g) { return g->adj_lite_avail && g->n_wa4 > 0 && g->n_wa1 > 0; }
-
-using AdjPersistKernel = void (*)(const RfxbInst*, const AdjInst*, int, RfxbAdjQueues, const CUtensorMap*, int, int,
-                                  int);
-AdjPersistKernel adj_persist_kernel_for(int zp) {
-  AdjPersistKernel k = adj_persist_kernel<kTY>;
-  allow_smem(reinterpret_cast<const void*>(k), adj_step_smem_bytes(5, 16));
-  (void)zp;
-  return k;
-}
 
 int ensure_adjoint(RfxbPlan* p, cudaStream_t st) {
   if (!p->adj_alloc) {
@@ -1832,19 +1708,17 @@ int group_adjoint_advance(RfxbBatch* g, const RfxbAdjointIO* aios, int step_hi, 
   if (int rc = upload_adjoint(g, aios, st)) return rc;
   const bool two = use_twopass();
   if (g->adj_mode < 0) group_adj_mode(g);
-  const int amode = g->adj_mode, zp = g->adj_zp;
-  AdjKernel akern = two ? nullptr : adj_kernel(amode);
-  const size_t asmem = adj_step_smem_bytes(amode, zp);
+  const int amode = g->adj_mode;
   auto launch = [&](cudaStream_t cs) -> int {
     int par = par0, fpar = fpar0;
-    if (g->adj_persist && amode == 2 && adj_persist_avail(g))
-      RFXB_CUDA(cudaMemsetAsync(g->d_qctr + 4, 0, 4 * sizeof(int), cs));
+    const bool persist = g->adj_persist && amode == 2 && adj_persist_avail(g);
+    if (persist) RFXB_CUDA(cudaMemsetAsync(g->d_qctr + 4, 0, 4 * sizeof(int), cs));
     for (int s = step_hi - 1; s >= step_hi - n_steps; --s) {
       if (two) {
         adj_pass_a<<<g->n_work, dim3(32, kTY), 0, cs>>>(g->d_inst, g->d_adj, g->d_work, s, par, fpar);
         adj_pass_b<<<g->n_work, dim3(32, kTY), 0, cs>>>(g->d_inst, g->d_adj, g->d_work, s, par, fpar);
       } else {
-        if (g->adj_persist && amode == 2 && adj_persist_avail(g)) {
+        if (persist) {
           RfxbAdjQueues Q{};
           Q.list[0] = g->d_wa2y;
           Q.count[0] = g->n_wa2y;
@@ -1857,65 +1731,43 @@ int group_adjoint_advance(RfxbBatch* g, const RfxbAdjointIO* aios, int step_hi, 
           Q.role_ctas = sm_count();
           Q.fault_cta = g->fault_cta;
           Q.wait_limit = g->wait_limit;
-          Q.zp = zp;
-          const size_t psmem = adj_step_smem_bytes(5, zp);
-          AdjPersistKernel pk = adj_persist_kernel_for(zp);
+          const size_t psmem = adjv_smem_bytes(1, true);
+          const auto pk = adjv_persist_kernel<8, 8>;
           if (g->adj_persist_grid <= 0) {
+            allow_smem(reinterpret_cast<const void*>(pk), psmem);
             int per_sm = 0;
-            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pk, 32 * kTY, psmem) != cudaSuccess || per_sm < 1)
+            if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pk, kFwdTile[1].threads, psmem) != cudaSuccess ||
+                per_sm < 1)
               per_sm = 1;
             g->adj_persist_grid = per_sm * sm_count();
           }
-          pk<<<g->adj_persist_grid, dim3(32, kTY), psmem, cs>>>(g->d_inst, g->d_adj, (int)g->plans.size(), Q,
-                                                               g->d_maps, s, par, fpar);
-        } else if (g->adj_split && amode != 0) {
-          // CPML tiles on the caller's stream, plain tiles beside them, and
-          // (variant 2 groups) the CPML work without a y slab on variant 4
-          const bool lite = g->adj_lite && amode == 2;
+          pk<<<g->adj_persist_grid, kFwdTile[1].threads, psmem, cs>>>(g->d_inst, g->d_adj, (int)g->plans.size(), Q,
+                                                                     g->d_maps, RFXB_MAP_AV0 + 6, s, par, fpar);
+        } else if (amode == 0) {
+          allow_smem(reinterpret_cast<const void*>(adj_step_kernel), adj_step_smem_bytes());
+          adj_step_kernel<<<g->n_work, dim3(32, kTY), adj_step_smem_bytes(), cs>>>(g->d_inst, g->d_adj, g->d_work, s, par,
+                                                                                 fpar);
+        } else if (g->adj_lite) {
+          // y-slab tiles on the caller's stream, the other CPML work and the
+          // CPML-free tiles beside them, in the capture order adj_order asks
+          // for (a, b, c of rfxb200.h: 4 the other CPML work, 2 y-slab tiles,
+          // 3 CPML-free tiles)
           RFXB_CUDA(cudaEventRecord(g->ev_fork, cs));
           RFXB_CUDA(cudaStreamWaitEvent(g->side_stream, g->ev_fork, 0));
-          auto v2 = [&]() {
-            if (lite) {
-              if (g->n_wa2y > 0)
-                akern<<<g->n_wa2y, dim3(32, kTY), asmem, cs>>>(g->d_inst, g->d_adj, g->d_wa2y, g->d_maps, s, par,
-                                                               fpar, zp);
-            } else {
-              akern<<<g->n_wa2, dim3(32, kTY), asmem, cs>>>(g->d_inst, g->d_adj, g->d_wa2, g->d_maps, s, par, fpar,
-                                                            zp);
-            }
-          };
-          auto v4 = [&]() {
-            if (lite)
-              adj_kernel(4)<<<g->n_wa4, dim3(32, kTY), adj_step_smem_bytes(4, zp), g->side2>>>(
-                  g->d_inst, g->d_adj, g->d_wa4, g->d_maps, s, par, fpar, zp);
-          };
-          auto v3 = [&]() {
-            if (g->n_wa1 > 0)
-              adj_kernel(3)<<<g->n_wa1, dim3(32, kTY), adj_step_smem_bytes(3, zp), g->side_stream>>>(
-                  g->d_inst, g->d_adj, g->d_wa1, g->d_maps, s, par, fpar, zp);
-          };
-          // capture order = the order the graph hands the branches' CTAs to
-          // the SMs (adj_order); the default 0 puts the largest, four-per-SM
-          // variant 4 first, then the y-slab variant 2, the plain variant 3
-          // last (measured best of the six orders, 3 % on the sweep's
-          // reverse phase)
-          if (lite) RFXB_CUDA(cudaStreamWaitEvent(g->side2, g->ev_fork, 0));
+          RFXB_CUDA(cudaStreamWaitEvent(g->side2, g->ev_fork, 0));
           static const char kOrder[6][3] = {{4, 2, 3}, {4, 3, 2}, {2, 4, 3}, {2, 3, 4}, {3, 4, 2}, {3, 2, 4}};
           for (int t = 0; t < 3; ++t) {
             const int v = kOrder[g->adj_order][t];
-            if (v == 4) v4();
-            else if (v == 2) v2();
-            else v3();
+            if (v == 4) launch_adj(1, true, g, g->d_wa4, g->n_wa4, s, par, fpar, g->side2);
+            else if (v == 2 && g->n_wa2y > 0) launch_adj(1, true, g, g->d_wa2y, g->n_wa2y, s, par, fpar, cs);
+            else if (v == 3 && g->n_wa1 > 0) launch_adj(1, false, g, g->d_wa1, g->n_wa1, s, par, fpar, g->side_stream);
           }
           RFXB_CUDA(cudaEventRecord(g->ev_join, g->side_stream));
           RFXB_CUDA(cudaStreamWaitEvent(cs, g->ev_join, 0));
-          if (lite) {
-            RFXB_CUDA(cudaEventRecord(g->ev_join2, g->side2));
-            RFXB_CUDA(cudaStreamWaitEvent(cs, g->ev_join2, 0));
-          }
+          RFXB_CUDA(cudaEventRecord(g->ev_join2, g->side2));
+          RFXB_CUDA(cudaStreamWaitEvent(cs, g->ev_join2, 0));
         } else {
-          akern<<<g->n_work, dim3(32, kTY), asmem, cs>>>(g->d_inst, g->d_adj, g->d_work, g->d_maps, s, par, fpar,
-                                                         zp);
+          launch_adj(g->vtile, amode == 2, g, g->d_wva, g->n_wva, s, par, fpar, cs);
         }
         fpar ^= 1;
       }
@@ -2177,7 +2029,6 @@ int rfxb_plan_set_materials(RfxbPlan* p, const float* eps_r, const float* sigma,
   if (edge_mask && !p->emask) {
     if (int rc = p->alloc(&p->emask, p->elems)) return rc;
     RFXB_CUDA(cudaMemsetAsync(p->emask, 0, p->elems, st));
-    if (int rc = encode_emask_map(p)) return rc;
   }
   p->inst.emask = edge_mask ? p->emask : nullptr;
   const long long cells = (long long)p->nx * p->ny * p->nz;
@@ -2539,8 +2390,8 @@ void step_launches(const RfxbBatch* g, int* fwd, int* rev) {
     if (g->adj_mode < 0) *rev = -1;
     else if (use_twopass()) *rev = 2;
     else if (g->adj_persist && g->adj_mode == 2 && adj_persist_avail(g)) *rev = 1;
-    else if (g->adj_split && g->adj_mode != 0)
-      *rev = ((g->adj_lite && g->adj_mode == 2) ? (g->n_wa2y > 0 ? 3 : 2) : 2) - (g->n_wa1 > 0 ? 0 : 1);
+    else if (g->adj_lite && g->adj_mode == 2)
+      *rev = 1 + (g->n_wa2y > 0 ? 1 : 0) + (g->n_wa1 > 0 ? 1 : 0);
     else *rev = 1;
   }
 }
@@ -2565,7 +2416,7 @@ void launch_config(const RfxbBatch* g, RfxbLaunchConfig* cur, RfxbLaunchConfig* 
                             g->adj_persist, g->plans[0]->l2promo, g->fwd_depth};
   if (lim)
     *lim = RfxbLaunchConfig{g->fwd_split_avail ? 1 : 0, g->fwd_split_avail ? 1 : 0, g->adj_lite_avail ? 1 : 0,
-                            g->adj_split ? 5 : 0, g->fwd_split_avail ? 3 : 0, adj_persist_avail(g) ? 1 : 0, 3, g->fwd_depth_avail ? 2 : 1};
+                            g->adj_lite_avail ? 5 : 0, g->fwd_split_avail ? 3 : 0, adj_persist_avail(g) ? 1 : 0, 3, g->fwd_depth_avail ? 2 : 1};
 }
 
 int set_launch_config(RfxbBatch* g, const RfxbLaunchConfig* c) {

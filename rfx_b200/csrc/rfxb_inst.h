@@ -19,39 +19,25 @@
 
 #define RFXB_TZ 32          // tile extent along z (one warp)
 #define RFXB_MAXC 6
-// TMA descriptors per instance: [0|1] fields parity 0|1 with the E box,
-// [2|3] with the H box, [4] coefficients with the ca/cb box, [5|6] adjoint
-// fields with the E box, [7|8] with the H box, [9] cb with the E box,
-// [10] one coefficient with the tile box, then the CPML psi of parity 0|1:
-// [11|12] H-side x, [13|14] H-side y, [15|16] H-side z (H boxes), [17|18]
-// E-side x, [19|20] E-side y, [21|22] E-side z (tile boxes); [23] one
-// coefficient with the H box; then the adjoint psi of parity 0|1: [24|25]
-// E-side x (H box), [26|27] E-side y (E box), [28|29] E-side z (E rows),
-// [30|31] H-side x (tile box), [32|33] H-side y (H box), [34|35] H-side z
-// (H rows); [36] the PEC edge-mask bytes with the tile box; [37] the
-// intermediate field state of a two-step pass with the E box, [38] with the
-// H box; the two-step kernel's boxes: [39|40] fields parity 0|1 with the
-// two-step E box, [41|42] with the two-step H box, [43] coefficients with the
-// two-step ca/cb box.
-#define RFXB_NMAPS 44
-#define RFXB_MAP_EMASK 36   // PEC edge mask bytes with the tile box
-#define RFXB_MAP_MIDE 37
-#define RFXB_MAP_MIDH 38
-#define RFXB_MAP_E2 39
-#define RFXB_MAP_H2 41
-#define RFXB_MAP_C2 43
-#define RFXB_MAP_PSH 11
-#define RFXB_MAP_PSE 17
-#define RFXB_MAP_APE 24
-#define RFXB_MAP_APH 30
+// TMA descriptors per instance.  For each of the step kernels' two tile shapes
+// (shape 0: 24 x 32 cells, shape 1: 8 x 32): the E box (one-cell halo) of forward
+// field buffers 0, 1, 2, the H box (low row) of the same buffers, the ca/cb box;
+// then the E box of the adjoint field buffers 0, 1 and of cb, the H box of the
+// adjoint buffers, the ca box.  Last the two-step kernel's boxes (two-cell halo):
+// E and H of field buffers 0, 1 and ca/cb.
+#define RFXB_MAP_V0 0       // + 7 * tile shape + (buffer | 3 + buffer | 6)
+#define RFXB_MAP_AV0 14     // + 6 * tile shape + (adjoint buffer | 2: cb | 3 + adjoint buffer | 5: ca)
+#define RFXB_MAP_E2 26
+#define RFXB_MAP_H2 28
+#define RFXB_MAP_C2 30
+#define RFXB_NMAPS 31
 
 // CPML psi layout per axis (q = which of the two corrected components,
 // n = layers, n4 = n rounded up to a multiple of 4):
 //   x: ((side*2 + q)*n + s)*ny*zs + j*zs + k
 //   y: ((side*2 + q)*nx + i)*n*zs + s*zs + k
 //   z: ((side*2 + q)*nx + i)*ny*n4 + j*n4 + s
-// Every row is a multiple of 16 bytes, so each axis is a TMA-tileable 4-D
-// array (rows along k for x and y, along s for z).
+// Every row is a multiple of 16 bytes (rows along k for x and y, along s for z).
 struct RfxbInst {
   int nx, ny, nz, zs;
   long long ps;            // plane stride (elements)
@@ -112,6 +98,7 @@ struct AdjInst {           // adjoint state of one instance (same layouts as the
   float* aPsiE[2][3];
 };
 
+#define RFXB_WORK_PLAIN (1 << 24)   // in RfxbWork::inst: no cell of the item needs a CPML term
 struct RfxbWork {          // one CTA: a (y, z) tile over an x range
   int inst;
   int y0, z0;
@@ -134,9 +121,10 @@ struct RfxbWork2 {
   int mid;
 };
 
+
 // Work queues of the persistent forward step (one launch per step).
 struct RfxbFwdQueues {
-  const RfxbWork* list[2];   // 0: tiles that reach a CPML slab (staged psi), 1: CPML-free tiles
+  const RfxbWork* list[2];   // 0: tiles that reach a CPML slab, 1: CPML-free tiles
   int count[2];
   int* ctr;                  // [3]: fetch counters of the two lists, CTAs finished (zero between launches)
   int* status;               // the group's status word (bit 1: a wait ran out, bit 2: an invalid item)
@@ -145,8 +133,8 @@ struct RfxbFwdQueues {
   int wait_limit;            // polls of a bounded mbarrier wait
 };
 
-// Work queues of the persistent reverse step: 0 tiles that reach a y slab
-// (variant 2), 1 the other CPML work (variant 4), 2 CPML-free tiles (variant 3).
+// Work queues of the persistent reverse step: 0 tiles that reach a y slab, 1
+// the other CPML work, 2 CPML-free tiles.
 struct RfxbAdjQueues {
   const RfxbWork* list[3];
   int count[3];
@@ -155,7 +143,6 @@ struct RfxbAdjQueues {
   int role_ctas;             // CTAs per role: blocks [r * role_ctas, (r+1) * role_ctas) have role r
   int fault_cta;
   int wait_limit;
-  int zp;                    // largest z-psi row of the group (ring slot size)
 };
 
 struct RfxbNtffFace {      // one face of one instance's NTFF box

@@ -41,9 +41,8 @@
 #include "rfxb_common.cuh"
 
 namespace rfxb {
-template <int TY, int MODE, bool EM>
-__global__ void fwd_step_kernel(const RfxbInst*, const RfxbWork*, const CUtensorMap*, int, int);
-size_t fwd_step_smem_bytes(int mode);
+__global__ void fwd_step_kernel(const RfxbInst*, const RfxbWork*, int, int);
+size_t fwd_step_smem_bytes();
 __global__ void pack_kernel(float*, const float*, RfxbInst);
 __global__ void unpack_kernel(float*, const float*, RfxbInst);
 __global__ void coef_kernel(RfxbInst, float*, float*, float*, float*, const float*, const float*, const float*,
@@ -85,9 +84,9 @@ unsigned char* scratch_address(int* rc) {
     std::lock_guard<std::mutex> lock(mu);
     a = addr[dev].load(std::memory_order_relaxed);
     if (!a) {
-      const cudaError_t ea = cudaFuncSetAttribute(reinterpret_cast<const void*>(fwd_step_kernel<8, 0, false>),
+      const cudaError_t ea = cudaFuncSetAttribute(reinterpret_cast<const void*>(fwd_step_kernel),
                                                   cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                  (int)fwd_step_smem_bytes(0));
+                                                  (int)fwd_step_smem_bytes());
       if (ea != cudaSuccess) {
         *rc = noalloc_fail(RFXB_E_LAUNCH, "rfxb_forward_noalloc: raising the step kernel's shared-memory limit failed");
         return nullptr;
@@ -317,8 +316,8 @@ extern "C" int rfxb_forward_noalloc(const RfxbDesc* d, const float* eps_r_dev, c
   const RfxbWork* dW = reinterpret_cast<const RfxbWork*>(base + o_work);
   int par = 0;
   for (int s = 0; s < n_steps; ++s) {
-    fwd_step_kernel<TY, 0, false><<<(unsigned)n_work, dim3(32, TY), fwd_step_smem_bytes(0), st>>>(dI, dW, nullptr, step0 + s,
-                                                                                           step_sel(par, par ^ 1, par));
+    fwd_step_kernel<<<(unsigned)n_work, dim3(32, TY), fwd_step_smem_bytes(), st>>>(dI, dW, step0 + s,
+                                                                                step_sel(par, par ^ 1, par));
     par ^= 1;
   }
   for (int c = 0; c < 6; ++c) unpack_kernel<<<blocks, 256, 0, st>>>(fields_dev[c], I.F[par][c], I);
