@@ -81,7 +81,7 @@ struct VSlab {
 
 // psi' = b psi + c g
 __device__ __forceinline__ float psi_next(float b, float psi, float c, float g) {
-  return __fmaf_rn(b, psi, __fmul_rn(c, g));
+  return __fmaf_rn(c, g, __fmul_rn(b, psi));
 }
 // f + s (psi' + km g), the two terms added one after the other
 __device__ __forceinline__ float psi_add(float f, float s, float p, float km, float g) {
