@@ -54,6 +54,8 @@ __global__ void fwdv_kernel(const RfxbInst*, const RfxbWork*, const CUtensorMap*
 template <int TY, int ZQ>
 __global__ void fwdv_persist_kernel(const RfxbInst*, int, RfxbFwdQueues, const CUtensorMap*, int, int, int);
 size_t fwdv_smem_bytes(int tile, bool cp);
+__global__ void fwd_resident_kernel(const RfxbInst*, ResidentShape, int, int, int, int, unsigned*, int);
+size_t resident_smem_bytes(const ResidentShape&, int n_axes);
 size_t adj_step_smem_bytes();
 template <int TY>
 __global__ void fwd2_step_kernel(const RfxbInst*, const RfxbWork2*, const CUtensorMap*, int, int);
@@ -179,6 +181,10 @@ struct RfxbBatch {
   int n_wv = 0;
   // forward steps split between the CPML-free tiles (list 1) and the others
   // (list 2), launched side by side on two streams
+  // all steps of an advance in one launch (small single plans; rfxb_resident.cu)
+  ResidentShape res{};
+  size_t res_smem = 0;
+  unsigned* d_resctr = nullptr;    // arrivals at the grid barrier
   bool fwd_split = false;
   bool fwd_split_avail = false;   // both forward lists exist (fwd_split may be chosen)
   int fwd_order = 0;              // split forward: 0 plain-tile launch first, 1 CPML-tile launch first
@@ -859,6 +865,56 @@ int resident_ctas(int tile, bool cp) {
   return r[tile][cp];
 }
 
+// Block partition of the resident forward kernel for one plan: at most one
+// block per SM, the cheapest one (cells computed per step, shell cells read at
+// half weight) whose state fits the shared memory of an SM.
+ResidentShape resident_shape(const RfxbPlan& p, int sms, size_t smem_max, size_t* smem) {
+  ResidentShape best{};
+  const int n[3] = {p.nx, p.ny, p.nz};
+  const unsigned ax = p.inst.ncp > 0 ? p.inst.cpml_axes : 0u;
+  const int na = (int)(ax & 1u) + (int)((ax >> 1) & 1u) + (int)((ax >> 2) & 1u);
+  int dev = 0, coop = 0;
+  cudaGetDevice(&dev);
+  if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop) return best;
+  if ((long long)n[0] * n[1] * n[2] > (long long)sms * 4096) return best;
+  double best_cost = 1e300;
+  for (int c0 = 1; c0 <= std::min(sms, n[0]); ++c0) {
+    const int b0 = (n[0] + c0 - 1) / c0;
+    if (b0 > 61 || (n[0] + b0 - 1) / b0 != c0) continue;
+    for (int c1 = 1; c0 * c1 <= sms && c1 <= n[1]; ++c1) {
+      const int b1 = (n[1] + c1 - 1) / c1;
+      if (b1 > 61 || (n[1] + b1 - 1) / b1 != c1) continue;
+      const int c2_max = std::min(sms / (c0 * c1), n[2]);
+      for (int c2 = 1; c2 <= c2_max; ++c2) {
+        const int b2 = (n[2] + c2 - 1) / c2;
+        if (b2 > 61 || (n[2] + b2 - 1) / b2 != c2) continue;
+        const ResidentShape R{{c0, c1, c2}, {b0, b1, b2}};
+        const size_t bytes = resident_smem_bytes(R, na);
+        if (bytes > smem_max) continue;
+        const double own = (double)b0 * b1 * b2, h = (b0 + 1.0) * (b1 + 1.0) * (b2 + 1.0);
+        const double cost = own + h + 0.5 * ((b0 + 2.0) * (b1 + 2.0) * (b2 + 2.0) - own);
+        if (cost < best_cost) {
+          best_cost = cost;
+          best = R;
+          *smem = bytes;
+        }
+      }
+    }
+  }
+  return best;
+}
+
+// Shared memory one block may use (opt-in).
+size_t smem_optin() {
+  static int n = -1;
+  if (n < 0) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (cudaDeviceGetAttribute(&n, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) n = 0;
+  }
+  return (size_t)n;
+}
+
 // TMA staging is the default; RFXB_STAGING=cpasync selects per-thread 16-byte
 // cp.async staging of the same planes.
 bool use_tma() {
@@ -1058,6 +1114,11 @@ int build_group(RfxbBatch* g) {
     g->allocs.push_back(*ptr);
     return 0;
   };
+  if (g->fwd_mode >= 1 && g->plans.size() == 1) {
+    g->res = resident_shape(*g->plans[0], sm_count(), smem_optin() - 1024, &g->res_smem);
+    if (g->res.nb[0] > 0)
+      if (int rc = galloc((void**)&g->d_resctr, sizeof(unsigned))) return rc;
+  }
   // the single-launch forward list
   if (g->fwd_mode >= 1) {
     g->vtile = pick_fwd_tile(g);
@@ -1475,6 +1536,33 @@ int launch_steps(RfxbBatch* g, int step0, int n_steps, int par0, int ppar0, bool
   return 0;
 }
 
+// Whether an advance runs in one launch of the resident kernel: a small single
+// plan on the default launch configuration, without per-step observers, history
+// recording or per-cell mu_r.
+bool resident_route(const RfxbBatch* g, bool observers, int step0, int n_steps, cudaStream_t st) {
+  const long long blocks = (long long)g->res.nb[0] * g->res.nb[1] * g->res.nb[2];
+  if (blocks == 0 || observers || n_steps < 2 || blocks * n_steps > INT_MAX) return false;
+  if (g->fwd_split || g->fwd_persist > 0 || two_step(g)) return false;
+  const RfxbPlan* p = g->plans[0];
+  const RfxbInst& I = p->inst;
+  if (I.ch) return false;
+  if (I.hist && I.hist_step0 < step0 + n_steps && I.hist_step0 + I.hist_nsteps > step0) return false;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;   // a caller's capture keeps its step launches
+  return cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
+}
+
+int launch_resident(RfxbBatch* g, int step0, int n_steps, int par0, int ppar0, cudaStream_t st) {
+  const void* k = reinterpret_cast<const void*>(fwd_resident_kernel);
+  allow_smem(k, smem_optin() - 1024);
+  RFXB_CUDA(cudaMemsetAsync(g->d_resctr, 0, sizeof(unsigned), st));
+  const RfxbInst* inst = g->d_inst;
+  int limit = g->wait_limit;
+  void* args[] = {&inst, &g->res, &step0, &n_steps, &par0, &ppar0, &g->d_resctr, &limit};
+  RFXB_CUDA(cudaLaunchCooperativeKernel(k, dim3(g->res.nb[0] * g->res.nb[1] * g->res.nb[2]), dim3(RFXB_RES_THREADS),
+                                        args, g->res_smem, st));
+  return 0;
+}
+
 // Launch sequences of more than a few steps are captured once into a CUDA
 // graph (keyed by step range and parities) and replayed; the descriptors the
 // kernels read are uploaded before each replay.  RFXB_GRAPHS=0 disables it.
@@ -1543,7 +1631,9 @@ int group_advance(RfxbBatch* g, const RfxbStepIO* ios, int step0, int n_steps, c
   // work, and their captured graphs measured slower to build and to replay
   // (1000 steps of a 513^3 grid: 0.9 s to capture, 1.58 s against 1.49 s per
   // replay)
-if (graphs_enabled() && n_steps >= 4 && !two_step(g)) {
+  if (resident_route(g, has_dft || has_flux || has_ntff, step0, n_steps, st)) {
+    if (int rc = launch_resident(g, step0, n_steps, par0, ppar0, st)) return rc;
+  } else if (graphs_enabled() && n_steps >= 4 && !two_step(g)) {
     const GraphKey key{0, step0, n_steps, par0, 0, (has_dft ? 1 : 0) | (has_flux ? 2 : 0) | (has_ntff ? 4 : 0),
                        ppar0};
     if (int rc = run_graph(g, key, st, [&](cudaStream_t cs) {

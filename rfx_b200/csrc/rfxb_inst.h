@@ -121,6 +121,13 @@ struct RfxbWork2 {
   int mid;
 };
 
+#define RFXB_RES_THREADS 512   // threads of a block of the resident forward kernel
+// Block partition of the resident forward kernel: blocks per axis and cells of
+// the largest block per axis (nb = 0: the plan does not fit).
+struct ResidentShape {
+  int nb[3];
+  int b[3];
+};
 
 // Work queues of the persistent forward step (one launch per step).
 struct RfxbFwdQueues {
