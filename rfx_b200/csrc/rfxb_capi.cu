@@ -57,7 +57,6 @@ size_t fwdv_smem_bytes(int tile, bool cp);
 __global__ void fwd_resident_kernel(const RfxbInst*, ResidentShape, int, int, int, int, unsigned*, int);
 size_t resident_smem_bytes(const ResidentShape&, int n_axes);
 size_t adj_step_smem_bytes();
-template <int TY>
 __global__ void fwd2_step_kernel(const RfxbInst*, const RfxbWork2*, const CUtensorMap*, int, int);
 size_t fwd2_step_smem_bytes();
 }  // namespace rfxb
@@ -639,6 +638,61 @@ int depth2_mid_flags(const RfxbPlan& p, const RfxbWork& w) {
   return mid;
 }
 
+// The two-step kernel's items: the 8 x 32 columns of the two-step segments (d2)
+// merged into rectangles (rows first, as long as every column of the row is
+// there) and cut into pieces of at most 13 rows x 56 columns, which the kernel's
+// 16 x 64 cells per plane can store; their x ranges balanced.
+void depth2_items(const std::vector<RfxbPlan*>& plans, const std::vector<WorkSeg>& d2, int resident,
+                  std::vector<RfxbWork2>& out) {
+  constexpr int kRows = RFXB_D2ROWS - 3, kCols = RFXB_D2COLS - 8;
+  std::map<std::tuple<int, int, int>, std::set<std::pair<int, int>>> groups;   // (plan, xa, xb) -> columns
+  for (const WorkSeg& s : d2) groups[{s.inst, s.xa, s.xb}].insert({s.y0, s.z0});
+  std::vector<WorkSeg> segs;
+  std::map<std::tuple<int, int, int>, std::pair<int, int>> ends;   // (plan, y0, z0) -> (yb, zb)
+  for (auto& [key, cols] : groups) {
+    const auto [inst, xa, xb] = key;
+    const RfxbPlan& p = *plans[inst];
+    while (!cols.empty()) {
+      const auto [y0, z0] = *cols.begin();
+      int ze = z0, ye = y0;
+      while (cols.count({y0, ze})) ze += 32;
+      auto row = [&](int y) {
+        for (int z = z0; z < ze; z += 32)
+          if (!cols.count({y, z})) return false;
+        return true;
+      };
+      while (row(ye)) {
+        for (int z = z0; z < ze; z += 32) cols.erase({ye, z});
+        ye += kTY;
+      }
+      ye = std::min(ye, p.ny);
+      ze = std::min(ze, p.nz);
+      const int my = (ye - y0 + kRows - 1) / kRows, mz = (ze - z0 + kCols - 1) / kCols;
+      const int dz = ((ze - z0 + mz - 1) / mz + 3) / 4 * 4;
+      for (int a = 0; a < my; ++a) {
+        const int ya = y0 + (ye - y0) * a / my, yb = y0 + (ye - y0) * (a + 1) / my;
+        for (int z = z0; z < ze; z += dz) {
+          segs.push_back(WorkSeg{inst, ya, z, xa, xb, p.nx, 0, 1.0, 0.0});
+          ends[{inst, ya, z}] = {yb, std::min(z + dz, ze)};
+        }
+      }
+    }
+  }
+  std::vector<RfxbWork> items;
+  balance_segments(segs, resident, 2.0, items);
+  out.clear();
+  for (const RfxbWork& w : items) {
+    const RfxbPlan& p = *plans[w.inst];
+    const auto [yb, zb] = ends[{w.inst, w.y0, w.z0}];
+    int mid = 0;
+    for (int y = w.y0 / kTY * kTY; y < yb; y += kTY)
+      for (int z = w.z0 / 32 * 32; z < zb; z += 32) mid |= depth2_mid_flags(p, RfxbWork{w.inst, y, z, w.xa, w.xb});
+    mid &= ~RFXB_MID_EDGE;
+    if (w.y0 < 2 || yb > p.ny - 2 || w.z0 < 2 || zb > p.nz - 2 || w.xa < 2 || w.xb > p.nx - 2) mid |= RFXB_MID_EDGE;
+    out.push_back(RfxbWork2{w.inst, w.y0, yb, w.z0, zb, w.xa, w.xb, mid});
+  }
+}
+
 void make_balanced_work(const std::vector<RfxbPlan*>& plans, int resident, double slab, double prologue,
                         std::vector<RfxbWork>& out) {
   std::vector<WorkSeg> segs;
@@ -784,9 +838,10 @@ int pick_fwd_tile(const RfxbBatch* g) {
 }
 
 // The two-step kernel with its dynamic shared memory enabled.
+constexpr int kFwd2Threads = RFXB_D2ROWS * RFXB_D2COLS / 4;
 using Fwd2Kernel = void (*)(const RfxbInst*, const RfxbWork2*, const CUtensorMap*, int, int);
 Fwd2Kernel fwd2_kernel() {
-  Fwd2Kernel k = fwd2_step_kernel<kTY>;
+  Fwd2Kernel k = fwd2_step_kernel;
   allow_smem(reinterpret_cast<const void*>(k), fwd2_step_smem_bytes());
   return k;
 }
@@ -796,7 +851,7 @@ int fwd2_resident() {
   static int r = -1;
   if (r < 0) {
     int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fwd2_kernel(), 32 * kTY, fwd2_step_smem_bytes()) !=
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fwd2_kernel(), kFwd2Threads, fwd2_step_smem_bytes()) !=
             cudaSuccess ||
         per_sm < 1)
       per_sm = 2;
@@ -997,10 +1052,10 @@ int encode_forward_maps(RfxbPlan* p) {
   }
   // the two-step kernel's boxes (two-cell halo)
   for (int s = 0; s < 2; ++s) {
-    if (int rc = encode_block_map(&p->tmaps[RFXB_MAP_E2 + s], *p, p->inst.F[s][0], 6, 40, ty + 4, 3)) return rc;
-    if (int rc = encode_block_map(&p->tmaps[RFXB_MAP_H2 + s], *p, p->inst.F[s][0], 6, 40, ty + 3, 3)) return rc;
+    if (int rc = encode_block_map(&p->tmaps[RFXB_MAP_E2 + s], *p, p->inst.F[s][0], 6, RFXB_D2COLS, RFXB_D2ROWS + 1, 3)) return rc;
+    if (int rc = encode_block_map(&p->tmaps[RFXB_MAP_H2 + s], *p, p->inst.F[s][0], 6, RFXB_D2COLS, RFXB_D2ROWS, 3)) return rc;
   }
-  if (int rc = encode_block_map(&p->tmaps[RFXB_MAP_C2], *p, p->ca, 3, 40, ty + 2, 2)) return rc;
+  if (int rc = encode_block_map(&p->tmaps[RFXB_MAP_C2], *p, p->ca, 3, RFXB_D2COLS, RFXB_D2ROWS, 2)) return rc;
   return 0;
 }
 
@@ -1204,14 +1259,11 @@ int build_group(RfxbBatch* g) {
     std::vector<WorkSeg> d2, plain, cpml;
     split_depth2_segments(g->plans, slab_weight(), d2, plain, cpml);
     if (!d2.empty()) {
-      std::vector<RfxbWork> wd, w1, w2;
-      balance_segments(d2, fwd2_resident(), 3.0, wd);
+      std::vector<RfxbWork> w1, w2;
       balance_segments(plain, resident_ctas(1, false), 3.0, w1);
       balance_segments(cpml, resident_ctas(1, true), 3.0, w2);
       std::vector<RfxbWork2> wd2;
-      wd2.reserve(wd.size());
-      for (const RfxbWork& w : wd)
-        wd2.push_back(RfxbWork2{w.inst, w.y0, w.z0, w.xa, w.xb, depth2_mid_flags(*g->plans[w.inst], w)});
+      depth2_items(g->plans, d2, fwd2_resident(), wd2);
       if (int rc = galloc((void**)&g->d_wd, sizeof(RfxbWork2) * wd2.size())) return rc;
       RFXB_CUDA(cudaMemcpy(g->d_wd, wd2.data(), sizeof(RfxbWork2) * wd2.size(), cudaMemcpyHostToDevice));
       g->n_wd = (int)wd2.size();
@@ -1455,7 +1507,7 @@ int launch_pass(RfxbBatch* g, int n, int par, int pp, cudaStream_t st) {
   RFXB_CUDA(cudaEventRecord(g->ev_fork, st));
   RFXB_CUDA(cudaStreamWaitEvent(g->side_stream, g->ev_fork, 0));
   RFXB_CUDA(cudaStreamWaitEvent(g->side2, g->ev_fork, 0));
-  fwd2_kernel()<<<g->n_wd, dim3(32, kTY), fwd2_step_smem_bytes(), g->side2>>>(g->d_inst, g->d_wd, g->d_maps, n, par);
+  fwd2_kernel()<<<g->n_wd, kFwd2Threads, fwd2_step_smem_bytes(), g->side2>>>(g->d_inst, g->d_wd, g->d_maps, n, par);
   if (g->n_wd1 > 0)
     launch_fwd(1, false, g, g->d_wd1, g->n_wd1, n, step_sel(par, 2, pp), g->side_stream);
   if (g->n_wd2 > 0) launch_fwd(1, true, g, g->d_wd2, g->n_wd2, n, step_sel(par, 2, pp), st);

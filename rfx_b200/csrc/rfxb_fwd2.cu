@@ -1,102 +1,65 @@
-// Two-step forward pass of the CPML-free interior (temporal blocking, depth 2).
+// Two-step forward pass of the CPML-free interior (temporal blocking, depth 2),
+// four cells per thread.
 //
-// One CTA owns a (TY x 32) tile of the (y, z) plane over an x range [xa, xb)
-// and advances it from step n to step n+2 in one pass over HBM: E^n,
-// H^{n-1/2} and ca/cb are read once with a two-cell halo, the intermediate
-// state (E^{n+1}, H^{n+1/2}) lives in shared memory on the tile plus the halo
-// its second step needs, and only (E^{n+2}, H^{n+3/2}) of the tile are
-// written.  The halo cells of the first step are recomputed by every CTA
-// that needs them (overlapped tiling), from step-n values that no CTA of the
-// pass overwrites (the pass reads F[par] and writes F[par ^ 1]).
+// One CTA owns a rectangle of at most 13 rows x 56 columns of the (y, z) plane
+// over an x range [xa, xb) and advances it from step n to step n+2 in one pass
+// over HBM: E^n, H^{n-1/2} and ca/cb are read once with a halo, the intermediate
+// state (E^{n+1}, H^{n+1/2}) stays in registers, and only (E^{n+2}, H^{n+3/2})
+// of the rectangle are written.  The halo cells of the first step are recomputed
+// by every CTA that needs them (overlapped tiling), from step-n values that no
+// CTA of the pass overwrites (the pass reads F[par] and writes F[par ^ 1]).
 //
-// The march along x skews the second step one plane behind the first.  At
-// plane p the CTA computes, each phase over its region of (y, z) cells:
-//   H^{n+1/2}(p)   rows y0-2 .. y0+TY,   columns z0-2 .. z0+32
-//   E^{n+1}(p)     rows y0-1 .. y0+TY,   columns z0-1 .. z0+32
-//   H^{n+3/2}(p-1) rows y0-1 .. y0+TY-1, columns z0-1 .. z0+31
-//   E^{n+2}(p-1)   the tile
-// with the arithmetic of the one-step kernel (rfx/core/yee.py:226-291 and
-// :347-404 through the shared rounding helpers), so every value equals the
-// one the one-step kernel computes, bit for bit.
+// 16 x 16 threads each hold one row and four consecutive columns -- rows y0-2 ..
+// y0+13, columns z0-4 .. z0+59 -- and march along x with the second step one
+// plane behind the first.  At plane p a thread computes, on its own cells,
+//   H^{n+1/2}(p);  E^{n+1}(p), H^{n+3/2}(p-1);  E^{n+2}(p-1)
+// with a block barrier at each semicolon: the y neighbour's values of the phase
+// before pass through shared memory, the z neighbour's come from the adjacent
+// lane, the x neighbour's are the thread's own.  A value at the rim whose
+// neighbour no thread holds is wrong and reaches no stored cell: H^{n+1/2} is
+// right on rows y0-2 .., E^{n+1} on y0-1 .. y0+13, H^{n+3/2} up to y0+12 and
+// E^{n+2} on y0 .. y0+12, alike in z.  The arithmetic is the one-step kernel's
+// (rfx/core/yee.py:226-291 and :347-404 through the shared rounding helpers),
+// so every value equals the one-step value bit for bit.
 //
-// The host gives this kernel only tiles whose cells, halo included, lie in no
-// CPML slab and hold no source, probe or gradient-history cell, in plans with
-// uniform H coefficients; cells at a grid face take the guarded path (zero
-// outside the grid, PEC faces) and a PEC edge mask applies to every E cell as
-// in the one-step kernel.  Everything else runs two one-step launches per
-// pass through the intermediate buffer F[2].
+// The host gives this kernel only cells that, halo included, lie in no CPML slab
+// and hold no source, probe or gradient-history cell, in plans with uniform H
+// coefficients; items at a grid face take the guarded path (zero outside the
+// grid, PEC faces) and a PEC edge mask applies to every E cell as in the
+// one-step kernel.  Everything else runs two one-step launches per pass through
+// the intermediate buffer F[2].
 // Where a one-step neighbour or a per-step observer (DFT plane, flux monitor,
-// NTFF face) reads this tile's intermediate state, the CTA also stores it to
+// NTFF face) reads this item's intermediate state, the CTA also stores it to
 // F[2] (RfxbWork2::mid).
+//
+// What bounds it: the latency of a plane (two barriers, two CTAs of eight warps
+// per SM) and, on grids far beyond L2, the halo rows read again.  16 x 64 cells
+// per plane store 71 % of what they compute; taller CTAs store more but leave
+// one per SM, lower ones store less.  One cell per thread on 8 x 32 tiles, with
+// the intermediate state in shared memory and four barriers per plane -> here,
+// per pass: 257^3 without CPML 399 -> 270 us, 513^3 2679 -> 2381 us (3.2 TB/s of
+// the 56 bytes per cell, 82 moved).
 #include "rfxb_common.cuh"
+#include "rfxb_vec.cuh"
 
 namespace rfxb {
 
-#define RFXB_D2W 40   // staged row: z in [z0 - 4, z0 + 36)
-#define RFXB_D2I 36   // row pitch of the intermediate arrays (35 columns used at most)
-#define RFXB_D2NS 3   // pipeline stages: planes p, p+1 and p+2 in flight
-
-template <int TY>
-struct Fwd2Dims {
-  static constexpr int NE = 3 * (TY + 4) * RFXB_D2W;
-  static constexpr int NH = 3 * (TY + 3) * RFXB_D2W;
-  static constexpr int NC = 2 * (TY + 2) * RFXB_D2W;
-  static constexpr int PH = (NE + NH) % 32 ? 32 - (NE + NH) % 32 : 32;   // cab on a 128-byte boundary
-  static constexpr unsigned BYTES = 4u * (NE + NH + NC);
-};
-
-template <int TY>
-struct __align__(128) Fwd2Stage {
-  float e[3][TY + 4][RFXB_D2W];   // E^n, rows y0-2 .. y0+TY+1
-  float h[3][TY + 3][RFXB_D2W];   // H^{n-1/2}, rows y0-2 .. y0+TY
-  float pad[Fwd2Dims<TY>::PH];
-  float cab[2][TY + 2][RFXB_D2W]; // ca, cb, rows y0-1 .. y0+TY
-};
-
-template <int TY>
 struct Fwd2Smem {
-  Fwd2Stage<TY> st[RFXB_D2NS];          // plane p in stage p % 3
-  float h1[2][3][TY + 3][RFXB_D2I];     // H^{n+1/2}: [y - (y0-2)][z - (z0-2)], slot p & 1
-  float e1[2][3][TY + 2][RFXB_D2I];     // E^{n+1}:   [y - (y0-1)][z - (z0-1)]
-  float h2[2][3][TY + 1][RFXB_D2I];     // H^{n+3/2}: [y - (y0-1)][z - (z0-1)]
-  float cabt[2][2][TY][RFXB_TZ];        // ca, cb of the tile, kept for the second step one plane on
-  float ytab[2][TY + 3];                // yh, ye at y0-2 .. y0+TY
-  float ztab[2][RFXB_D2I];              // zh, ze at z0-2 .. z0+32
+  static constexpr int R = RFXB_D2ROWS, C = RFXB_D2COLS;   // rows and columns of the threads
+  static constexpr int CE = (R + 1) * C, CH = R * C;       // component strides of an E and an H / coefficient stage
+  float e[3][3 * CE];      // E^n, rows y0-2 .. y0+14, plane p in stage (p - xa + 2) % 3
+  float h[2][3 * CH];      // H^{n-1/2}, rows y0-2 .. y0+13
+  float cab[2][2 * CH];    // ca, cb
+  float x1[2][CH];         // hx, hz of H^{n+1/2}(p)
+  float x2[2][2][CH];      // ex, ez of E^{n+1}(p) in slot p & 1
+  float x3[2][CH];         // hx, hz of H^{n+3/2}(p-1)
+  float zt[2][C];          // zh, ze of the columns
   RfxbInst P;
-  unsigned long long mbar[RFXB_D2NS];
+  unsigned long long mbar[RFXB_VBARS];   // E stages, H stages, coefficient stages
 };
+static_assert(2 * (sizeof(Fwd2Smem) + 128 + 1024) <= 228 * 1024, "two CTAs per SM");
 
-size_t fwd2_step_smem_bytes() { return sizeof(Fwd2Smem<8>); }
-
-// Issue the TMA boxes of plane ip (one thread): E and H of the field block of
-// parity par with the two-step boxes, ca/cb with the two-step coefficient box.
-template <int TY>
-__device__ __forceinline__ void tma_stage2(Fwd2Smem<TY>& S, const CUtensorMap* tm, int par, int y0, int z0, int ip) {
-  const int s = (ip + RFXB_D2NS) % RFXB_D2NS;   // ip >= -2
-  const uint32_t mb = smem_u32(&S.mbar[s]);
-  mbar_expect_tx(mb, Fwd2Dims<TY>::BYTES);
-  // map coordinates: (z, j + 1, i + 1, component)
-  tma_load_4d(smem_u32(&S.st[s].e[0][0][0]), tm + RFXB_MAP_E2 + par, z0 - 4, y0 - 1, ip + 1, 0, mb);
-  tma_load_4d(smem_u32(&S.st[s].h[0][0][0]), tm + RFXB_MAP_H2 + par, z0 - 4, y0 - 1, ip + 1, 3, mb);
-  tma_load_4d(smem_u32(&S.st[s].cab[0][0][0]), tm + RFXB_MAP_C2, z0 - 4, y0, ip + 1, 0, mb);
-}
-
-// The cells of a phase region: its 32 middle columns row by row, one warp
-// per row and one lane per column (so every shared-memory row access is 32
-// consecutive words), and its NEDGE edge columns one cell per thread on the
-// last threads.  f(r, c) is called with the region's row and column;
-// edge(k) is the column of edge k.
-template <int TY, int ROWS, int C0, int NEDGE>
-__device__ __forceinline__ void for_region(int ty, int lane, int tid, auto&& edge, auto&& f) {
-#pragma unroll
-  for (int r = ty; r < ROWS; r += TY) f(r, C0 + lane);
-  constexpr int e0 = 32 * TY - NEDGE * ROWS;
-  static_assert(e0 >= 0, "more edge cells than threads");
-  if (tid >= e0) {
-    const int e = tid - e0;
-    f(e / NEDGE, edge(e % NEDGE));
-  }
-}
+size_t fwd2_step_smem_bytes() { return sizeof(Fwd2Smem); }
 
 // PEC faces of the E update (rfx/boundaries/pec.py:13-47), as the one-step
 // kernel applies them.
@@ -108,250 +71,260 @@ __device__ __forceinline__ void pec_faces(unsigned pec, int i, int j, int k, int
   if ((pec & 4u) && k == nz - 1) ez = 0.f;
 }
 
-// PEC edge mask of one E cell (rfx/boundaries/pec.py:179-208), as the
-// one-step kernel applies it after the PEC faces.
-__device__ __forceinline__ void edge_mask(unsigned m, float& ex, float& ey, float& ez) {
-  if (m) {
-    ex = ex * (1.f - (float)(m & 1u));
-    ey = ey * (1.f - (float)((m >> 1) & 1u));
-    ez = ez * (1.f - (float)((m >> 2) & 1u));
-  }
-}
-
 // One work item.  EDGE: the item's cells reach a grid face (no CPML on that
 // axis): cells outside the grid stay zero (the guards the one-step kernel
 // reads) and E takes the PEC faces; otherwise every computed cell is an
 // interior cell and those checks are compiled out.
-template <int TY, bool EDGE>
-__device__ __forceinline__ void fwd2_item(Fwd2Smem<TY>& S, const RfxbWork2& w, const CUtensorMap* __restrict__ maps,
+template <bool EDGE>
+__device__ __forceinline__ void fwd2_item(Fwd2Smem& S, const RfxbWork2& w, const CUtensorMap* __restrict__ maps,
                                           int par) {
-  constexpr int NT = 32 * TY;
-  const int lane = threadIdx.x, ty = threadIdx.y;
-  const int tid = ty * 32 + lane;
+  constexpr int C = Fwd2Smem::C, R = Fwd2Smem::R, CE = Fwd2Smem::CE, CH = Fwd2Smem::CH, NT = R * C / 4, ZQ = C / 4;
+  const int tid = threadIdx.x, r = tid / ZQ, zq = tid % ZQ;
   const RfxbInst& P = S.P;
   const int y0 = w.y0, z0 = w.z0, xa = w.xa, xb = w.xb;
   const int nx = P.nx, ny = P.ny, nz = P.nz;
+  const long long ps = P.ps, cs = P.cs;
   const unsigned pec = P.pec_axes;
-  const unsigned char* emask = P.emask;   // PEC edge mask bits (1 ex, 2 ey, 4 ez) or null
   const CUtensorMap* tm = maps + (size_t)w.inst * RFXB_NMAPS;
-  const int producer = NT - 32;   // lane 0 of the last warp issues the boxes
   const int wlim = kWaitLimit;
-  // planes are staged in order xa-2, xa-1, ..., xb+1 (from -2 on at the low
-  // x face): plane p is the ((p - xa + 2) / 3)-th fill of stage (p + 3) % 3
-  auto stg = [](int p) { return (p + RFXB_D2NS) % RFXB_D2NS; };
-  auto sparity = [&](int p) -> uint32_t { return (uint32_t)(((p - xa + 2) / RFXB_D2NS) & 1); };
-  if (tid == producer)
-    for (int p = xa - 2; p <= min(xa, xb + 1); ++p) tma_stage2<TY>(S, tm, par, y0, z0, p);
-  // spacing tables (entries -1 .. n exist; the cells beyond are zero anyway)
-  for (int t = tid; t < TY + 3; t += NT) {
-    const int j = min(max(y0 - 2 + t, -1), ny);
-    S.ytab[0][t] = __ldg(P.yh + j);
-    S.ytab[1][t] = __ldg(P.ye + j);
+  // The boxes: E of planes xa-2 .. xb+1, H of xa-2 .. xb, coefficients of xa-1 .. xb
+  // (map coordinates: z, j + 1, i + 1, component)
+  const bool producer = tid == NT - 1;
+  auto sE = [&](int p) { return (p - xa + 2) % 3; };
+  auto sH = [&](int p) { return (p - xa + 2) & 1; };
+  auto sC = [&](int p) { return (p - xa + 1) & 1; };
+  auto issue_e = [&](int p) {
+    const uint32_t mb = smem_u32(&S.mbar[sE(p)]);
+    mbar_expect_tx(mb, 4u * 3 * CE);
+    tma_load_4d(smem_u32(&S.e[sE(p)][0]), tm + RFXB_MAP_E2 + par, z0 - 4, y0 - 1, p + 1, 0, mb);
+  };
+  auto issue_h = [&](int p) {
+    const uint32_t mb = smem_u32(&S.mbar[3 + sH(p)]);
+    mbar_expect_tx(mb, 4u * 3 * CH);
+    tma_load_4d(smem_u32(&S.h[sH(p)][0]), tm + RFXB_MAP_H2 + par, z0 - 4, y0 - 1, p + 1, 3, mb);
+  };
+  auto issue_c = [&](int p) {
+    const uint32_t mb = smem_u32(&S.mbar[5 + sC(p)]);
+    mbar_expect_tx(mb, 4u * 2 * CH);
+    tma_load_4d(smem_u32(&S.cab[sC(p)][0]), tm + RFXB_MAP_C2, z0 - 4, y0 - 1, p + 1, 0, mb);
+  };
+  if (producer) {
+    issue_e(xa - 2);
+    issue_e(xa - 1);
+    issue_h(xa - 2);
+    issue_h(xa - 1);
+    issue_e(xa);
+    issue_c(xa - 1);
+    issue_c(xa);
   }
-  for (int t = tid; t < 35; t += NT) {
-    const int k = min(max(z0 - 2 + t, -1), nz);
-    S.ztab[0][t] = __ldg(P.zh + k);
-    S.ztab[1][t] = __ldg(P.ze + k);
+  int last_e = xa, last_h = xa - 1, last_c = xa;   // planes issued so far (xb > xa)
+  // spacing tables (entries -1 .. n exist; the cells beyond are zero or unused)
+  if (tid < C) {
+    const int k = min(max(z0 - 4 + tid, -1), nz);
+    S.zt[0][tid] = __ldg(P.zh + k);
+    S.zt[1][tid] = __ldg(P.ze + k);
   }
+  __syncthreads();   // the first plane reads them before its barrier
   auto xclamp = [&](int i) { return min(max(i, -1), nx); };
   const float ch = P.ch0;
   float* Fo = P.F[par ^ 1][0];
   float* Fm = P.F[2][0];
-  const long long cs = P.cs;
-  // the tile cell of this thread in phase 4 and in the stores
-  const int jt = y0 + ty, kt = z0 + lane;
-  const bool own = !EDGE || (jt < ny && kt < nz);
-  const long long e_row = P.off0 + (long long)jt * P.zs + kt;
-  auto inside = [&](int i, int j, int k) {
-    return !EDGE || ((unsigned)i < (unsigned)nx && (unsigned)j < (unsigned)ny && (unsigned)k < (unsigned)nz);
+  const int j = y0 - 2 + r, k = z0 - 4 + 4 * zq;
+  const float yh = __ldg(P.yh + min(max(j, -1), ny)), ye = __ldg(P.ye + min(max(j, -1), ny));
+  const int oh = r * C + 4 * zq;                       // place in a component of every array here
+  const int om = max(r - 1, 0) * C + 4 * zq, op = min(r + 1, R - 1) * C + 4 * zq;   // rows below and above
+  const long long col = P.off0 + (long long)j * P.zs + k;
+  const bool own = j >= y0 && j < w.yb && k >= z0 && k < w.zb;
+  const bool rim = j == 0 || j == ny - 1 || k == 0 || (k < nz && k + 3 >= nz - 1);   // holds a cell of a y or z face
+  const bool inyz = j >= 0 && j < ny && k >= 0 && k < nz;
+  const unsigned char* emask = P.emask && inyz ? P.emask + col : nullptr;   // PEC edge mask bits (1 ex, 2 ey, 4 ez)
+  // zero outside the grid (EDGE)
+  auto clip = [&](bool in_x, Vec<4>& a, Vec<4>& b, Vec<4>& c) {
+    if (!EDGE) return;
+    const int kv = in_x && inyz ? nz - k : 0;
+    if (kv >= 4) return;
+#pragma unroll
+    for (int l = 0; l < 4; ++l)
+      if (l >= kv) { a[l] = 0.f; b[l] = 0.f; c[l] = 0.f; }
   };
-  // x spacing entries: plane p (loaded one plane ahead) and plane p-1
-  float xh_n = __ldg(P.xh + xclamp(xa - 2)), xe_n = __ldg(P.xe + xclamp(xa - 2));
-  float xh_q = 0.f, xe_q = 0.f;
-  // edge columns of the phase regions (region column indices)
-  auto edge1 = [](int k) { return k < 2 ? k : 34; };   // z0-2, z0-1, z0+32
-  auto edge2 = [](int k) { return k ? 33 : 0; };       // z0-1, z0+32
-  auto edge3 = [](int) { return 0; };                  // z0-1
+  // PEC faces and the edge mask of the four cells
+  auto finish_e = [&](int i, unsigned em, Vec<4>& ex, Vec<4>& ey, Vec<4>& ez) {
+    if (EDGE && (rim || i == 0 || i == nx - 1)) {
+#pragma unroll
+      for (int l = 0; l < 4; ++l) pec_faces(pec, i, j, k + l, nx, ny, nz, ex[l], ey[l], ez[l]);
+    }
+    if (em) {
+#pragma unroll
+      for (int l = 0; l < 4; ++l) {
+        const unsigned m = em >> (8 * l);
+        ex[l] = ex[l] * (1.f - (float)(m & 1u));
+        ey[l] = ey[l] * (1.f - (float)((m >> 1) & 1u));
+        ez[l] = ez[l] * (1.f - (float)((m >> 2) & 1u));
+      }
+    }
+  };
+  // H of the four cells from E (own), the row above, the next plane and the next column
+  auto h_update = [&](const Vec<4>* E, const Vec<4>& uex, const Vec<4>& uez, const Vec<4>& ney, const Vec<4>& nez,
+                      float xh, Vec<4>& hx, Vec<4>& hy, Vec<4>& hz) {
+    const float ex4 = __shfl_down_sync(0xffffffffu, E[0][0], 1, ZQ), ey4 = __shfl_down_sync(0xffffffffu, E[1][0], 1, ZQ);
+    const Vec<4> zh = vld<4>(&S.zt[0][4 * zq]);
+#pragma unroll
+    for (int l = 0; l < 4; ++l) {
+      const float dEz_y = uez[l] - E[2][l], dEx_y = uex[l] - E[0][l];
+      const float dEy_z = (l < 3 ? E[1][l < 3 ? l + 1 : l] : ey4) - E[1][l];
+      const float dEx_z = (l < 3 ? E[0][l < 3 ? l + 1 : l] : ex4) - E[0][l];
+      const float dEz_x = nez[l] - E[2][l], dEy_x = ney[l] - E[1][l];
+      hx[l] = yee_h(hx[l], ch, yee_diff2(dEz_y, yh, dEy_z, zh[l]));
+      hy[l] = yee_h(hy[l], ch, yee_diff2(dEx_z, zh[l], dEz_x, xh));
+      hz[l] = yee_h(hz[l], ch, yee_diff2(dEy_x, xh, dEx_y, yh));
+    }
+  };
+  // E of the four cells from H (own), the row below, the plane before and the column before
+  auto e_update = [&](const Vec<4>* H, const Vec<4>& dhx, const Vec<4>& dhz, const Vec<4>& phy, const Vec<4>& phz,
+                      float xe, const Vec<4>& ca, const Vec<4>& cb, Vec<4>& ex, Vec<4>& ey, Vec<4>& ez) {
+    const float hxm = __shfl_up_sync(0xffffffffu, H[0][3], 1, ZQ), hym = __shfl_up_sync(0xffffffffu, H[1][3], 1, ZQ);
+    const Vec<4> ze = vld<4>(&S.zt[1][4 * zq]);
+#pragma unroll
+    for (int l = 0; l < 4; ++l) {
+      const float dHz_y = H[2][l] - dhz[l], dHx_y = H[0][l] - dhx[l];
+      const float dHy_z = H[1][l] - (l ? H[1][l ? l - 1 : 0] : hym);
+      const float dHx_z = H[0][l] - (l ? H[0][l ? l - 1 : 0] : hxm);
+      const float dHz_x = H[2][l] - phz[l], dHy_x = H[1][l] - phy[l];
+      ex[l] = yee_e(ca[l], ex[l], cb[l], yee_diff2(dHz_y, ye, dHy_z, ze[l]));
+      ey[l] = yee_e(ca[l], ey[l], cb[l], yee_diff2(dHx_z, ze[l], dHz_x, xe));
+      ez[l] = yee_e(ca[l], ez[l], cb[l], yee_diff2(dHy_x, xe, dHx_y, ye));
+    }
+  };
+  auto put = [&](float* F, long long e, const Vec<4>* E, const Vec<4>* H) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      vst<4>(F + c * cs + e, E[c]);
+      vst<4>(F + (3 + c) * cs + e, H[c]);
+    }
+  };
+  unsigned phase = 0u;
+  auto wait = [&](int b) -> bool {
+    const bool ok = mbar_wait_bounded(smem_u32(&S.mbar[b]), (phase >> b) & 1u, wlim);
+    phase ^= 1u << b;
+    return ok;
+  };
 
+  Vec<4> g[3], h1[3], h2y = vzero<4>(), h2z = vzero<4>(), caq = vzero<4>(), cbq = vzero<4>();   // of plane p-1
+#pragma unroll
+  for (int c = 0; c < 3; ++c) g[c] = h1[c] = vzero<4>();
+  unsigned em_q = 0u;
+  float xh_n = __ldg(P.xh + xclamp(xa - 2)), xe_n = __ldg(P.xe + xclamp(xa - 2)), xh_q = 0.f, xe_q = 0.f;
+  bool bad = !wait(0);
+  int sA = 0, sB = 1;   // stages of planes p and p+1
+#pragma unroll 1
   for (int p = xa - 2; p <= xb; ++p) {
-    // planes p and p+1 are needed (p+1 is the furthest); p was waited for in
-    // the previous iteration, except in the first
-    bool ok = mbar_wait_bounded(smem_u32(&S.mbar[stg(p + 1)]), sparity(p + 1), wlim);
-    if (p == xa - 2) ok = ok && mbar_wait_bounded(smem_u32(&S.mbar[stg(p)]), sparity(p), wlim);
-    if (__syncthreads_or(!ok)) {
-      // a wait ran out: flag the launch and drain the boxes in flight
-      if (tid == 0) {
-        atomicOr(P.status, 1);
-        const int last = min(xb + 1, max(xa, p + 1));
-        for (int r = (p == xa - 2 ? p : p + 1); r <= last; ++r)
-          mbar_wait_bounded(smem_u32(&S.mbar[stg(r)]), sparity(r), wlim);
-      }
-      return;
-    }
-    // every thread is done with iteration p-1, so plane p-1's stage is free
-    if (tid == producer && p >= xa - 1 && p + 2 <= xb + 1) tma_stage2<TY>(S, tm, par, y0, z0, p + 2);
     const float xh = xh_n, xe = xe_n;
-    if (p + 1 <= xb) { xh_n = __ldg(P.xh + xclamp(p + 1)); xe_n = __ldg(P.xe + xclamp(p + 1)); }
-
-    // ---- phase 1: H^{n+1/2}(p), rows y0-2 .. y0+TY, columns z0-2 .. z0+32 ----
+    if (p < xb) { xh_n = __ldg(P.xh + xclamp(p + 1)); xe_n = __ldg(P.xe + xclamp(p + 1)); }
+    unsigned em = 0u;
+    if (emask && p >= 0 && p < nx) em = *reinterpret_cast<const unsigned*>(emask + p * ps);
+    bad = !wait(sB) | bad;
+    bad = !wait(3 + sH(p)) | bad;
+    // ---- H^{n+1/2}(p) ----
+    Vec<4> E[3], H[3];
     {
-      const Fwd2Stage<TY>& A = S.st[stg(p)];
-      const Fwd2Stage<TY>& B = S.st[stg(p + 1)];
-      auto& H1 = S.h1[p & 1];
-      for_region<TY, TY + 3, 2, 3>(ty, lane, tid, edge1, [&](int r, int q) {
-        if (!inside(p, y0 - 2 + r, z0 - 2 + q)) {
-          H1[0][r][q] = 0.f; H1[1][r][q] = 0.f; H1[2][r][q] = 0.f;
-          return;
-        }
-        const int lz = q + 2;                   // staged column: z - (z0-4)
-        const float Ex = A.e[0][r][lz], Ey = A.e[1][r][lz], Ez = A.e[2][r][lz];
-        const float dEz_y = A.e[2][r + 1][lz] - Ez;
-        const float dEy_z = A.e[1][r][lz + 1] - Ey;
-        const float dEx_z = A.e[0][r][lz + 1] - Ex;
-        const float dEz_x = B.e[2][r][lz] - Ez;
-        const float dEy_x = B.e[1][r][lz] - Ey;
-        const float dEx_y = A.e[0][r + 1][lz] - Ex;
-        const float yh = S.ytab[0][r], zh = S.ztab[0][q];
-        H1[0][r][q] = yee_h(A.h[0][r][lz], ch, yee_diff2(dEz_y, yh, dEy_z, zh));
-        H1[1][r][q] = yee_h(A.h[1][r][lz], ch, yee_diff2(dEx_z, zh, dEz_x, xh));
-        H1[2][r][q] = yee_h(A.h[2][r][lz], ch, yee_diff2(dEy_x, xh, dEx_y, yh));
-      });
-    }
-    __syncthreads();
-
-    // ---- phase 2: E^{n+1}(p), rows y0-1 .. y0+TY, columns z0-1 .. z0+32 ----
-    if (p >= xa - 1) {
-      const Fwd2Stage<TY>& A = S.st[stg(p)];
-      const auto& H1 = S.h1[p & 1];
-      const auto& H1m = S.h1[(p - 1) & 1];
-      auto& E1 = S.e1[p & 1];
-      for_region<TY, TY + 2, 1, 2>(ty, lane, tid, edge2, [&](int r, int q) {
-        const int j = y0 - 1 + r, k = z0 - 1 + q;
-        if (!inside(p, j, k)) {
-          E1[0][r][q] = 0.f; E1[1][r][q] = 0.f; E1[2][r][q] = 0.f;
-          return;
-        }
-        const int hr = r + 1, hq = q + 1;       // the same cell in H1 / the tables
-        const float hx = H1[0][hr][hq], hy = H1[1][hr][hq], hz = H1[2][hr][hq];
-        const float dHz_y = hz - H1[2][hr - 1][hq];
-        const float dHy_z = hy - H1[1][hr][hq - 1];
-        const float dHx_z = hx - H1[0][hr][hq - 1];
-        const float dHz_x = hz - H1m[2][hr][hq];
-        const float dHy_x = hy - H1m[1][hr][hq];
-        const float dHx_y = hx - H1[0][hr - 1][hq];
-        const float ye = S.ytab[1][hr], ze = S.ztab[1][hq];
-        const float cx_ = yee_diff2(dHz_y, ye, dHy_z, ze);
-        const float cy_ = yee_diff2(dHx_z, ze, dHz_x, xe);
-        const float cz_ = yee_diff2(dHy_x, xe, dHx_y, ye);
-        const float cav = A.cab[0][r][q + 3], cbv = A.cab[1][r][q + 3];
-        float ex = yee_e(cav, A.e[0][hr][q + 3], cbv, cx_);
-        float ey = yee_e(cav, A.e[1][hr][q + 3], cbv, cy_);
-        float ez = yee_e(cav, A.e[2][hr][q + 3], cbv, cz_);
-        if (EDGE) pec_faces(pec, p, j, k, nx, ny, nz, ex, ey, ez);
-        if (emask) edge_mask(emask[P.off0 + (long long)p * P.ps + (long long)j * P.zs + k], ex, ey, ez);
-        E1[0][r][q] = ex;
-        E1[1][r][q] = ey;
-        E1[2][r][q] = ez;
-      });
-      // the tile's ca / cb for its second step one plane on (plane p's stage
-      // takes plane p+3 before that)
-      S.cabt[p & 1][0][ty][lane] = A.cab[0][ty + 1][lane + 4];
-      S.cabt[p & 1][1][ty][lane] = A.cab[1][ty + 1][lane + 4];
-    }
-    __syncthreads();
-
-    // ---- phase 3: H^{n+3/2}(p-1), rows y0-1 .. y0+TY-1, columns z0-1 .. z0+31 ----
-    const int q = p - 1;
-    if (q >= xa - 1) {
-      const auto& E1 = S.e1[q & 1];
-      const auto& E1n = S.e1[p & 1];
-      const auto& H1 = S.h1[q & 1];
-      auto& H2 = S.h2[q & 1];
-      for_region<TY, TY + 1, 1, 1>(ty, lane, tid, edge3, [&](int r, int s) {
-        if (!inside(q, y0 - 1 + r, z0 - 1 + s)) {
-          H2[0][r][s] = 0.f; H2[1][r][s] = 0.f; H2[2][r][s] = 0.f;
-          return;
-        }
-        const float Ex = E1[0][r][s], Ey = E1[1][r][s], Ez = E1[2][r][s];
-        const float dEz_y = E1[2][r + 1][s] - Ez;
-        const float dEy_z = E1[1][r][s + 1] - Ey;
-        const float dEx_z = E1[0][r][s + 1] - Ex;
-        const float dEz_x = E1n[2][r][s] - Ez;
-        const float dEy_x = E1n[1][r][s] - Ey;
-        const float dEx_y = E1[0][r + 1][s] - Ex;
-        const float yh = S.ytab[0][r + 1], zh = S.ztab[0][s + 1];
-        H2[0][r][s] = yee_h(H1[0][r + 1][s + 1], ch, yee_diff2(dEz_y, yh, dEy_z, zh));
-        H2[1][r][s] = yee_h(H1[1][r + 1][s + 1], ch, yee_diff2(dEx_z, zh, dEz_x, xh_q));
-        H2[2][r][s] = yee_h(H1[2][r + 1][s + 1], ch, yee_diff2(dEy_x, xh_q, dEx_y, yh));
-      });
-    }
-    __syncthreads();
-
-    // ---- phase 4: E^{n+2}(p-1) on the tile, and the stores ----
-    if (q >= xa && own) {
-      const auto& H2 = S.h2[q & 1];
-      const auto& H2m = S.h2[(q - 1) & 1];
-      const auto& E1 = S.e1[q & 1];
-      const int r = ty + 1, s = lane + 1;      // in H2 / E1: y - (y0-1), z - (z0-1)
-      const float hx = H2[0][r][s], hy = H2[1][r][s], hz = H2[2][r][s];
-      const float dHz_y = hz - H2[2][r - 1][s];
-      const float dHy_z = hy - H2[1][r][s - 1];
-      const float dHx_z = hx - H2[0][r][s - 1];
-      const float dHz_x = hz - H2m[2][r][s];
-      const float dHy_x = hy - H2m[1][r][s];
-      const float dHx_y = hx - H2[0][r - 1][s];
-      const float ye = S.ytab[1][ty + 2], ze = S.ztab[1][lane + 2];
-      const float cx_ = yee_diff2(dHz_y, ye, dHy_z, ze);
-      const float cy_ = yee_diff2(dHx_z, ze, dHz_x, xe_q);
-      const float cz_ = yee_diff2(dHy_x, xe_q, dHx_y, ye);
-      const float cav = S.cabt[q & 1][0][ty][lane], cbv = S.cabt[q & 1][1][ty][lane];
-      float ex = yee_e(cav, E1[0][r][s], cbv, cx_);
-      float ey = yee_e(cav, E1[1][r][s], cbv, cy_);
-      float ez = yee_e(cav, E1[2][r][s], cbv, cz_);
-      if (EDGE) pec_faces(pec, q, jt, kt, nx, ny, nz, ex, ey, ez);
-      if (emask) edge_mask(emask[e_row + (long long)q * P.ps], ex, ey, ez);
-      const long long e = e_row + (long long)q * P.ps;
-      Fo[e] = ex;
-      Fo[cs + e] = ey;
-      Fo[2 * cs + e] = ez;
-      Fo[3 * cs + e] = hx;
-      Fo[4 * cs + e] = hy;
-      Fo[5 * cs + e] = hz;
-      // the intermediate state of plane q where a one-step neighbour or an
-      // observer reads it
-      if ((w.mid & RFXB_MID_ALL) || (q == xa && (w.mid & RFXB_MID_LO)) || (q == xb - 1 && (w.mid & RFXB_MID_HI))) {
-        const auto& H1 = S.h1[q & 1];
-        Fm[e] = E1[0][r][s];
-        Fm[cs + e] = E1[1][r][s];
-        Fm[2 * cs + e] = E1[2][r][s];
-        Fm[3 * cs + e] = H1[0][r + 1][s + 1];
-        Fm[4 * cs + e] = H1[1][r + 1][s + 1];
-        Fm[5 * cs + e] = H1[2][r + 1][s + 1];
+      const float* A = &S.e[sA][oh];
+      const float* B = &S.e[sB][oh];
+      const float* Ho = &S.h[sH(p)][oh];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        E[c] = vld<4>(A + c * CE);
+        H[c] = vld<4>(Ho + c * CH);
       }
+      h_update(E, vld<4>(A + C), vld<4>(A + 2 * CE + C), vld<4>(B + CE), vld<4>(B + 2 * CE), xh, H[0], H[1], H[2]);
+      clip(p >= 0 && p < nx, H[0], H[1], H[2]);
+      vst<4>(&S.x1[0][oh], H[0]);
+      vst<4>(&S.x1[1][oh], H[2]);
     }
+    if (bar_or<NT>(bad)) { bad = true; break; }
+    // every thread is done with E and H of plane p in shared memory
+    if (producer) {
+      if (p + 3 <= xb + 1) issue_e(p + 3);
+      if (p + 2 <= xb) issue_h(p + 2);
+    }
+    last_e = min(p + 3, xb + 1);
+    last_h = min(p + 2, xb);
+    if (p >= xa - 1) {
+      bad = !wait(5 + sC(p));
+      // ---- E^{n+1}(p) ----
+      const Vec<4> ca = vld<4>(&S.cab[sC(p)][oh]), cb = vld<4>(&S.cab[sC(p)][oh + CH]);
+      e_update(H, vld<4>(&S.x1[0][om]), vld<4>(&S.x1[1][om]), h1[1], h1[2], xe, ca, cb, E[0], E[1], E[2]);
+      finish_e(p, em, E[0], E[1], E[2]);
+      clip(p >= 0 && p < nx, E[0], E[1], E[2]);
+      // the intermediate state of plane p where a one-step neighbour or an observer reads it
+      if (own && p >= xa && p < xb &&
+          ((w.mid & RFXB_MID_ALL) || (p == xa && (w.mid & RFXB_MID_LO)) || (p == xb - 1 && (w.mid & RFXB_MID_HI))))
+        put(Fm, col + p * ps, E, H);
+      vst<4>(&S.x2[p & 1][0][oh], E[0]);
+      vst<4>(&S.x2[p & 1][1][oh], E[2]);
+      const int q = p - 1;
+      if (p >= xa) {
+        // ---- H^{n+3/2}(p-1) ----
+        h_update(g, vld<4>(&S.x2[q & 1][0][op]), vld<4>(&S.x2[q & 1][1][op]), E[1], E[2], xh_q, h1[0], h1[1], h1[2]);
+        clip(q >= 0 && q < nx, h1[0], h1[1], h1[2]);
+        vst<4>(&S.x3[0][oh], h1[0]);
+        vst<4>(&S.x3[1][oh], h1[2]);
+      }
+      __syncthreads();
+      if (producer && p + 2 <= xb) issue_c(p + 2);   // every thread has its coefficients of plane p
+      last_c = max(last_c, min(p + 2, xb));
+      if (p >= xa) {
+        if (q >= xa) {
+          // ---- E^{n+2}(p-1), and the stores ----
+          e_update(h1, vld<4>(&S.x3[0][om]), vld<4>(&S.x3[1][om]), h2y, h2z, xe_q, caq, cbq, g[0], g[1], g[2]);
+          finish_e(q, em_q, g[0], g[1], g[2]);
+          clip(true, g[0], g[1], g[2]);
+          if (own) put(Fo, col + q * ps, g, h1);
+        }
+        h2y = h1[1];
+        h2z = h1[2];
+      }
+#pragma unroll
+      for (int c = 0; c < 3; ++c) g[c] = E[c];
+      caq = ca;
+      cbq = cb;
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) h1[c] = H[c];
+    em_q = em;
     xh_q = xh;
     xe_q = xe;
+    sA = sB;
+    sB = sB == 2 ? 0 : sB + 1;
+  }
+  if (bar_or<NT>(bad) && producer) {
+    // a wait ran out: flag the launch and wait (bounded) for the last box of every stage
+    atomicOr(P.status, 1);
+    auto drain = [&](int b, int fill) { mbar_wait_bounded(smem_u32(&S.mbar[b]), (uint32_t)fill & 1u, wlim); };
+#pragma unroll 1
+    for (int p = max(xa - 2, last_e - 2); p <= last_e; ++p) drain(sE(p), (p - xa + 2) / 3);
+#pragma unroll 1
+    for (int p = max(xa - 2, last_h - 1); p <= last_h; ++p) drain(3 + sH(p), (p - xa + 2) >> 1);
+#pragma unroll 1
+    for (int p = max(xa - 1, last_c - 1); p <= last_c; ++p) drain(5 + sC(p), (p - xa + 1) >> 1);
   }
 }
 
-template <int TY>
-__global__ void __launch_bounds__(32 * TY, 3)
+__global__ void __launch_bounds__(RFXB_D2ROWS * RFXB_D2COLS / 4, 2)
 fwd2_step_kernel(const RfxbInst* __restrict__ insts, const RfxbWork2* __restrict__ work,
                  const CUtensorMap* __restrict__ maps, int n, int par) {
   extern __shared__ __align__(128) unsigned char fwd2_smem_raw[];
-  Fwd2Smem<TY>& S = *reinterpret_cast<Fwd2Smem<TY>*>(fwd2_smem_raw);
-  const int tid = threadIdx.y * 32 + threadIdx.x;
+  Fwd2Smem& S = *reinterpret_cast<Fwd2Smem*>(fwd2_smem_raw);
+  const int tid = threadIdx.x;
   const RfxbWork2 w = work[blockIdx.x];
   if (tid == 0) {
-    for (int q = 0; q < RFXB_D2NS; ++q) mbar_init(smem_u32(&S.mbar[q]), 1);
+#pragma unroll 1
+    for (int q = 0; q < RFXB_VBARS; ++q) mbar_init(smem_u32(&S.mbar[q]), 1);
     mbar_fence_init();
   }
-  load_inst(S.P, insts + w.inst, tid, 32 * TY);
+  load_inst(S.P, insts + w.inst, tid, blockDim.x);
   __syncthreads();
-  if (w.mid & RFXB_MID_EDGE) fwd2_item<TY, true>(S, w, maps, par);
-  else fwd2_item<TY, false>(S, w, maps, par);
+  if (w.mid & RFXB_MID_EDGE) fwd2_item<true>(S, w, maps, par);
+  else fwd2_item<false>(S, w, maps, par);
 }
-
-template __global__ void fwd2_step_kernel<8>(const RfxbInst*, const RfxbWork2*, const CUtensorMap*, int, int);
 
 }  // namespace rfxb

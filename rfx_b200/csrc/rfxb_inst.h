@@ -105,7 +105,7 @@ struct RfxbWork {          // one CTA: a (y, z) tile over an x range
   int xa, xb;
 };
 
-// One CTA of the two-step kernel: a tile over an x range, advanced two time
+// One CTA of the two-step kernel: a rectangle over an x range, advanced two time
 // steps, and where the intermediate state must also be stored (the cells that
 // one-step neighbours or per-step observers read): bit 0 every plane, bit 1
 // plane xa, bit 2 plane xb-1; bit 3: the item's cells reach a grid face (the
@@ -114,9 +114,11 @@ struct RfxbWork {          // one CTA: a (y, z) tile over an x range
 #define RFXB_MID_LO 2
 #define RFXB_MID_HI 4
 #define RFXB_MID_EDGE 8
+#define RFXB_D2ROWS 16   // rows and columns the threads of a CTA hold; the inner
+#define RFXB_D2COLS 64   // 13 x 56 of them can be stored
 struct RfxbWork2 {
   int inst;
-  int y0, z0;
+  int y0, yb, z0, zb;   // [y0, yb) x [z0, zb)
   int xa, xb;
   int mid;
 };
