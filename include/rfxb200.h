@@ -200,6 +200,11 @@ void rfxb_plan_destroy(RfxbPlan* plan);
  * float32.  mu_r_dev may be NULL (mu_r = 1).  edge_mask_dev (uint8, bits
  * 1/2/4 = ex/ey/ez zeroed after each E update, the output of
  * tangential_edge_masks at rfx/boundaries/pec.py:90-176) may be NULL. */
+/* Packed tangential edge bits (1 x, 2 y, 4 z) of an (nx, ny, nz) cell mask, both
+ * uint8 on the device, in stream order: bit a where the cell and one of its two
+ * neighbours along a are set (rfx/boundaries/pec.py:90-176, no periodic axes). */
+int rfxb_edge_mask(int nx, int ny, int nz, const uint8_t* cells_dev, uint8_t* bits_dev, void* stream);
+
 int rfxb_plan_set_materials(RfxbPlan* plan, const float* eps_r_dev, const float* sigma_dev,
                             const float* mu_r_dev, const uint8_t* edge_mask_dev, void* stream);
 

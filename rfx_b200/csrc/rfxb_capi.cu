@@ -29,6 +29,7 @@ size_t fwd_step_smem_bytes();
 __global__ void dft_kernel(const RfxbInst*, const RfxbDftPlane*, int, int, int);
 __global__ void pack_kernel(float*, const float*, RfxbInst);
 __global__ void unpack_kernel(float*, const float*, RfxbInst);
+__global__ void edge_mask_kernel(int, int, int, const unsigned char*, unsigned char*);
 __global__ void coef_kernel(RfxbInst, float*, float*, float*, float*, const float*, const float*,
                             const float*, const unsigned char*, unsigned char*, float);
 __global__ void adj_pass_a(const RfxbInst*, const AdjInst*, const RfxbWork*, int, int, int);
@@ -2157,6 +2158,15 @@ void rfxb_plan_destroy(RfxbPlan* p) {
   cudaDeviceSynchronize();
   delete p->self_group;
   delete p;
+}
+
+int rfxb_edge_mask(int nx, int ny, int nz, const uint8_t* cells, uint8_t* bits, void* stream) {
+  if (nx < 1 || ny < 1 || nz < 1 || !cells || !bits) return fail(RFXB_E_INVALID, "rfxb_edge_mask: bad arguments");
+  const long long total = (long long)nx * ny * nz;
+  const int blocks = (int)std::min<long long>((total + 255) / 256, 65535LL * 8);
+  edge_mask_kernel<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(nx, ny, nz, cells, bits);
+  RFXB_CUDA(cudaGetLastError());
+  return 0;
 }
 
 int rfxb_plan_set_materials(RfxbPlan* p, const float* eps_r, const float* sigma, const float* mu_r,

@@ -308,6 +308,14 @@ class Plan:
         check(self._lib.rfxb_plan_set_materials(self._h, _dptr(e), _dptr(s), _dptr(m), _dptr(em), _stream()),
               "rfxb_plan_set_materials")
 
+    def edge_mask(self, cells):
+        """Packed tangential edge bits of a PEC cell mask of the grid's shape, on
+        the device (``rfx_b200.simulation.tangential_edge_masks``)."""
+        m = self._dev(np.ascontiguousarray(cells, dtype=bool).view(np.uint8), torch.uint8)
+        bits = torch.empty_like(m)
+        check(self._lib.rfxb_edge_mask(*self.shape, _dptr(m), _dptr(bits), _stream()), "rfxb_edge_mask")
+        return bits
+
     def reset(self):
         check(self._lib.rfxb_plan_reset(self._h, _stream()), "rfxb_plan_reset")
 

@@ -297,7 +297,10 @@ def prepare_device_run(grid, materials, n_steps, *, cpml_axes, pec_axes, sources
                          ntff=ntff_descriptor(ntff_box) if ntff_box is not None else None),
                 dev)
     try:
-        em = tangential_edge_masks(_to_np(pec_mask, bool)) if pec_mask is not None else None
+        em = None
+        if pec_mask is not None:
+            cells = _to_np(pec_mask, bool)
+            em = plan.edge_mask(cells) if cells.shape == shape else tangential_edge_masks(cells)
         mu = getattr(materials, "mu_r", None)
         plan.set_materials(_to_np(materials.eps_r), _to_np(materials.sigma),
                            None if mu is None else _to_np(mu), em)
