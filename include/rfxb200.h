@@ -195,16 +195,25 @@ const char* rfxb_last_error(void);
 int rfxb_plan_create(const RfxbDesc* desc, RfxbPlan** out);
 void rfxb_plan_destroy(RfxbPlan* plan);
 
-/* Materials -> per-cell update coefficients (ca, cb of rfx/core/yee.py:387-393,
- * ce of rfx/boundaries/cpml.py:536, ch of cpml.py:818), computed on device in
- * float32.  mu_r_dev may be NULL (mu_r = 1).  edge_mask_dev (uint8, bits
- * 1/2/4 = ex/ey/ez zeroed after each E update, the output of
- * tangential_edge_masks at rfx/boundaries/pec.py:90-176) may be NULL. */
 /* Packed tangential edge bits (1 x, 2 y, 4 z) of an (nx, ny, nz) cell mask, both
  * uint8 on the device, in stream order: bit a where the cell and one of its two
  * neighbours along a are set (rfx/boundaries/pec.py:90-176, no periodic axes). */
 int rfxb_edge_mask(int nx, int ny, int nz, const uint8_t* cells_dev, uint8_t* bits_dev, void* stream);
 
+/* n arrays of bytes[q] between pageable host memory and the device through a
+ * pinned staging buffer of stage_bytes (at least 32 KB), the host side on several
+ * threads.  Enqueued on `stream` behind what it holds; the host arrays have been
+ * read / written, and the staging buffer is free, when the call returns. */
+int rfxb_copy_to_host(int n, void* const* host, void* const* dev, const int64_t* bytes, void* stage,
+                      int64_t stage_bytes, void* stream);
+int rfxb_copy_to_device(int n, void* const* host, void* const* dev, const int64_t* bytes, void* stage,
+                        int64_t stage_bytes, void* stream);
+
+/* Materials -> per-cell update coefficients (ca, cb of rfx/core/yee.py:387-393,
+ * ce of rfx/boundaries/cpml.py:536, ch of cpml.py:818), computed on device in
+ * float32.  mu_r_dev may be NULL (mu_r = 1).  edge_mask_dev (uint8, bits
+ * 1/2/4 = ex/ey/ez zeroed after each E update, the output of
+ * tangential_edge_masks at rfx/boundaries/pec.py:90-176) may be NULL. */
 int rfxb_plan_set_materials(RfxbPlan* plan, const float* eps_r_dev, const float* sigma_dev,
                             const float* mu_r_dev, const uint8_t* edge_mask_dev, void* stream);
 
@@ -355,7 +364,8 @@ int rfxb_batch_adjoint_variant(const RfxbBatch* batch);
  * one-step list) and per reverse time step (*rev: 1, 2 or 3 with
  * the split into plain tiles, CPML tiles that reach a y slab and the other CPML
  * tiles; -1 before the first adjoint advance), not counting DFT / flux / NTFF epilogue
- * kernels.  A diagnostic of this implementation. */
+ * kernels; an advance of a small grid that keeps its state in shared memory is
+ * one launch for all its steps.  A diagnostic of this implementation. */
 int rfxb_plan_step_launches(const RfxbPlan* plan, int* fwd, int* rev);
 int rfxb_batch_step_launches(const RfxbBatch* batch, int* fwd, int* rev);
 

@@ -95,6 +95,10 @@ SIGNATURES = {
     "rfxb_plan_create": (C.c_int, [C.POINTER(RfxbDesc), C.POINTER(C.c_void_p)]),
     "rfxb_plan_destroy": (None, [C.c_void_p]),
     "rfxb_edge_mask": (C.c_int, [C.c_int, C.c_int, C.c_int, C.c_void_p, C.c_void_p, C.c_void_p]),
+    "rfxb_copy_to_host": (C.c_int, [C.c_int, C.POINTER(C.c_void_p), C.POINTER(C.c_void_p), C.POINTER(C.c_int64),
+                                    C.c_void_p, C.c_int64, C.c_void_p]),
+    "rfxb_copy_to_device": (C.c_int, [C.c_int, C.POINTER(C.c_void_p), C.POINTER(C.c_void_p), C.POINTER(C.c_int64),
+                                      C.c_void_p, C.c_int64, C.c_void_p]),
     "rfxb_plan_set_materials": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]),
     "rfxb_plan_reset": (C.c_int, [C.c_void_p, C.c_void_p]),
     "rfxb_plan_load_fields": (C.c_int, [C.c_void_p, C.POINTER(C.c_void_p), C.c_void_p]),

@@ -173,7 +173,7 @@ def run_nonuniform_until_decay(grid, materials, *, decay_by=1e-3, check_interval
                     below = 0
         plan.check_device()
         ts = r.probe_out[:done].cpu().numpy() if r.probe_out is not None else np.zeros((done, 0), np.float32)
-        fields = [t.cpu().numpy() for t in plan.store_fields()]
+        fields = plan.fetch_fields()
         if not flux_stop and not fired:   # rfx/nonuniform.py:2234-2242
             from .simulation import warn_static_remnant_cap_hit
             warn_static_remnant_cap_hit(fields, materials, grid)

@@ -368,7 +368,7 @@ def run_device(grid, materials, n_steps, *, cpml_axes, pec_axes, sources, probes
             lumped = tuple(lumped)
         state = None
         if return_state:
-            f = [t.cpu().numpy() for t in plan.store_fields()]
+            f = plan.fetch_fields()
             state = FDTDState(*f, step=n_steps)
         out_flux = []
         for m, a in zip(flux_monitors, r.flux_accs):
@@ -566,7 +566,7 @@ def run_until_decay(grid, materials, *, decay_by=1e-3, check_interval=50, min_st
         state = None
         fields = None
         if return_state or (absorbing and not flux_stop and not fired):
-            fields = [t.cpu().numpy() for t in plan.store_fields()]
+            fields = plan.fetch_fields()
         if absorbing and not flux_stop and not fired:
             warn_static_remnant_cap_hit(fields, materials, grid)
         if return_state:

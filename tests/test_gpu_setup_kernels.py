@@ -1,10 +1,14 @@
-"""Set-up on the device: the PEC edge mask kernel against the host's."""
+"""Set-up on the device: the PEC edge mask kernel against the host's, the field
+layout round trip, and staged host <-> device copies of sizes around the staging
+threshold and its slots."""
 
 import numpy as np
 import pytest
+import torch
 
 import oracle
-from rfx_b200.engine import Plan, PlanSpec
+from rfx_b200 import engine
+from rfx_b200.engine import Plan, PlanSpec, to_host
 
 pytestmark = pytest.mark.gpu
 
@@ -28,5 +32,20 @@ def test_edge_mask_kernel_equals_host(cuda, shape):
             assert np.array_equal(p.edge_mask(m).cpu().numpy(), _bits(m))
         # a mask in another memory order
         assert np.array_equal(p.edge_mask(np.asfortranarray(m)).cpu().numpy(), _bits(m))
+    finally:
+        p.close()
+
+
+@pytest.mark.parametrize("extra", [-1, 0, 1, engine._STAGE_BYTES // 4 + 3, 3 * engine._STAGE_BYTES // 4 - 1])
+def test_staged_copies_round_trip(cuda, extra):
+    p = _plan((4, 4, 4))
+    try:
+        n = engine._STAGED_UP // 4 + extra
+        a = np.random.default_rng(2).standard_normal(n).astype(np.float32)
+        d = p._dev(a)
+        assert np.array_equal(d.cpu().numpy(), a)
+        x, y = to_host([d, d * 2.0])
+        assert np.array_equal(x, a) and np.array_equal(y, a * np.float32(2.0))
+        assert x.flags.writeable and x.base is not y.base
     finally:
         p.close()
