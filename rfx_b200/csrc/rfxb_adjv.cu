@@ -22,11 +22,11 @@
 //
 // What bounds it: instructions and, in the slabs, instruction fetch (the CPML
 // path is 98 KB of code; the rare work -- probes, sources, gradient, failure --
-// therefore sits behind single sites over indexed copies: the step of 64 grids
+// therefore sits behind single sites over indexed copies: the step of 20 grids
 // of 64-160 cells a side 1477 -> 1380 us).  One cell per thread with the
 // relations of the neighbours evaluated again in place -> here: that step
 // 1810 -> 1375 us (three launches against one), 221x141x69 with CPML 10
-// 157 -> 100, 97x83x109 with CPML 8 103 -> 46.
+// 157 -> 100, 97x83x109 with CPML 8 103 -> 43.
 #include "rfxb_common.cuh"
 #include "rfxb_vec.cuh"
 

@@ -27,8 +27,8 @@ namespace rfxb {
 __global__ void fwd_step_kernel(const RfxbInst*, const RfxbWork*, int, int);
 size_t fwd_step_smem_bytes();
 __global__ void dft_kernel(const RfxbInst*, const RfxbDftPlane*, int, int, int);
-__global__ void pack_kernel(float*, const float*, RfxbInst);
-__global__ void unpack_kernel(float*, const float*, RfxbInst);
+template <bool PACK>
+__global__ void relayout_kernel(RfxbSixPtrs, RfxbSixPtrs, RfxbInst);
 __global__ void edge_mask_kernel(int, int, int, const unsigned char*, unsigned char*);
 __global__ void coef_kernel(RfxbInst, float*, float*, float*, float*, const float*, const float*,
                             const float*, const unsigned char*, unsigned char*, float);
@@ -308,7 +308,8 @@ void make_work(const RfxbPlan& p, int inst_index, int chunks, std::vector<RfxbWo
 // plane and tile lie in, plus `prologue` plane-costs for its start-up (the
 // extra planes it stages and the H it recomputes at xa-1).  Each tile's x
 // line is cut into pieces of about equal cost; the piece size is chosen, over
-// one to four waves of the resident CTA capacity, by simulating the block
+// one to four waves of the resident CTA capacity (or two counts from min_waves
+// on), by simulating the block
 // scheduler's greedy dispatch of the pieces in decreasing cost order (the
 // order the list is emitted in), so heavy CPML tiles and large instances of a
 // batch no longer set the step time.
@@ -385,7 +386,7 @@ void balance_segments(const std::vector<WorkSeg>& segs, int resident, double pro
   };
   std::vector<Item> best, cur;
   double best_t = 1e300;
-  for (int waves = min_waves; waves <= min_waves + 3; ++waves) {
+  for (int waves = min_waves; waves <= (min_waves > 1 ? min_waves + 1 : 4); ++waves) {
     cut(W / ((double)resident * waves), cur);
     const double t = makespan(cur);
     if (t < best_t * (1.0 - 0.02)) { best_t = t; best = cur; }   // more waves only for a clear gain
@@ -830,7 +831,7 @@ void launch_fwd_generic(const RfxbBatch* g, int n, int sel, cudaStream_t st) {
 // grid needs enough of them; the line lies where eight-plane pieces still give
 // every SM its two CTAs.  Below it (97x83x109, 24 rows / 8 rows): forward 35 / 32
 // us, reverse 45 / 43; above it (the 221x141x69 grid) forward 78 / 90, reverse
-// 100 / 133, (64 grids of 64-160 a side) forward 1005 / 1207, reverse 1375 / 1839.
+// 100 / 133, (20 grids of 64-160 a side) forward 1005 / 1207, reverse 1375 / 1839.
 int pick_fwd_tile(const RfxbBatch* g) {
   long long items = 0;
   for (const RfxbPlan* p : g->plans)
@@ -863,8 +864,8 @@ int fwd2_resident() {
 
 // Default depth of the forward passes: RFXB_FWD_DEPTH=1 or 2 sets it for
 // every group with two-step tiles; unset, groups without any CPML of at least
-// 2^24 cells take two steps per pass (the 513^3 PEC benchmark: 78.1 -> 98.1
-// G cells/s) and the others one (with CPML the gain measured 0-2 %, and on
+// 2^24 cells take two steps per pass (per step, one and two: 257^3 183 and 135
+// us, 513^3 1740 and 1190 us) and the others one (with CPML the gain measured 0-2 %, and on
 // small grids the directly launched passes lose the graphs' launch rate;
 // the autotuner chooses per workload).
 int fwd_depth_default(const RfxbBatch* g) {
@@ -2213,12 +2214,13 @@ int rfxb_plan_reset(RfxbPlan* p, void* stream) {
 int rfxb_plan_load_fields(RfxbPlan* p, const float* const* fields, void* stream) {
   if (!p || !fields) return fail(RFXB_E_INVALID, "null argument");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const long long cells = (long long)p->nx * p->ny * p->nz;
-  const int blocks = (int)std::min<long long>((cells + 255) / 256, 65535LL * 8);
+  RfxbSixPtrs ref, own;
   for (int c = 0; c < 6; ++c) {
     if (!fields[c]) return fail(RFXB_E_INVALID, "null field pointer");
-    pack_kernel<<<blocks, 256, 0, st>>>(p->inst.F[p->par][c], fields[c], p->inst);
+    ref.p[c] = const_cast<float*>(fields[c]);
+    own.p[c] = p->inst.F[p->par][c];
   }
+  relayout_kernel<true><<<dim3(relayout_blocks(p->nx, p->ny), 6), 256, 0, st>>>(ref, own, p->inst);
   RFXB_CUDA(cudaGetLastError());
   return 0;
 }
@@ -2226,12 +2228,13 @@ int rfxb_plan_load_fields(RfxbPlan* p, const float* const* fields, void* stream)
 int rfxb_plan_store_fields(RfxbPlan* p, float* const* fields, void* stream) {
   if (!p || !fields) return fail(RFXB_E_INVALID, "null argument");
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const long long cells = (long long)p->nx * p->ny * p->nz;
-  const int blocks = (int)std::min<long long>((cells + 255) / 256, 65535LL * 8);
+  RfxbSixPtrs ref, own;
   for (int c = 0; c < 6; ++c) {
     if (!fields[c]) return fail(RFXB_E_INVALID, "null field pointer");
-    unpack_kernel<<<blocks, 256, 0, st>>>(fields[c], p->inst.F[p->par][c], p->inst);
+    ref.p[c] = fields[c];
+    own.p[c] = p->inst.F[p->par][c];
   }
+  relayout_kernel<false><<<dim3(relayout_blocks(p->nx, p->ny), 6), 256, 0, st>>>(ref, own, p->inst);
   RFXB_CUDA(cudaGetLastError());
   return 0;
 }

@@ -30,7 +30,7 @@
 // psi 4 bytes at a time.  24 x 32 tiles take two CTAs per SM (seven warps, 128
 // registers, up to 110 KB); taller ones leave one, lower ones reread more halo.
 // Measured, one cell per thread -> here: 217x217x121 with CPML 12 182 -> 129 us a
-// step, 131x147x103 with CPML 8 96 -> 61, 277^3 with CPML 10 327 -> 316 (of
+// step, 131x147x103 with CPML 8 96 -> 61, 277^3 with CPML 10 about 325 -> 316 (of
 // which CPML-free items 160).  H and the coefficients loaded into registers one
 // plane ahead instead of staged: 263 us instead of 183 on 257^3.
 #include "rfxb_common.cuh"

@@ -92,6 +92,15 @@ struct RfxbInst {
   int* status;             // device status word: bit 0 = a pipeline wait ran out
 };
 
+struct RfxbSixPtrs {       // one array per field component
+  float* p[6];
+};
+// Blocks (of eight warps, a z row each) of a relayout launch, per component.
+inline int relayout_blocks(int nx, int ny) {
+  const int rows8 = (nx * ny + 7) / 8;
+  return rows8 < 1184 ? rows8 : 1184;
+}
+
 struct AdjInst {           // adjoint state of one instance (same layouts as the forward state)
   float* aF[2][6];         // ping-pong: aex aey aez ahx ahy ahz (component stride cs)
   float* aPsiH[2][3];      // ping-pong

@@ -43,8 +43,8 @@
 namespace rfxb {
 __global__ void fwd_step_kernel(const RfxbInst*, const RfxbWork*, int, int);
 size_t fwd_step_smem_bytes();
-__global__ void pack_kernel(float*, const float*, RfxbInst);
-__global__ void unpack_kernel(float*, const float*, RfxbInst);
+template <bool PACK>
+__global__ void relayout_kernel(RfxbSixPtrs, RfxbSixPtrs, RfxbInst);
 __global__ void coef_kernel(RfxbInst, float*, float*, float*, float*, const float*, const float*, const float*,
                             const unsigned char*, unsigned char*, float);
 void set_last_error(const char* msg);   // the message rfxb_last_error() returns
@@ -311,7 +311,12 @@ extern "C" int rfxb_forward_noalloc(const RfxbDesc* d, const float* eps_r_dev, c
   const int blocks = (int)std::min<long long>((cells + 255) / 256, 65535LL * 8);
   coef_kernel<<<blocks, 256, 0, st>>>(I, coef, coef + elems, coef + 2 * elems, nullptr, eps_r_dev, sigma_dev, nullptr,
                                       nullptr, nullptr, (float)d->dt);
-  for (int c = 0; c < 6; ++c) pack_kernel<<<blocks, 256, 0, st>>>(I.F[0][c], fields_dev[c], I);
+  RfxbSixPtrs ref, own;
+  for (int c = 0; c < 6; ++c) {
+    ref.p[c] = fields_dev[c];
+    own.p[c] = I.F[0][c];
+  }
+  relayout_kernel<true><<<dim3(relayout_blocks(I.nx, I.ny), 6), 256, 0, st>>>(ref, own, I);
   const RfxbInst* dI = reinterpret_cast<const RfxbInst*>(base + o_inst);
   const RfxbWork* dW = reinterpret_cast<const RfxbWork*>(base + o_work);
   int par = 0;
@@ -320,7 +325,8 @@ extern "C" int rfxb_forward_noalloc(const RfxbDesc* d, const float* eps_r_dev, c
                                                                                 step_sel(par, par ^ 1, par));
     par ^= 1;
   }
-  for (int c = 0; c < 6; ++c) unpack_kernel<<<blocks, 256, 0, st>>>(fields_dev[c], I.F[par][c], I);
+  for (int c = 0; c < 6; ++c) own.p[c] = I.F[par][c];
+  relayout_kernel<false><<<dim3(relayout_blocks(I.nx, I.ny), 6), 256, 0, st>>>(ref, own, I);
   if (!ok(cudaGetLastError())) return noalloc_fail(RFXB_E_LAUNCH, "rfxb_forward_noalloc: kernel launch failed");
   return 0;
 }

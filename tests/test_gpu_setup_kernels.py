@@ -36,6 +36,18 @@ def test_edge_mask_kernel_equals_host(cuda, shape):
         p.close()
 
 
+@pytest.mark.parametrize("shape", [(2, 2, 2), (3, 5, 31), (9, 2, 128), (4, 7, 129), (2, 33, 300), (120, 90, 33)])
+def test_fields_round_trip_through_the_padded_layout(cuda, shape):
+    p = _plan(shape)
+    try:
+        f = np.random.default_rng(3).standard_normal((6,) + shape).astype(np.float32)
+        p.load_fields(list(f))
+        for a, b in zip(f, p.store_fields()):
+            assert np.array_equal(a, b.cpu().numpy())
+    finally:
+        p.close()
+
+
 @pytest.mark.parametrize("extra", [-1, 0, 1, engine._STAGE_BYTES // 4 + 3, 3 * engine._STAGE_BYTES // 4 - 1])
 def test_staged_copies_round_trip(cuda, extra):
     p = _plan((4, 4, 4))
