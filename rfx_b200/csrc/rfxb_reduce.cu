@@ -116,16 +116,26 @@ __global__ void flux_kernel(const RfxbInst* __restrict__ insts, const RfxbFluxPl
   v[2] = (P.F[par][M.comp[2]][em1] + P.F[par][M.comp[2]][e]) * 0.5f;
   v[3] = (P.F[par][M.comp[3]][em1] + P.F[par][M.comp[3]][e]) * 0.5f;
   const double2* kn = M.kern + (long long)n * 2 * M.nf;
-  for (int f = 0; f < M.nf; ++f) {
-    const double2 ke = kn[f], kh = kn[M.nf + f];
+  // two frequencies' loads in flight at once (one load after the other: 7.5 us
+  // for four frequencies of an 85 x 61 region; here 4.2)
+  for (int f0 = 0; f0 < M.nf; f0 += 2) {
+    double2 s[2][4];
 #pragma unroll
-    for (int t = 0; t < 4; ++t) {
-      const double2 k2 = t < 2 ? ke : kh;
-      double2* acc = M.acc + ((long long)t * M.nf + f) * cells + c;
-      double2 s = *acc;
-      s.x += (double)v[t] * k2.x;
-      s.y += (double)v[t] * k2.y;
-      *acc = s;
+    for (int u = 0; u < 2; ++u)
+#pragma unroll
+      for (int t = 0; t < 4; ++t)
+        if (f0 + u < M.nf) s[u][t] = M.acc[((long long)t * M.nf + f0 + u) * cells + c];
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      if (f0 + u >= M.nf) break;
+      const double2 ke = kn[f0 + u], kh = kn[M.nf + f0 + u];
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        const double2 k2 = t < 2 ? ke : kh;
+        s[u][t].x += (double)v[t] * k2.x;
+        s[u][t].y += (double)v[t] * k2.y;
+        M.acc[((long long)t * M.nf + f0 + u) * cells + c] = s[u][t];
+      }
     }
   }
 }
@@ -156,26 +166,41 @@ __global__ void __launch_bounds__(256) ntff_kernel(const RfxbInst* __restrict__ 
 #pragma unroll
   for (int t = 0; t < 4; ++t) v[t] = P.F[par][A.comp[t]][e];
   const float2* ph = A.phase + (long long)n * 2 * A.nf;
-  for (int f = 0; f < A.nf; ++f) {
-    const float2 we = __ldg(ph + f), wh = __ldg(ph + A.nf + f);
-    float4* sp = reinterpret_cast<float4*>(A.acc + ((long long)f * cells + c) * 4);
-    float4* rp = reinterpret_cast<float4*>(A.cmp + ((long long)f * cells + c) * 4);
+  // two frequencies' loads in flight at once (half of one after the other: 7.7 us
+  // for three frequencies of the faces of a 71 x 79 x 55 box; here 6.2)
+  for (int f0 = 0; f0 < A.nf; f0 += 2) {
+    float4 s[2][2], r[2][2];           // [frequency][0: the E pair, 1: the H pair]
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {    // h = 0: the E pair, h = 1: the H pair
-      const float2 w = h == 0 ? we : wh;
-      float4 s = sp[h], r = rp[h];
-      float* sv = reinterpret_cast<float*>(&s);
-      float* rv = reinterpret_cast<float*>(&r);
+    for (int g = 0; g < 2; ++g)
+      if (f0 + g < A.nf) {
+        const long long o = ((long long)(f0 + g) * cells + c) * 4;
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {  // (re, im) of the two components
-        const float val = __fmul_rn(v[2 * h + (u >> 1)], (u & 1) ? w.y : w.x);
-        const float y = val - rv[u];
-        const float t = sv[u] + y;
-        rv[u] = (t - sv[u]) - y;
-        sv[u] = t;
+        for (int h = 0; h < 2; ++h) {
+          s[g][h] = reinterpret_cast<const float4*>(A.acc + o)[h];
+          r[g][h] = reinterpret_cast<const float4*>(A.cmp + o)[h];
+        }
       }
-      sp[h] = s;
-      rp[h] = r;
+#pragma unroll
+    for (int g = 0; g < 2; ++g) {
+      if (f0 + g >= A.nf) break;
+      const long long o = ((long long)(f0 + g) * cells + c) * 4;
+      const float2 we = __ldg(ph + f0 + g), wh = __ldg(ph + A.nf + f0 + g);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const float2 w = h == 0 ? we : wh;
+        float* sv = reinterpret_cast<float*>(&s[g][h]);
+        float* rv = reinterpret_cast<float*>(&r[g][h]);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {  // (re, im) of the two components
+          const float val = __fmul_rn(v[2 * h + (u >> 1)], (u & 1) ? w.y : w.x);
+          const float y = val - rv[u];
+          const float t = sv[u] + y;
+          rv[u] = (t - sv[u]) - y;
+          sv[u] = t;
+        }
+        reinterpret_cast<float4*>(A.acc + o)[h] = s[g][h];
+        reinterpret_cast<float4*>(A.cmp + o)[h] = r[g][h];
+      }
     }
   }
 }
