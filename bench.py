@@ -280,22 +280,22 @@ def run_ours(args, rank, world, local_rank):
                 "traffic": (round(tpc * cells) if tpc else None), "algorithmic_bytes_per_step": int(alg),
                 "share_of_step": round(ms / total_ms, 3), "what": what}
 
-    roof_adj = roof("adj_step_kernel", sum(p.adjoint_algorithmic_bytes_per_step() for p in sw.plans), adj_ms,
-                    "fused reverse step, batched over all instances: variant 2 on the tiles that reach a y slab, "
-                    "variant 4 on the other CPML work, variant 3 on the plain tiles, three streams; one step = "
-                    "the three launches")
+    roof_adj = roof("adjv_kernel", sum(p.adjoint_algorithmic_bytes_per_step() for p in sw.plans), adj_ms,
+                    "fused reverse step, four cells per thread, batched over all instances: one launch over all "
+                    "tiles, or three side by side where the autotuner chose the split; one step = its launches")
     two_step = (sw.batch or sw.plans[0]).launch_config()[0].get("fwd_depth", 1) == 2
     if two_step:
-        roof_fwd = roof("fwd_step_kernel", sum(p.algorithmic_bytes_per_step() for p in sw.plans), fwd_ms,
+        roof_fwd = roof("fwdv_kernel", sum(p.algorithmic_bytes_per_step() for p in sw.plans), fwd_ms,
                         "forward in two-step passes, batched over all instances: fwd2_step_kernel advances the "
                         "tiles clear of CPML, sources, probes and the gradient region two steps per read of the "
-                        "state, beside two launches of variant 2 (CPML tiles) and variant 1 (the other CPML-free "
-                        "work) per pass; algorithmic bytes counted per step",
+                        "state, beside two launches of fwdv_kernel each on the CPML tiles and on the other "
+                        "CPML-free work per pass; algorithmic bytes counted per step",
                         key="small_case_dram_bytes_per_cell_per_step_two_step")
     else:
-        roof_fwd = roof("fwd_step_kernel", sum(p.algorithmic_bytes_per_step() for p in sw.plans), fwd_ms,
-                        "fused forward step, batched over all instances: variant 2 on the CPML tiles and variant 1 "
-                        "on the plain tiles, two streams; one step = both launches")
+        roof_fwd = roof("fwdv_kernel", sum(p.algorithmic_bytes_per_step() for p in sw.plans), fwd_ms,
+                        "fused forward step, four cells per thread, batched over all instances: one launch over "
+                        "all tiles, or two side by side where the autotuner chose the split; one step = its "
+                        "launches")
     roofline, roofline_other = (roof_adj, roof_fwd) if adj_ms >= fwd_ms else (roof_fwd, roof_adj)
 
     # single-instance comparison (each simulation launched on its own)
@@ -356,8 +356,8 @@ def run_ours(args, rank, world, local_rank):
 
     # our kernels per bench step: N forward steps, one adjoint init per
     # simulation launch group, N reverse steps, each step as many step-kernel
-    # launches as the library reports (CPML / plain split, variant 4; per
-    # pass of two steps with two-step passes)
+    # launches as the library reports (one, or the split ones; per pass of two
+    # steps with two-step passes)
     fl, rl = sw.step_launches()
     cfg = (sw.batch or sw.plans[0]).launch_config()[0]
     launches = args.steps * (forward_launches(fl, cfg, N) + N * rl + (1 if sw.batch is not None else len(sw.plans)))
@@ -608,7 +608,7 @@ def run_pec_uniform(args, emit, hbm_peak, peak_src):
     step_s = ms / 1e3 / (args.steps * N)
     depth2 = cfg.get("fwd_depth", 1) == 2
     kernel = ("fwd2_step_kernel (two steps per pass; algorithmic bytes counted per step)"
-              if depth2 else "fwd_step_kernel (CPML-free variant)")
+              if depth2 else "fwdv_kernel (CPML-free)")
     # DRAM bytes per cell-step of the 257^3 capture of the same scene
     tpc = _traffic_per_cell("fwd2_step_kernel", "pec_257_dram_bytes_per_cell_per_step_" +
                             ("two_step" if depth2 else "one_step"))
