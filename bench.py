@@ -467,7 +467,7 @@ def run_secondary(args, which, emit=True):
         dft_bytes = sum(32 * len(d.freqs) * int(np.prod(a.shape[1:])) for d, a in zip(planes, r.dft_accs))
         alg = plan.algorithmic_bytes_per_step() + dft_bytes
         metric = "Mcell-steps/s forward, 1 B200"
-        kernel = "fwd_step_kernel + dft_kernel (whole step)"
+        kernel = "fwdv_kernel + dft_kernel (whole step)"
     else:
         from rfx_b200.adjoint import AdjointRunner, probe_dft_objective
         g, eps, sig, src, probes, box, freqs = workloads.adjoint_region(n_steps=N)
@@ -488,7 +488,7 @@ def run_secondary(args, which, emit=True):
         # forward + segment recompute + reverse step, each ~ one forward's bytes
         alg = 3 * plan.algorithmic_bytes_per_step()
         metric = "Mcell-steps/s fwd+adjoint grad (checkpoint every 64), 1 B200"
-        kernel = "fwd_step_kernel x2 + adj_step_kernel (whole step)"
+        kernel = "fwdv_kernel x2 + adjv_kernel (whole step)"
     # launch configuration of this plan chosen by the autotuner (trial runs
     # before the warm-up; every timed run starts from a reset state)
     launch = {"chosen_by": "defaults", "config": plan.launch_config()[0]}
