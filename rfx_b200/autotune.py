@@ -2,10 +2,9 @@
 
 A plan or batch can launch its step kernels in several equivalent ways (the
 ``RfxbLaunchConfig`` fields of ``rfxb200.h``): the forward tiles split
-between the CPML-free kernel and the staged-psi kernel on two streams or run
-as one launch, which of the concurrent launches the captured graph hands to
-the SMs first, whether the reverse step's CPML work without a y slab runs
-on variant 4 or on variant 2, whether a persistent launch over device work
+between the CPML-free and the CPML kernel on two streams or run as one launch, which of the concurrent launches the captured graph hands to
+the SMs first, whether the reverse step runs as one launch or as three (CPML
+tiles without a y slab, those with one, plain tiles), whether a persistent launch over device work
 queues replaces the split launches, and the L2 promotion of the TMA boxes
 (how much of a partly covered line a halo miss fetches; 64 B measured 1.6 %
 faster than 128 B on the batched sweep and 2.8 % slower on a 513^3 PEC
@@ -25,9 +24,9 @@ import json
 import os
 from dataclasses import dataclass, field
 
-# Reverse launch orders (rfxb200.h): permutations of (variant 4, variant 2,
-# variant 3) by index.  Without variant 4 only the relative order of 2 and 3
-# counts, so orders 0 (2 before 3) and 1 (3 before 2) represent all six.
+# Reverse launch orders (rfxb200.h): permutations by index of the split launches
+# 4 (CPML tiles without a y slab), 2 (those with one) and 3 (plain tiles).
+# Unsplit (adj_lite 0) only the relative order of 2 and 3 is told apart, so orders 0 (2 before 3) and 1 (3 before 2) represent all six.
 REVERSE_ORDERS = ((4, 2, 3), (4, 3, 2), (2, 4, 3), (2, 3, 4), (3, 4, 2), (3, 2, 4))
 
 _memory_cache: dict = {}
@@ -86,7 +85,7 @@ def forward_candidates(limits: dict, current: dict) -> list:
 
 
 def reverse_candidates(limits: dict, current: dict) -> list:
-    """Reverse settings to time: every order with variant 4, and the two
+    """Reverse settings to time: every order of the split, and the two
     distinct orders without it, as far as the limits allow (the current
     setting first)."""
     c = []

@@ -211,8 +211,8 @@ struct RfxbBatch {
   cudaStream_t side2 = nullptr;
   cudaEvent_t ev_join2 = nullptr;
   // two-step passes (fwd_depth 2): the two-step kernel's tiles, and the
-  // one-step work of a pass -- the other CPML-free tiles (variant 1) and the
-  // CPML tiles (variant 2) -- launched once per step of the pass through the
+  // one-step work of a pass -- the other CPML-free tiles and the
+  // CPML tiles -- launched once per step of the pass through the
   // intermediate buffer F[2]
   int fwd_depth = 1;
   bool fwd_depth_avail = false;
@@ -249,7 +249,7 @@ struct RfxbBatch {
   int wait_limit = rfxb::kWaitLimit;
   int adj_persist_grid = 0;        // CTAs of the persistent reverse launch (resident at once)
   int fwd_mode = 0;                // forward step kernel variant (see rfxb_fwd.cu)
-  int adj_mode = -1;               // reverse step kernel variant (see rfxb_adj_fused.cu), -1 not chosen yet
+  int adj_mode = -1;               // reverse step kernel variant (see rfxb200.h), -1 not chosen yet
   std::vector<RfxbDftPlane> dft;
   int dft_blocks = 0;
   std::vector<void*> allocs;
@@ -429,10 +429,9 @@ struct SlabCost {
   SlabCost(double sx, double sy, double sz, double c) : x(sx), y(sy), z(sz), cp(c) {}
 };
 
-// Split of the forward work between the CPML-free kernel (variant 1) and the
-// staged-psi kernel (variant 2): a tile that reaches no y/z slab runs planes
-// ncp+1 .. nx-ncp-1 (whose x-1 prologue plane is outside the x slab too) on
-// variant 1, everything else on variant 2.
+// Split of the forward work between the CPML-free and the CPML code: a tile that
+// reaches no y/z slab runs planes ncp+1 .. nx-ncp-1 (whose x-1 prologue plane is
+// outside the x slab too) on the first, everything else on the second.
 void split_segments(const std::vector<RfxbPlan*>& plans, const SlabCost& slab, std::vector<WorkSeg>& plain,
                     std::vector<WorkSeg>& cpml, int ty = kTY, int tz = 32) {
   for (size_t q = 0; q < plans.size(); ++q) {
@@ -551,7 +550,7 @@ void depth2_xrange(const RfxbPlan& p, int& dlo, int& dhi) {
 }
 
 // Work of a two-step pass: two-step segments (d2), the other CPML-free work
-// (plain, variant 1) and the CPML work (cpml, variant 2; the same split as
+// (plain) and the CPML work (cpml; the same split as
 // split_segments).  Together they cover every cell of every plan once.
 void split_depth2_segments(const std::vector<RfxbPlan*>& plans, double slab, std::vector<WorkSeg>& d2,
                            std::vector<WorkSeg>& plain, std::vector<WorkSeg>& cpml) {
@@ -904,8 +903,8 @@ int fwd_persist_default() {
   return std::string(e) == "0" ? 0 : 2;
 }
 
-// The persistent reverse launch needs the three reverse lists (variant 2 on
-// y-slab tiles, variant 4 on the other CPML work, variant 3 on plain tiles).
+// The persistent reverse launch needs the three reverse lists (y-slab tiles, the
+// other CPML work, plain tiles).
 bool adj_persist_avail(const RfxbBatch* g);
 
 // CTAs of a forward tile shape resident at once.
