@@ -2,17 +2,18 @@
 
 A plan or batch can launch its step kernels in several equivalent ways (the
 ``RfxbLaunchConfig`` fields of ``rfxb200.h``): the forward tiles split
-between the CPML-free and the CPML kernel on two streams or run as one launch, which of the concurrent launches the captured graph hands to
-the SMs first, whether the reverse step runs as one launch or as three (CPML
-tiles without a y slab, those with one, plain tiles), whether a persistent launch over device work
-queues replaces the split launches, and the L2 promotion of the TMA boxes
+between the CPML-free and the CPML kernel on two streams or run as one launch,
+which of the concurrent launches the captured graph hands to the SMs first,
+whether the reverse step runs as one launch or as three (CPML tiles without a
+y slab, those with one, plain tiles), whether a persistent launch over device
+work queues replaces the split launches, and the L2 promotion of the TMA boxes
 (how much of a partly covered line a halo miss fetches; 64 B measured 1.6 %
 faster than 128 B on the batched sweep and 2.8 % slower on a 513^3 PEC
-grid).  Every setting computes the same steps; which
-one is fastest depends on the workload (grid sizes, CPML share, number of
-instances).  The autotuner times a few steps of each candidate with CUDA
-events on the real workload, keeps the fastest, and caches the choice by a
-workload signature (in memory, and in a JSON file when a path is given).
+grid).  Every setting computes the same steps; which one is fastest depends on
+the workload (grid sizes, CPML share, number of instances).  The autotuner
+times a few steps of each candidate with CUDA events on the real workload,
+keeps the fastest, and caches the choice by a workload signature (in memory,
+and in a JSON file when a path is given) for the kernels it was timed with.
 
 The reference has no counterpart: XLA schedules its scan body itself.
 """
@@ -26,7 +27,8 @@ from dataclasses import dataclass, field
 
 # Reverse launch orders (rfxb200.h): permutations by index of the split launches
 # 4 (CPML tiles without a y slab), 2 (those with one) and 3 (plain tiles).
-# Unsplit (adj_lite 0) only the relative order of 2 and 3 is told apart, so orders 0 (2 before 3) and 1 (3 before 2) represent all six.
+# Unsplit (adj_lite 0) the step is one launch whatever the order; orders 0 and 1
+# stand for the six there.
 REVERSE_ORDERS = ((4, 2, 3), (4, 3, 2), (2, 4, 3), (2, 3, 4), (3, 4, 2), (3, 2, 4))
 
 _memory_cache: dict = {}
@@ -85,9 +87,9 @@ def forward_candidates(limits: dict, current: dict) -> list:
 
 
 def reverse_candidates(limits: dict, current: dict) -> list:
-    """Reverse settings to time: every order of the split, and the two
-    distinct orders without it, as far as the limits allow (the current
-    setting first)."""
+    """Reverse settings to time: every order of the split, and the unsplit
+    launch under both order fields it is stored with, as far as the limits
+    allow (the current setting first)."""
     c = []
     if limits["adj_order"] > 0:
         if limits["adj_lite"]:
@@ -96,11 +98,11 @@ def reverse_candidates(limits: dict, current: dict) -> list:
     else:
         c.append({"adj_lite": 0, "adj_order": 0})
     cur = {"adj_lite": current["adj_lite"], "adj_order": current["adj_order"]}
-    if not cur["adj_lite"]:   # the representative of the current relative order of 2 and 3
+    if not cur["adj_lite"]:   # the stored order of the unsplit launch
         o = REVERSE_ORDERS[cur["adj_order"]]
         cur["adj_order"] = 0 if o.index(2) < o.index(3) else 1
     if limits.get("adj_persist", 0):
-        # the persistent launch runs variants 2, 4 and 3 over all three lists
+        # the persistent launch runs over all three lists of the split
         c = [dict(x, adj_persist=0) for x in c] + [{"adj_lite": 1, "adj_order": 0, "adj_persist": 1}]
         cur = (dict(cur, adj_persist=0) if not current.get("adj_persist", 0)
                else {"adj_lite": 1, "adj_order": 0, "adj_persist": 1})
@@ -139,6 +141,17 @@ def _time(fn, repeats, timer):
     return min(timer(fn) for _ in range(max(1, repeats)))
 
 
+def library_id() -> str:
+    """Digest of the built kernels: another build may give a launch field other
+    kernels or another meaning, so its timings say nothing about this one's."""
+    from ._lib import LIB_PATH
+    try:
+        with open(LIB_PATH, "rb") as f:
+            return hashlib.sha1(f.read()).hexdigest()
+    except OSError:
+        return ""
+
+
 def _load_cache(path):
     if path and os.path.exists(path):
         with open(path) as f:
@@ -163,7 +176,7 @@ def autotune(target, run_forward, run_reverse=None, *, signature=None, cache_pat
     timer = timer or cuda_timer
     key = None
     if signature is not None:
-        key = hashlib.sha1(json.dumps(signature, sort_keys=True, default=str).encode()).hexdigest()
+        key = hashlib.sha1(json.dumps([library_id(), signature], sort_keys=True, default=str).encode()).hexdigest()
         hit = _memory_cache.get(key) or _load_cache(cache_path).get(key)
         if hit is not None:
             target.set_launch_config(**hit)

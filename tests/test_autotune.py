@@ -175,6 +175,21 @@ def test_cache_by_signature(tmp_path, monkeypatch):
     assert not res3.cached and len(json.load(open(path))) == 2
 
 
+def test_cached_choice_is_for_one_build_of_the_kernels(tmp_path, monkeypatch):
+    """A choice stored by another build of the library is timed anew: the launch
+    fields may stand for other kernels there."""
+    path = str(tmp_path / "tune.json")
+    sig = {"device": "fake", "instances": []}
+    for build, best in (("a", 1), ("b", 0), ("a", 1)):
+        monkeypatch.setattr(at, "_memory_cache", {})
+        monkeypatch.setattr(at, "library_id", lambda b=build: b, raising=False)
+        t = FakeTarget(FULL)
+        timer, rf, rr, _ = _timer_for(t, lambda c: 5.0 if c["fwd_split"] == best else 9.0, lambda c: 5.0)
+        res = at.autotune(t, rf, rr, signature=sig, cache_path=path, timer=timer, repeats=1)
+        assert res.config["fwd_split"] == best and t.cur["fwd_split"] == best
+    assert res.cached and len(json.load(open(path))) == 2
+
+
 def test_launch_config_bindings_validate_fields():
     from rfx_b200 import engine
 
