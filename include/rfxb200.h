@@ -369,6 +369,13 @@ int rfxb_batch_adjoint_variant(const RfxbBatch* batch);
 int rfxb_plan_step_launches(const RfxbPlan* plan, int* fwd, int* rev);
 int rfxb_batch_step_launches(const RfxbBatch* batch, int* fwd, int* rev);
 
+/* How the last forward advance of a plan (or batch) ran (*route: 0 none yet, 1
+ * launches per step, 2 one launch for all steps with the state in shared memory)
+ * and the rows of the tiles of its one-launch-per-step lists (*tile_rows: 24 or
+ * 8, 0 for the generic kernels).  A diagnostic of this implementation. */
+int rfxb_plan_forward_route(const RfxbPlan* plan, int* route, int* tile_rows);
+int rfxb_batch_forward_route(const RfxbBatch* batch, int* route, int* tile_rows);
+
 /* Launch configuration of a plan's (or batch's) step launches: the choices
  * the autotuner (rfx_b200/autotune.py) searches.  Every setting computes the
  * same steps; they differ in how the tiles are split among kernel variants
@@ -438,6 +445,9 @@ int rfxb_batch_set_launch_config(RfxbBatch* batch, const RfxbLaunchConfig* confi
  * persistent kernels skip and report as RFXB_E_WORK.  Both leave the batch's
  * state invalid: only the status check is meaningful afterwards. */
 int rfxb_batch_debug_fault(RfxbBatch* batch, int cta, int wait_limit);
+/* on != 0: the one-launch advance of a small grid counts as refused by the
+ * driver, as a device without room for its cooperative launch would. */
+int rfxb_batch_debug_refuse_resident(RfxbBatch* batch, int on);
 int rfxb_batch_debug_poison(RfxbBatch* batch, int list, int index);
 
 /* Host only, no device needed: the work list (x ranges of (TY x 32) tiles)

@@ -140,6 +140,9 @@ SIGNATURES = {
     "rfxb_batch_set_launch_config": (C.c_int, [C.c_void_p, C.POINTER(RfxbLaunchConfig)]),
     "rfxb_debug_work_lists": (C.c_int, [C.c_int, C.POINTER(C.c_int32), C.c_int32, C.c_int32, C.POINTER(C.c_int32),
                                         C.c_int32, C.POINTER(C.c_int32)]),
+    "rfxb_plan_forward_route": (C.c_int, [C.c_void_p, C.POINTER(C.c_int), C.POINTER(C.c_int)]),
+    "rfxb_batch_forward_route": (C.c_int, [C.c_void_p, C.POINTER(C.c_int), C.POINTER(C.c_int)]),
+    "rfxb_batch_debug_refuse_resident": (C.c_int, [C.c_void_p, C.c_int]),
     "rfxb_batch_debug_fault": (C.c_int, [C.c_void_p, C.c_int, C.c_int]),
     "rfxb_batch_debug_poison": (C.c_int, [C.c_void_p, C.c_int, C.c_int]),
     "rfxb_forward_noalloc": (C.c_int, [C.POINTER(RfxbDesc), C.c_void_p, C.c_void_p, C.POINTER(C.c_void_p),

@@ -185,6 +185,8 @@ struct RfxbBatch {
   ResidentShape res{};
   size_t res_smem = 0;
   unsigned* d_resctr = nullptr;    // arrivals at the grid barrier
+  bool refuse_resident = false;    // test only: the resident launch counts as refused
+  int route = 0;                   // last forward advance: 0 none yet, 1 step launches, 2 one resident launch
   bool fwd_split = false;
   bool fwd_split_avail = false;   // both forward lists exist (fwd_split may be chosen)
   int fwd_order = 0;              // split forward: 0 plain-tile launch first, 1 CPML-tile launch first
@@ -1604,15 +1606,27 @@ bool resident_route(const RfxbBatch* g, bool observers, int step0, int n_steps, 
   return cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
 }
 
-int launch_resident(RfxbBatch* g, int step0, int n_steps, int par0, int ppar0, cudaStream_t st) {
+// *refused: the driver does not take the cooperative launch here (fewer SMs than
+// the partition was made for, no cooperative launches); nothing was enqueued but
+// the counter's reset.
+int launch_resident(RfxbBatch* g, int step0, int n_steps, int par0, int ppar0, cudaStream_t st, bool* refused) {
+  *refused = false;
   const void* k = reinterpret_cast<const void*>(fwd_resident_kernel);
   allow_smem(k, smem_optin() - 1024);
   RFXB_CUDA(cudaMemsetAsync(g->d_resctr, 0, sizeof(unsigned), st));
   const RfxbInst* inst = g->d_inst;
   int limit = g->wait_limit;
   void* args[] = {&inst, &g->res, &step0, &n_steps, &par0, &ppar0, &g->d_resctr, &limit};
-  RFXB_CUDA(cudaLaunchCooperativeKernel(k, dim3(g->res.nb[0] * g->res.nb[1] * g->res.nb[2]), dim3(RFXB_RES_THREADS),
-                                        args, g->res_smem, st));
+  const cudaError_t e =
+      g->refuse_resident ? cudaErrorCooperativeLaunchTooLarge
+                         : cudaLaunchCooperativeKernel(k, dim3(g->res.nb[0] * g->res.nb[1] * g->res.nb[2]),
+                                                       dim3(RFXB_RES_THREADS), args, g->res_smem, st);
+  if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorLaunchOutOfResources || e == cudaErrorNotSupported) {
+    cudaGetLastError();
+    *refused = true;
+    return 0;
+  }
+  RFXB_CUDA(e);
   return 0;
 }
 
@@ -1684,8 +1698,18 @@ int group_advance(RfxbBatch* g, const RfxbStepIO* ios, int step0, int n_steps, c
   // work, and their captured graphs measured slower to build and to replay
   // (1000 steps of a 513^3 grid: 0.9 s to capture, 1.58 s against 1.49 s per
   // replay)
-  if (resident_route(g, has_dft || has_flux || has_ntff, step0, n_steps, st)) {
-    if (int rc = launch_resident(g, step0, n_steps, par0, ppar0, st)) return rc;
+  bool resident = resident_route(g, has_dft || has_flux || has_ntff, step0, n_steps, st);
+  if (resident) {
+    bool refused = false;
+    if (int rc = launch_resident(g, step0, n_steps, par0, ppar0, st, &refused)) return rc;
+    if (refused) {   // step launches from here on
+      g->res = ResidentShape{};
+      resident = false;
+    }
+  }
+  g->route = resident ? 2 : 1;
+  if (resident) {
+    // every step is in the one launch
   } else if (graphs_enabled() && n_steps >= 4 && !two_step(g)) {
     const GraphKey key{0, step0, n_steps, par0, 0, (has_dft ? 1 : 0) | (has_flux ? 2 : 0) | (has_ntff ? 4 : 0),
                        ppar0};
@@ -2618,6 +2642,11 @@ int debug_fault(RfxbBatch* g, int cta, int wait_limit) {
   return 0;
 }
 
+void forward_route(const RfxbBatch* g, int* route, int* tile_rows) {
+  if (route) *route = g->route;
+  if (tile_rows) *tile_rows = g->fwd_mode >= 1 ? kFwdTile[g->vtile].ty : 0;
+}
+
 int debug_poison(RfxbBatch* g, int list, int index) {
   RfxbWork* lists[5] = {g->d_wf2, g->d_wf1, g->d_wa2y, g->d_wa4, g->d_wa1};
   const int counts[5] = {g->n_wf2, g->n_wf1, g->n_wa2y, g->n_wa4, g->n_wa1};
@@ -2635,6 +2664,24 @@ int debug_poison(RfxbBatch* g, int list, int index) {
 int rfxb_batch_debug_fault(RfxbBatch* g, int cta, int wait_limit) {
   if (!g) return fail(RFXB_E_INVALID, "null batch");
   return debug_fault(g, cta, wait_limit);
+}
+
+int rfxb_batch_debug_refuse_resident(RfxbBatch* g, int on) {
+  if (!g) return fail(RFXB_E_INVALID, "null batch");
+  g->refuse_resident = on != 0;
+  return 0;
+}
+
+int rfxb_plan_forward_route(const RfxbPlan* p, int* route, int* tile_rows) {
+  if (!p || !p->self_group) return fail(RFXB_E_INVALID, "null plan");
+  forward_route(p->self_group, route, tile_rows);
+  return 0;
+}
+
+int rfxb_batch_forward_route(const RfxbBatch* g, int* route, int* tile_rows) {
+  if (!g) return fail(RFXB_E_INVALID, "null batch");
+  forward_route(g, route, tile_rows);
+  return 0;
 }
 
 int rfxb_batch_debug_poison(RfxbBatch* g, int list, int index) {

@@ -89,6 +89,12 @@ _LAUNCH_FIELDS = ("fwd_split", "fwd_order", "adj_lite", "adj_order", "fwd_persis
                   "fwd_depth")
 
 
+def _forward_route(fn, handle):
+    route, rows = C.c_int(), C.c_int()
+    check(fn(handle, C.byref(route), C.byref(rows)), fn.__name__)
+    return route.value, rows.value
+
+
 def _get_launch(getter, h):
     cur, lim = RfxbLaunchConfig(), RfxbLaunchConfig()
     check(getter(h, C.byref(cur), C.byref(lim)), getter.__name__)
@@ -320,6 +326,11 @@ class Plan:
         check(self._lib.rfxb_plan_step_launches(self._h, C.byref(f), C.byref(r)), "rfxb_plan_step_launches")
         return f.value, r.value
 
+    def forward_route(self):
+        """(how the last forward advance ran: 0 none yet, 1 launches per step,
+        2 one launch for all steps; rows of the one-launch-per-step tiles)."""
+        return _forward_route(self._lib.rfxb_plan_forward_route, self._h)
+
     def launch_config(self):
         """(current, limits) launch configuration dicts (``rfxb200.h``
         ``RfxbLaunchConfig``: fwd_split, fwd_order, adj_lite, adj_order)."""
@@ -535,6 +546,10 @@ class Batch:
         f, r = C.c_int(), C.c_int()
         check(self._lib.rfxb_batch_step_launches(self._h, C.byref(f), C.byref(r)), "rfxb_batch_step_launches")
         return f.value, r.value
+
+    def forward_route(self):
+        """As ``Plan.forward_route``, for the whole batch."""
+        return _forward_route(self._lib.rfxb_batch_forward_route, self._h)
 
     def launch_config(self):
         """(current, limits) launch configuration dicts, as ``Plan.launch_config``."""

@@ -10,8 +10,10 @@ and probes than one mask word holds.
 
 import numpy as np
 import pytest
+import torch
 
-from rfx_b200 import workloads
+from rfx_b200 import _lib, workloads
+from rfx_b200.engine import Batch
 from rfx_b200.grid import Grid, make_nonuniform_grid
 from rfx_b200.simulation import MaterialArrays, prepare_device_run
 from tests.test_gpu_fullsize import _advance, _random_fields
@@ -67,4 +69,43 @@ def test_resident_advance_on_graded_spacing(cuda):
     try:
         _compare(r, g.shape, n)
     finally:
+        r.plan.close()
+
+
+def _small_run(n, seed=4):
+    shape, rng = (33, 29, 31), np.random.default_rng(seed)
+    g = Grid(freq_max=20e9, domain=tuple((s - 13) * 1e-3 for s in shape), dx=1e-3, cpml_layers=6)
+    eps = (1.0 + rng.random(shape)).astype(np.float32)
+    return prepare_device_run(g, MaterialArrays(eps, np.zeros(shape, np.float32), np.ones(shape, np.float32)), n,
+                              cpml_axes="xyz", pec_axes="",
+                              sources=[(16, 14, 15, "ez", rng.standard_normal(n).astype(np.float32))],
+                              probes=[(18, 14, 15, "ez")], dft_planes=[], pec_mask=None, dft_time_offset=1)
+
+
+def _batch_advance(r, b, n):
+    r.plan.reset()
+    r.probe_out.zero_()
+    b.advance(0, n, [dict(src_table=r.src_table, probe_out=r.probe_out)])
+    torch.cuda.synchronize()
+    b.check_device()
+    return [r.probe_out.cpu().numpy().copy()] + [f.cpu().numpy().copy() for f in r.plan.store_fields()]
+
+
+def test_refused_resident_launch_takes_step_launches(cuda):
+    """A cooperative launch that the driver does not take (the launch is not made
+    here, its error code is) leaves the advance to the step launches."""
+    n = 12
+    r = _small_run(n)
+    b = Batch([r.plan])
+    try:
+        ref = _batch_advance(r, b, n)
+        assert b.forward_route()[0] == 2 and np.abs(ref[0]).max() > 0
+        assert _lib.load().rfxb_batch_debug_refuse_resident(b._h, 1) == 0
+        for _ in range(2):
+            got = _batch_advance(r, b, n)
+            assert b.forward_route()[0] == 1
+            for x, y in zip(ref, got):
+                assert np.array_equal(x, y)
+    finally:
+        b.close()
         r.plan.close()
