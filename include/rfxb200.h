@@ -454,17 +454,25 @@ int rfxb_batch_debug_poison(RfxbBatch* batch, int list, int index);
  * that a batch of plans with these shapes launches for one step, for tests
  * of the tiling.  dims: 5 ints per plan (nx, ny, nz, CPML layers, CPML axes
  * bits x=1 y=2 z=4); resident: the CTA capacity the lists are balanced for.
- * which: 0 every tile on one kernel; 1 / 2 forward CPML-free / staged-psi
- * tiles; 3 / 4 reverse CPML-free / CPML tiles; 5 / 6 the reverse CPML tiles
- * split into those that reach a y slab (variant 2) and the rest (variant 4);
- * 7 / 8 / 9 a two-step pass's two-step tiles / one-step CPML-free work /
- * one-step CPML work (for 7 the plan index carries, from bit 16 on, where the
- * item also stores its intermediate state: 1 every plane, 2 its first plane,
- * 4 its last plane).
+ * which: 0 every tile, for the generic kernels; 1 / 2 the split forward's
+ * CPML-free / CPML tiles; 3 / 4 reverse CPML-free / CPML tiles, 4 split for the
+ * launch into 5 / 6, those that reach a y slab and the rest; 7 / 8 / 9 a
+ * two-step pass's two-step segments before they are merged into items (those:
+ * rfxb_debug_launch_items) / one-step CPML-free work / one-step CPML work (for 7
+ * the plan index carries, from bit 16 on, where the segment also stores its
+ * intermediate state: 1 every plane, 2 its first plane, 4 its last plane).
  * out: 5 ints per item (plan, y0, z0, xa, xb), *n_out the item count (with
  * out == NULL only the count).  A diagnostic of this implementation. */
 int rfxb_debug_work_lists(int n_plans, const int32_t* dims, int32_t resident, int32_t which, int32_t* out,
                           int32_t cap, int32_t* n_out);
+
+/* The same for the lists of the default launches, 8 ints per item (plan, y0, yb,
+ * z0, zb, xa, xb, flags; cells [y0, yb) x [z0, zb) x [xa, xb)).  which: 0 / 1 the
+ * single forward launch on 24 x 32 / 8 x 32 tiles, 2 / 3 the single reverse
+ * launch (flags 1: the item runs the CPML-free code); 4 the two-step kernel's
+ * items (flags: 1 / 2 / 4 as above, 8 the path that guards grid faces). */
+int rfxb_debug_launch_items(int n_plans, const int32_t* dims, int32_t resident, int32_t which, int32_t* out,
+                            int32_t cap, int32_t* n_out);
 
 #ifdef __cplusplus
 }

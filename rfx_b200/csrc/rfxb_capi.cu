@@ -650,8 +650,9 @@ void depth2_items(const std::vector<RfxbPlan*>& plans, const std::vector<WorkSeg
   constexpr int kRows = RFXB_D2ROWS - 3, kCols = RFXB_D2COLS - 8;
   std::map<std::tuple<int, int, int>, std::set<std::pair<int, int>>> groups;   // (plan, xa, xb) -> columns
   for (const WorkSeg& s : d2) groups[{s.inst, s.xa, s.xb}].insert({s.y0, s.z0});
+  struct Piece { int yb, zb, xa, xb; };
   std::vector<WorkSeg> segs;
-  std::map<std::tuple<int, int, int>, std::pair<int, int>> ends;   // (plan, y0, z0) -> (yb, zb)
+  std::map<std::tuple<int, int, int>, std::vector<Piece>> pieces;   // (plan, y0, z0) -> the rectangles that start there
   for (auto& [key, cols] : groups) {
     const auto [inst, xa, xb] = key;
     const RfxbPlan& p = *plans[inst];
@@ -676,7 +677,7 @@ void depth2_items(const std::vector<RfxbPlan*>& plans, const std::vector<WorkSeg
         const int ya = y0 + (ye - y0) * a / my, yb = y0 + (ye - y0) * (a + 1) / my;
         for (int z = z0; z < ze; z += dz) {
           segs.push_back(WorkSeg{inst, ya, z, xa, xb, p.nx, 0, 1.0, 0.0});
-          ends[{inst, ya, z}] = {yb, std::min(z + dz, ze)};
+          pieces[{inst, ya, z}].push_back(Piece{yb, std::min(z + dz, ze), xa, xb});
         }
       }
     }
@@ -686,7 +687,12 @@ void depth2_items(const std::vector<RfxbPlan*>& plans, const std::vector<WorkSeg
   out.clear();
   for (const RfxbWork& w : items) {
     const RfxbPlan& p = *plans[w.inst];
-    const auto [yb, zb] = ends[{w.inst, w.y0, w.z0}];
+    int yb = 0, zb = 0;
+    for (const Piece& c : pieces[{w.inst, w.y0, w.z0}])
+      if (w.xa >= c.xa && w.xb <= c.xb) {
+        yb = c.yb;
+        zb = c.zb;
+      }
     int mid = 0;
     for (int y = w.y0 / kTY * kTY; y < yb; y += kTY)
       for (int z = w.z0 / 32 * 32; z < zb; z += 32) mid |= depth2_mid_flags(p, RfxbWork{w.inst, y, z, w.xa, w.xb});
@@ -736,6 +742,18 @@ const SlabCost kFwdCost(0.4, 0.1, 0.7, 0.15), kAdjCost(0.3, 0.3, 0.3, 0.1);
 // start-up evaluates two planes of fluxes (100 us at one wave, 113 at three).
 constexpr double kFwdPrologue = 0.3, kAdjPrologue = 3.0;
 constexpr int kFwdWaves = 4, kAdjWaves = 1;
+
+// The list of a forward or reverse step in one launch, tiles of ty x tz cells;
+// items that need no CPML term carry RFXB_WORK_PLAIN.
+void single_launch_items(const std::vector<RfxbPlan*>& plans, bool reverse, int ty, int tz, int resident,
+                         std::vector<RfxbWork>& out) {
+  std::vector<WorkSeg> segs, cpml;
+  if (reverse) split_adj_segments(plans, kAdjCost, segs, cpml, nullptr, ty, tz);
+  else split_segments(plans, kFwdCost, segs, cpml, ty, tz);
+  for (WorkSeg& s : segs) s.inst |= RFXB_WORK_PLAIN;
+  segs.insert(segs.end(), cpml.begin(), cpml.end());
+  balance_segments(segs, resident, reverse ? kAdjPrologue : kFwdPrologue, out, reverse ? kAdjWaves : kFwdWaves);
+}
 
 // RFXB_ADJ_LITE=1 starts groups with CPML on the split reverse launches.
 bool adj_lite_enabled() {
@@ -1177,27 +1195,16 @@ int build_group(RfxbBatch* g) {
     if (g->res.nb[0] > 0)
       if (int rc = galloc((void**)&g->d_resctr, sizeof(unsigned))) return rc;
   }
-  // the single-launch forward list
+  // the single-launch lists
   if (g->fwd_mode >= 1) {
     g->vtile = pick_fwd_tile(g);
     const FwdTile& T = kFwdTile[g->vtile];
-    std::vector<WorkSeg> segs, cpml;
-    split_segments(g->plans, kFwdCost, segs, cpml, T.ty, T.tz);
-    auto merge = [&]() {
-      for (WorkSeg& s : segs) s.inst |= RFXB_WORK_PLAIN;
-      segs.insert(segs.end(), cpml.begin(), cpml.end());
-    };
-    merge();
     std::vector<RfxbWork> wv;
-    balance_segments(segs, resident_ctas(g->vtile, g->fwd_mode == 2), kFwdPrologue, wv, kFwdWaves);
+    single_launch_items(g->plans, false, T.ty, T.tz, resident_ctas(g->vtile, g->fwd_mode == 2), wv);
     if (int rc = galloc((void**)&g->d_wv, sizeof(RfxbWork) * wv.size())) return rc;
     RFXB_CUDA(cudaMemcpy(g->d_wv, wv.data(), sizeof(RfxbWork) * wv.size(), cudaMemcpyHostToDevice));
     g->n_wv = (int)wv.size();
-    segs.clear();
-    cpml.clear();
-    split_adj_segments(g->plans, kAdjCost, segs, cpml, nullptr, T.ty, T.tz);
-    merge();
-    balance_segments(segs, (g->vtile == 0 ? 2 : 5) * sm_count(), kAdjPrologue, wv, kAdjWaves);
+    single_launch_items(g->plans, true, T.ty, T.tz, (g->vtile == 0 ? 2 : 5) * sm_count(), wv);
     if (int rc = galloc((void**)&g->d_wva, sizeof(RfxbWork) * wv.size())) return rc;
     RFXB_CUDA(cudaMemcpy(g->d_wva, wv.data(), sizeof(RfxbWork) * wv.size(), cudaMemcpyHostToDevice));
     g->n_wva = (int)wv.size();
@@ -2711,16 +2718,14 @@ int rfxb_batch_set_launch_config(RfxbBatch* g, const RfxbLaunchConfig* config) {
   return set_launch_config(g, config);
 }
 
-int rfxb_debug_work_lists(int n_plans, const int32_t* dims, int32_t resident, int32_t which, int32_t* out,
-                          int32_t cap, int32_t* n_out) {
-  if (n_plans <= 0 || !dims || resident <= 0 || which < 0 || which > 9 || !n_out)
-    return fail(RFXB_E_INVALID, "rfxb_debug_work_lists: bad arguments");
-  std::vector<std::unique_ptr<RfxbPlan>> own;
-  std::vector<RfxbPlan*> plans;
+namespace {
+// Host-only plans of the given shapes, for the work-list diagnostics.
+int plans_of_dims(int n_plans, const int32_t* dims, std::vector<std::unique_ptr<RfxbPlan>>& own,
+                  std::vector<RfxbPlan*>& plans) {
   for (int q = 0; q < n_plans; ++q) {
     const int32_t* d = dims + 5 * q;
     if (d[0] < 2 || d[1] < 2 || d[2] < 2 || d[3] < 0 || d[4] < 0 || d[4] > 7)
-      return fail(RFXB_E_INVALID, "rfxb_debug_work_lists: bad plan dims");
+      return fail(RFXB_E_INVALID, "work-list diagnostic: bad plan dims");
     auto p = std::make_unique<RfxbPlan>();
     p->nx = d[0];
     p->ny = d[1];
@@ -2730,6 +2735,52 @@ int rfxb_debug_work_lists(int n_plans, const int32_t* dims, int32_t resident, in
     plans.push_back(p.get());
     own.push_back(std::move(p));
   }
+  return 0;
+}
+}  // namespace
+
+int rfxb_debug_launch_items(int n_plans, const int32_t* dims, int32_t resident, int32_t which, int32_t* out,
+                            int32_t cap, int32_t* n_out) {
+  if (n_plans <= 0 || !dims || resident <= 0 || which < 0 || which > 4 || !n_out)
+    return fail(RFXB_E_INVALID, "rfxb_debug_launch_items: bad arguments");
+  std::vector<std::unique_ptr<RfxbPlan>> own;
+  std::vector<RfxbPlan*> plans;
+  if (int rc = plans_of_dims(n_plans, dims, own, plans)) return rc;
+  std::vector<RfxbWork2> items;
+  if (which == 4) {
+    std::vector<WorkSeg> d2, plain, cpml;
+    split_depth2_segments(plans, slab_weight(), d2, plain, cpml);
+    depth2_items(plans, d2, resident, items);
+  } else {
+    const FwdTile& T = kFwdTile[which & 1];
+    std::vector<RfxbWork> w;
+    single_launch_items(plans, which >= 2, T.ty, T.tz, resident, w);
+    for (const RfxbWork& it : w) {
+      const int q = it.inst & ~RFXB_WORK_PLAIN;
+      items.push_back(RfxbWork2{q, it.y0, std::min(it.y0 + T.ty, plans[q]->ny), it.z0,
+                                std::min(it.z0 + T.tz, plans[q]->nz), it.xa, it.xb,
+                                (it.inst & RFXB_WORK_PLAIN) ? 1 : 0});
+    }
+  }
+  *n_out = (int32_t)items.size();
+  if (!out) return 0;
+  if (cap < (int32_t)items.size())
+    return fail(RFXB_E_INVALID, "rfxb_debug_launch_items: output capacity too small");
+  for (size_t t = 0; t < items.size(); ++t) {
+    const RfxbWork2& w = items[t];
+    const int32_t v[8] = {w.inst, w.y0, w.yb, w.z0, w.zb, w.xa, w.xb, w.mid};
+    std::copy(v, v + 8, out + 8 * t);
+  }
+  return 0;
+}
+
+int rfxb_debug_work_lists(int n_plans, const int32_t* dims, int32_t resident, int32_t which, int32_t* out,
+                          int32_t cap, int32_t* n_out) {
+  if (n_plans <= 0 || !dims || resident <= 0 || which < 0 || which > 9 || !n_out)
+    return fail(RFXB_E_INVALID, "rfxb_debug_work_lists: bad arguments");
+  std::vector<std::unique_ptr<RfxbPlan>> own;
+  std::vector<RfxbPlan*> plans;
+  if (int rc = plans_of_dims(n_plans, dims, own, plans)) return rc;
   const double slab = slab_weight();
   std::vector<RfxbWork> w;
   if (which == 0) {
