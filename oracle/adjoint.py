@@ -136,7 +136,7 @@ def _cpml_transpose(st, aF, apsi, table, coef_full, fwd):
 
 def forward_adjoint(grid, materials, n_steps, *, nonuniform=False, boundary="cpml", cpml_axes="xyz",
                     pec_axes=None, sources=(), probes=(), pec_mask=None, box, objective_grad,
-                    dtype=np.float64):
+                    dtype=np.float64, kappa_max=1.0):
     """Forward run, then the reverse sweep.
 
     ``objective_grad(ts) -> g`` maps the probe traces (n_steps, n_probes) to
@@ -148,7 +148,7 @@ def forward_adjoint(grid, materials, n_steps, *, nonuniform=False, boundary="cpm
         axes = cpml_axes if boundary == "cpml" else ""
         pec_axes = "xyz" if pec_axes is None else pec_axes
     st = _RecStepper(grid, materials, dtype=dtype, nonuniform=nonuniform, cpml_axes=axes,
-                     pec_axes=pec_axes, pec_mask=pec_mask, box=box)
+                     pec_axes=pec_axes, pec_mask=pec_mask, kappa_max=kappa_max, box=box)
     f = st.f
     ts = np.zeros((n_steps, len(probes)), f)
     for n in range(n_steps):

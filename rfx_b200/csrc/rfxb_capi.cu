@@ -2103,17 +2103,20 @@ int rfxb_plan_create(const RfxbDesc* d, RfxbPlan** out) {
       if (!(d->cpml_cell[f] > 0.0)) return bail(fail(RFXB_E_INVALID, "CPML cell sizes must be positive"));
       I.ib[f] = (float)(1.0 / d->cpml_cell[f]);
     }
-    // (b, c / cell, (1/kappa - 1) / cell) per face and layer for the staged-psi kernel
-    std::vector<float4> t4(6 * ncp);
+    // per face and layer: the reverse kernels' table, then the forward kernels'
+    std::vector<float4> t4(12 * ncp);
     for (int f = 0; f < 6; ++f)
-      for (int s = 0; s < ncp; ++s)
-        t4[f * ncp + s] = make_float4(tb[(f * 3 + 0) * ncp + s], (float)((double)tb[(f * 3 + 1) * ncp + s] * I.ib[f]),
-                                      (float)((double)tb[(f * 3 + 2) * ncp + s] * I.ib[f]), 0.f);
+      for (int s = 0; s < ncp; ++s) {
+        const float b = tb[(f * 3 + 0) * ncp + s], c = tb[(f * 3 + 1) * ncp + s], km = tb[(f * 3 + 2) * ncp + s];
+        t4[f * ncp + s] = make_float4(b, (float)((double)c * I.ib[f]), (float)((double)km * I.ib[f]), 0.f);
+        t4[(6 + f) * ncp + s] = make_float4(b, c, km, I.ib[f]);
+      }
     float4* dct = nullptr;
     if (int rc = p->alloc(&dct, t4.size())) return bail(rc);
     if (cudaMemcpy(dct, t4.data(), t4.size() * sizeof(float4), cudaMemcpyHostToDevice) != cudaSuccess)
       return bail(fail(RFXB_E_LAUNCH, "cudaMemcpy"));
     I.cpt = dct;
+    I.cpu = dct + 6 * ncp;
     p->psi_elems[0] = 4LL * ncp * d->ny * I.zs;
     p->psi_elems[1] = 4LL * d->nx * ncp * I.zs;
     p->psi_elems[2] = 4LL * d->nx * d->ny * I.ncp4;

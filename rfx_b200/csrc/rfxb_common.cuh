@@ -91,6 +91,18 @@ __device__ __forceinline__ float yee_e(float ca, float e, float cb, float curl) 
   return __fmaf_rn(cb, curl, __fmul_rn(ca, e));
 }
 
+// CPML of the forward step, from a field difference over a cell, g = difference *
+// (1 / cell):  psi' = b psi + c g,  f + s (psi' + km g).  c and km are the tables'
+// own values: with 1 / cell folded into them each coefficient is rounded once
+// more, alike in every step (error against float64 up to 1.13 times this one's
+// over grids of 43x37x33 to 72x70x75), and the operations are as many.
+__device__ __forceinline__ float psi_next(float b, float psi, float c, float g) {
+  return __fmaf_rn(c, g, __fmul_rn(b, psi));
+}
+__device__ __forceinline__ float psi_add(float f, float s, float p, float km, float g) {
+  return __fmaf_rn(s, __fmaf_rn(km, g, p), f);
+}
+
 // Buffer selector of a forward step launch: the field state is read from
 // F[in] and written to F[out] (0 and 1: the ping-pong pair; 2: the
 // intermediate state of a two-step pass), the CPML psi are read from parity

@@ -64,7 +64,7 @@ struct __align__(128) VSmem {
   float h[2][2][TY][D::TZ];               // hx, hz of plane i in slot i & 1: rows y0-1 .. y0+TY-2
   float hc[2][2][TY];                     // hx, hy of column z0-1
   float zt[2][D::TZ];                     // zh, ze of the tile's columns
-  float zp[3][D::TZ];                     // z profile of the columns (b, c/cell, (1/kappa-1)/cell)
+  float zp[3][D::TZ];                     // z profile of the columns (b, c, 1/kappa-1)
   float ps[CP ? RFXB_PSLOTS : 1][CP ? D::MAIN : 1][4];
   RfxbInst P;
   unsigned long long mbar[RFXB_VBARS];    // E stages, H stages, coefficient stages
@@ -74,55 +74,48 @@ struct __align__(128) VSmem {
 struct VSlab {
   bool y = false;              // in a y slab
   unsigned z = 0u;             // cells in a z slab (zslab_of)
-  float4 cy;                   // y profile (b, c/cell, (1/kappa-1)/cell)
+  float4 cy;                   // y profile (b, c, 1/kappa-1, 1/cell)
   int oy = 0;                  // y psi element of (q 0, plane 0): + i * ncp * zs
   int oz = 0;                  // z psi element of the first cell's (q 0, plane 0): + i * ny * ncp4
 };
 
-// psi' = b psi + c g
-__device__ __forceinline__ float psi_next(float b, float psi, float c, float g) {
-  return __fmaf_rn(c, g, __fmul_rn(b, psi));
-}
-// f + s (psi' + km g), the two terms added one after the other
-__device__ __forceinline__ float psi_add(float f, float s, float p, float km, float g) {
-  return __fmaf_rn(s, __fmul_rn(km, g), __fmaf_rn(s, p, f));
-}
-
-// One psi term of an x or y slab: f += SGN s (psi' + km g) from the old psi p,
-// psi' written to `out` when WRITE; with K, k += SGN (psi' + km g) (the gradient history's
-// correction before its scaling).
+// One psi term of an x or y slab from the differences d and the old psi p:
+// f += SGN s (psi' + km g), psi' written to `out` when WRITE; with K,
+// k += SGN (psi' + km g) (the gradient history's correction before its scaling).
 template <int L, int SGN, bool WRITE, bool K>
 __device__ __forceinline__ void psi_xy(Vec<L>& f, const Vec<L>& s, Vec<L> p, float* out, const float4& c,
-                                       const Vec<L>& g, Vec<L>& k, bool rec = false) {
+                                       const Vec<L>& d, Vec<L>& k, bool rec = false) {
 #pragma unroll
   for (int l = 0; l < L; ++l) {
-    p[l] = psi_next(c.x, p[l], c.y, g[l]);
-    f[l] = psi_add(f[l], SGN > 0 ? s[l] : -s[l], p[l], c.z, g[l]);
+    const float g = __fmul_rn(d[l], c.w);
+    p[l] = psi_next(c.x, p[l], c.y, g);
+    f[l] = psi_add(f[l], SGN > 0 ? s[l] : -s[l], p[l], c.z, g);
   }
   if (K && rec) {
 #pragma unroll
     for (int l = 0; l < L; ++l) {
-      const float t = __fmaf_rn(c.z, g[l], p[l]);
+      const float t = __fmaf_rn(c.z, __fmul_rn(d[l], c.w), p[l]);
       k[l] = SGN > 0 ? __fadd_rn(k[l], t) : __fsub_rn(k[l], t);
     }
   }
   if (WRITE) vst<L>(out, p);
 }
-// The same for a z slab: profile per column, psi at the columns' layers.
+// The same for a z slab: profile per column, psi at the columns' layers, ib = 1/cell.
 template <int L, int SGN, bool WRITE, bool K>
 __device__ __forceinline__ void psi_z(Vec<L>& f, const Vec<L>& s, Vec<L> p, float* out, unsigned m, const float* zp,
-                                      int zstride, const Vec<L>& g, Vec<L>& k, bool rec = false) {
+                                      int zstride, float ib, const Vec<L>& d, Vec<L>& k, bool rec = false) {
   const Vec<L> b = vld<L>(zp), c = vld<L>(zp + zstride), km = vld<L>(zp + 2 * zstride);
 #pragma unroll
   for (int l = 0; l < L; ++l) {
-    p[l] = psi_next(b[l], p[l], c[l], g[l]);
-    if ((m >> l) & 1u) f[l] = psi_add(f[l], SGN > 0 ? s[l] : -s[l], p[l], km[l], g[l]);
+    const float g = __fmul_rn(d[l], ib);
+    p[l] = psi_next(b[l], p[l], c[l], g);
+    if ((m >> l) & 1u) f[l] = psi_add(f[l], SGN > 0 ? s[l] : -s[l], p[l], km[l], g);
   }
   if (K && rec) {
 #pragma unroll
     for (int l = 0; l < L; ++l) {
       if (!((m >> l) & 1u)) continue;
-      const float t = __fmaf_rn(km[l], g[l], p[l]);
+      const float t = __fmaf_rn(km[l], __fmul_rn(d[l], ib), p[l]);
       k[l] = SGN > 0 ? __fadd_rn(k[l], t) : __fsub_rn(k[l], t);
     }
   }
@@ -138,7 +131,7 @@ template <int L, int MASK, bool CP, bool WRITE, int EW, int CE, class Hold, clas
 __device__ __forceinline__ void h_vec(const float* A, const float* B, int o, const Vec<L>* e0, float exz, float eyz,
                                       Hold&& hold, Old&& old, float xh, float yh, const Vec<L>& zh, const Vec<L>& ch,
                                       const RfxbInst& P, int par, bool xon, const float4& cx, int ox, const VSlab& S,
-                                      const float* zp, int i, int qx, int qy, int qz, int ncp, Vec<L>& hx, Vec<L>& hy,
+                                      const float* zp, float ibz, int i, int qx, int qy, int qz, int ncp, Vec<L>& hx, Vec<L>& hy,
                                       Vec<L>& hz) {
   constexpr int ZS = EW - 8;
   const int iy = S.oy + i * ncp * P.zs, iz = S.oz + i * P.ny * P.ncp4;
@@ -154,7 +147,7 @@ __device__ __forceinline__ void h_vec(const float* A, const float* B, int o, con
     }
     if (CP && S.y) psi_xy<L, -1, WRITE, false>(hx, ch, old(1, 0), P.psH[par ^ 1][1] + iy, S.cy, gy, none);
     if (CP && S.z)
-      psi_z<L, +1, WRITE, false>(hx, ch, old(2, 0), P.psH[par ^ 1][2] + iz, S.z, zp, ZS, gz, none);
+      psi_z<L, +1, WRITE, false>(hx, ch, old(2, 0), P.psH[par ^ 1][2] + iz, S.z, zp, ZS, ibz, gz, none);
   }
   if (MASK & 2) {   // Hy += ch psi(dEz/dx) [x q0], Hy -= ch psi(dEx/dz) [z q1]
     Vec<L> gx = vld<L>(B + o + 2 * CE), gz;
@@ -167,7 +160,7 @@ __device__ __forceinline__ void h_vec(const float* A, const float* B, int o, con
     }
     if (CP && xon) psi_xy<L, +1, WRITE, false>(hy, ch, old(0, 0), P.psH[par ^ 1][0] + ox, cx, gx, none);
     if (CP && S.z)
-      psi_z<L, -1, WRITE, false>(hy, ch, old(2, 1), P.psH[par ^ 1][2] + iz + qz, S.z, zp, ZS, gz, none);
+      psi_z<L, -1, WRITE, false>(hy, ch, old(2, 1), P.psH[par ^ 1][2] + iz + qz, S.z, zp, ZS, ibz, gz, none);
   }
   if (MASK & 4) {   // Hz -= ch psi(dEy/dx) [x q1], Hz += ch psi(dEx/dy) [y q1]
     Vec<L> gx = vld<L>(B + o + CE), gy = vld<L>(A + o + EW);
@@ -252,8 +245,8 @@ __device__ __forceinline__ bool fwdv_item(VSmem<TY, ZQ, CP>& S, const RfxbInst* 
     S.zt[1][t] = k < nz ? __ldg(P.ze + k) : 0.f;
     if (CP) {
       float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (cpz && k < ncp) c = __ldg(P.cpt + 4 * ncp + k);
-      else if (cpz && k >= kb && k < nz) c = __ldg(P.cpt + 5 * ncp + (k - kb));
+      if (cpz && k < ncp) c = __ldg(P.cpu + 4 * ncp + k);
+      else if (cpz && k >= kb && k < nz) c = __ldg(P.cpu + 5 * ncp + (k - kb));
       S.zp[0][t] = c.x;
       S.zp[1][t] = c.y;
       S.zp[2][t] = c.z;
@@ -293,7 +286,7 @@ __device__ __forceinline__ bool fwdv_item(VSmem<TY, ZQ, CP>& S, const RfxbInst* 
     if (cpy && (j < ncp || j >= jb)) {
       const int sd = j < ncp ? 0 : 1, s = sd ? j - jb : j;
       B.y = true;
-      B.cy = __ldg(P.cpt + (2 + sd) * ncp + s);
+      B.cy = __ldg(P.cpu + (2 + sd) * ncp + s);
       B.oy = 2 * sd * qy + s * zs + k;
     }
     if (cpz) {
@@ -306,7 +299,7 @@ __device__ __forceinline__ bool fwdv_item(VSmem<TY, ZQ, CP>& S, const RfxbInst* 
   auto xslab = [&](int p, float4& c, int& base) -> bool {
     if (!CP || !cpx || p < 0 || (p >= ncp && p < nx - ncp) || p >= nx) return false;
     const int sd = p < ncp ? 0 : 1, s = sd ? p - (nx - ncp) : p;
-    c = __ldg(P.cpt + sd * ncp + s);
+    c = __ldg(P.cpu + sd * ncp + s);
     base = 2 * sd * qx + s * ny * zs;
     return true;
   };
@@ -359,6 +352,7 @@ __device__ __forceinline__ bool fwdv_item(VSmem<TY, ZQ, CP>& S, const RfxbInst* 
     const int jk = j * zs + k;
     const float yh = own ? __ldg(P.yh + j) : 0.f, ye = own ? __ldg(P.ye + j) : 0.f;
     const float* zp = &S.zp[0][4 * zq];
+    const float ibz = CP ? P.ib[4 + (k >= ncp)] : 0.f;
     const bool last_q = zq == ZQ - 1, first_q = zq == 0;
     // sources and probes in this thread's columns
     unsigned smask = 0u, pmask = 0u;
@@ -415,7 +409,7 @@ __device__ __forceinline__ bool fwdv_item(VSmem<TY, ZQ, CP>& S, const RfxbInst* 
               if (a == 1) return vld<4>(p + B.oy + (xa - 1) * ncp * zs + q * qy);
               return zpsi_load<4>(p + B.oz + (xa - 1) * ny * n4 + q * qz, B.z);
             },
-            __ldg(xh_tab + xa - 1), yh, vld<4>(&S.zt[0][4 * zq]), ch, P, par, xon, cx, xbase + jk, B, zp, xa - 1, qx, qy, qz,
+            __ldg(xh_tab + xa - 1), yh, vld<4>(&S.zt[0][4 * zq]), ch, P, par, xon, cx, xbase + jk, B, zp, ibz, xa - 1, qx, qy, qz,
             ncp, t, hyp, hzp);
       }
 #pragma unroll
@@ -465,7 +459,7 @@ __device__ __forceinline__ bool fwdv_item(VSmem<TY, ZQ, CP>& S, const RfxbInst* 
                 if (a == 0 && B.y) return vld<4>(P.psH[par][0] + xbase + jk + q * qx);
                 return vld<4>(slot + (a == 2 ? 4 + q : q) * SS);
               },
-              xh, yh, vld<4>(&S.zt[0][4 * zq]), ch, P, par, xon, cx, xbase + jk, B, zp, i, qx, qy, qz, ncp, hx, hy, hz);
+              xh, yh, vld<4>(&S.zt[0][4 * zq]), ch, P, par, xon, cx, xbase + jk, B, zp, ibz, i, qx, qy, qz, ncp, hx, hy, hz);
           if (kv < 4) {
 #pragma unroll
             for (int l = 1; l < 4; ++l)
@@ -518,7 +512,7 @@ __device__ __forceinline__ bool fwdv_item(VSmem<TY, ZQ, CP>& S, const RfxbInst* 
           }
           if (CP && B.y) psi_xy<4, +1, true, true>(ex, ce, vld<4>(slot + 2 * SS), P.psE[par ^ 1][1] + iy, B.cy, gy, kk, hist_i);
           if (CP && B.z)
-            psi_z<4, -1, true, true>(ex, ce, vld<4>(slot + 6 * SS), P.psE[par ^ 1][2] + iz, B.z, zp, 4 * ZQ, gz, kk, hist_i);
+            psi_z<4, -1, true, true>(ex, ce, vld<4>(slot + 6 * SS), P.psE[par ^ 1][2] + iz, B.z, zp, 4 * ZQ, ibz, gz, kk, hist_i);
           if (hist_i) keep(0, cu);
         }
         {   // Ey -= ce psi(dHz/dx) [x q0], Ey += ce psi(dHx/dz) [z q1]
@@ -532,7 +526,7 @@ __device__ __forceinline__ bool fwdv_item(VSmem<TY, ZQ, CP>& S, const RfxbInst* 
           }
           if (CP && xon) psi_xy<4, -1, true, true>(ey, ce, vld<4>(B.y ? P.psE[par][0] + ix : slot + 2 * SS), P.psE[par ^ 1][0] + ix, cx, gx, kk, hist_i);
           if (CP && B.z)
-            psi_z<4, +1, true, true>(ey, ce, vld<4>(slot + 7 * SS), P.psE[par ^ 1][2] + iz + qz, B.z, zp, 4 * ZQ, gz, kk, hist_i);
+            psi_z<4, +1, true, true>(ey, ce, vld<4>(slot + 7 * SS), P.psE[par ^ 1][2] + iz + qz, B.z, zp, 4 * ZQ, ibz, gz, kk, hist_i);
           if (hist_i) keep(1, cu);
         }
         {   // Ez += ce psi(dHy/dx) [x q1], Ez -= ce psi(dHx/dy) [y q1]
@@ -671,8 +665,8 @@ __device__ __forceinline__ bool fwdv_item(VSmem<TY, ZQ, CP>& S, const RfxbInst* 
     float4 czc = make_float4(0.f, 0.f, 0.f, 0.f);
     if (colm) {
       zhc = __ldg(P.zh + k);
-      if (CP && cpz && k < ncp) czc = __ldg(P.cpt + 4 * ncp + k);
-      else if (CP && cpz && k >= kb) czc = __ldg(P.cpt + 5 * ncp + (k - kb));
+      if (CP && cpz && k < ncp) czc = __ldg(P.cpu + 4 * ncp + k);
+      else if (CP && cpz && k >= kb) czc = __ldg(P.cpu + 5 * ncp + (k - kb));
     }
     // the column's old hx, hy and old psi (x q0, y q0, z q0, q1), and the row's
     // old psi (x q1, y q0, q1, z q0), one plane ahead
@@ -738,7 +732,7 @@ __device__ __forceinline__ bool fwdv_item(VSmem<TY, ZQ, CP>& S, const RfxbInst* 
           h_vec<4, 5, CP, false, EW, CE>(
               A, Bp, o, e0, A[o + 4], A[o + 4 + CE], [&](int c) { return vld<4>(H + c * D::CH + 4 * lane); },
               [&](int a, int q) { return a == 0 ? pr[0] : a == 2 ? pr[3] : q == 0 ? pr[1] : pr[2]; }, xh, yh,
-              vld<4>(&S.zt[0][4 * lane]), ch, P, par, xon, cx, xbase + jk, B, &S.zp[0][4 * lane], i, qx, qy, qz, ncp, hx, hy,
+              vld<4>(&S.zt[0][4 * lane]), ch, P, par, xon, cx, xbase + jk, B, &S.zp[0][4 * lane], P.ib[4 + (k >= ncp)], i, qx, qy, qz, ncp, hx, hy,
               hz);
         }
         vst<4>(&S.h[sl][0][0][4 * lane], hx);
@@ -755,16 +749,17 @@ __device__ __forceinline__ bool fwdv_item(VSmem<TY, ZQ, CP>& S, const RfxbInst* 
           hy = yee_h(hcy, chv, yee_diff2(dEx_z, zhc, dEz_x, xh));
           if (CP) {
             if (xon) {
-              const float p = psi_next(cx.x, pc[0], cx.y, dEz_x);
-              hy = psi_add(hy, chv, p, cx.z, dEz_x);
+              const float g = __fmul_rn(dEz_x, cx.w);
+              hy = psi_add(hy, chv, psi_next(cx.x, pc[0], cx.y, g), cx.z, g);
             }
             if (B.y) {
-              const float p = psi_next(B.cy.x, pc[1], B.cy.y, dEz_y);
-              hx = psi_add(hx, -chv, p, B.cy.z, dEz_y);
+              const float g = __fmul_rn(dEz_y, B.cy.w);
+              hx = psi_add(hx, -chv, psi_next(B.cy.x, pc[1], B.cy.y, g), B.cy.z, g);
             }
             if (B.z) {
-              hx = psi_add(hx, chv, psi_next(czc.x, pc[2], czc.y, dEy_z), czc.z, dEy_z);
-              hy = psi_add(hy, -chv, psi_next(czc.x, pc[3], czc.y, dEx_z), czc.z, dEx_z);
+              const float g0 = __fmul_rn(dEy_z, czc.w), g1 = __fmul_rn(dEx_z, czc.w);
+              hx = psi_add(hx, chv, psi_next(czc.x, pc[2], czc.y, g0), czc.z, g0);
+              hy = psi_add(hy, -chv, psi_next(czc.x, pc[3], czc.y, g1), czc.z, g1);
             }
           }
         }

@@ -59,7 +59,8 @@ struct RfxbInst {
   int ncp4;                // ncp rounded up to a multiple of 4 (z psi row length)
   unsigned cpml_axes;      // bit a set -> axis a absorbs
   const float* cpb;        // [face][3][ncp]: b, c, (1/kappa - 1); face = 2*axis + side
-  const float4* cpt;       // [face][ncp]: (b, c / cell, (1/kappa - 1) / cell, 0)
+  const float4* cpt;       // [face][ncp]: (b, c / cell, (1/kappa - 1) / cell, 0), reverse step
+  const float4* cpu;       // [face][ncp]: (b, c, 1/kappa - 1, 1 / cell), forward step
   float ib[6];             // 1 / boundary cell size per face
   float* psH[2][3];        // H-side psi per axis, ping-pong
   float* psE[2][3];        // E-side psi per axis, ping-pong

@@ -49,13 +49,6 @@ size_t resident_smem_bytes(const ResidentShape& R, int n_axes) {
   return sizeof(RfxbInst) + 256 + 4 * resident_floats(R, n_axes);
 }
 
-__device__ __forceinline__ float res_psi(float b, float psi, float c, float g) {
-  return __fmaf_rn(c, g, __fmul_rn(b, psi));
-}
-__device__ __forceinline__ float res_add(float f, float s, float p, float km, float g) {
-  return __fmaf_rn(s, __fmul_rn(km, g), __fmaf_rn(s, p, f));
-}
-
 // All CTAs of the launch have arrived `gen` times: true, or false when the
 // bounded wait ran out.
 __device__ __forceinline__ bool grid_barrier(unsigned* ctr, unsigned target, int limit, int* ok_smem) {
@@ -148,10 +141,7 @@ fwd_resident_kernel(const RfxbInst* __restrict__ insts, ResidentShape R, int ste
       if (in && (axes & (1u << a))) {
         int s;
         const int sd = cpml_side(x, nn[a], ncp, s);
-        if (sd >= 0) {
-          c = __ldg(P.cpt + (2 * a + sd) * ncp + s);
-          c.w = 1.f;
-        }
+        if (sd >= 0) c = __ldg(P.cpu + (2 * a + sd) * ncp + s);
       }
       prof[po[a] + t] = c;
     }
@@ -254,27 +244,30 @@ fwd_resident_kernel(const RfxbInst* __restrict__ insts, ResidentShape R, int ste
       float hz = yee_h(H[2 * NH + t], ch, yee_diff2(dEy_x, xh[li], dEx_y, yh[lj]));
       if (v & RES_X) {
         const float4 c = prof[li];
-        const float p0 = res_psi(c.x, psH[0][t], c.y, dEz_x), p1 = res_psi(c.x, psH[0][NH + t], c.y, dEy_x);
+        const float g0 = __fmul_rn(dEz_x, c.w), g1 = __fmul_rn(dEy_x, c.w);
+        const float p0 = psi_next(c.x, psH[0][t], c.y, g0), p1 = psi_next(c.x, psH[0][NH + t], c.y, g1);
         psH[0][t] = p0;
         psH[0][NH + t] = p1;
-        hy = res_add(hy, ch, p0, c.z, dEz_x);
-        hz = res_add(hz, -ch, p1, c.z, dEy_x);
+        hy = psi_add(hy, ch, p0, c.z, g0);
+        hz = psi_add(hz, -ch, p1, c.z, g1);
       }
       if (v & RES_Y) {
         const float4 c = prof[po[1] + lj];
-        const float p0 = res_psi(c.x, psH[1][t], c.y, dEz_y), p1 = res_psi(c.x, psH[1][NH + t], c.y, dEx_y);
+        const float g0 = __fmul_rn(dEz_y, c.w), g1 = __fmul_rn(dEx_y, c.w);
+        const float p0 = psi_next(c.x, psH[1][t], c.y, g0), p1 = psi_next(c.x, psH[1][NH + t], c.y, g1);
         psH[1][t] = p0;
         psH[1][NH + t] = p1;
-        hx = res_add(hx, -ch, p0, c.z, dEz_y);
-        hz = res_add(hz, ch, p1, c.z, dEx_y);
+        hx = psi_add(hx, -ch, p0, c.z, g0);
+        hz = psi_add(hz, ch, p1, c.z, g1);
       }
       if (v & RES_Z) {
         const float4 c = prof[po[2] + lk];
-        const float p0 = res_psi(c.x, psH[2][t], c.y, dEy_z), p1 = res_psi(c.x, psH[2][NH + t], c.y, dEx_z);
+        const float g0 = __fmul_rn(dEy_z, c.w), g1 = __fmul_rn(dEx_z, c.w);
+        const float p0 = psi_next(c.x, psH[2][t], c.y, g0), p1 = psi_next(c.x, psH[2][NH + t], c.y, g1);
         psH[2][t] = p0;
         psH[2][NH + t] = p1;
-        hx = res_add(hx, ch, p0, c.z, dEy_z);
-        hy = res_add(hy, -ch, p1, c.z, dEx_z);
+        hx = psi_add(hx, ch, p0, c.z, g0);
+        hy = psi_add(hy, -ch, p1, c.z, g1);
       }
       H[t] = hx;
       H[NH + t] = hy;
@@ -302,27 +295,30 @@ fwd_resident_kernel(const RfxbInst* __restrict__ insts, ResidentShape R, int ste
         const float ce = __ldg(P.ce + e);
         if (v & RES_X) {
           const float4 c = prof[li + 1];
-          const float p0 = res_psi(c.x, psE[0][t], c.y, dHz_x), p1 = res_psi(c.x, psE[0][NC + t], c.y, dHy_x);
+          const float g0 = __fmul_rn(dHz_x, c.w), g1 = __fmul_rn(dHy_x, c.w);
+          const float p0 = psi_next(c.x, psE[0][t], c.y, g0), p1 = psi_next(c.x, psE[0][NC + t], c.y, g1);
           psE[0][t] = p0;
           psE[0][NC + t] = p1;
-          ey = res_add(ey, -ce, p0, c.z, dHz_x);
-          ez = res_add(ez, ce, p1, c.z, dHy_x);
+          ey = psi_add(ey, -ce, p0, c.z, g0);
+          ez = psi_add(ez, ce, p1, c.z, g1);
         }
         if (v & RES_Y) {
           const float4 c = prof[po[1] + lj + 1];
-          const float p0 = res_psi(c.x, psE[1][t], c.y, dHz_y), p1 = res_psi(c.x, psE[1][NC + t], c.y, dHx_y);
+          const float g0 = __fmul_rn(dHz_y, c.w), g1 = __fmul_rn(dHx_y, c.w);
+          const float p0 = psi_next(c.x, psE[1][t], c.y, g0), p1 = psi_next(c.x, psE[1][NC + t], c.y, g1);
           psE[1][t] = p0;
           psE[1][NC + t] = p1;
-          ex = res_add(ex, ce, p0, c.z, dHz_y);
-          ez = res_add(ez, -ce, p1, c.z, dHx_y);
+          ex = psi_add(ex, ce, p0, c.z, g0);
+          ez = psi_add(ez, -ce, p1, c.z, g1);
         }
         if (v & RES_Z) {
           const float4 c = prof[po[2] + lk + 1];
-          const float p0 = res_psi(c.x, psE[2][t], c.y, dHy_z), p1 = res_psi(c.x, psE[2][NC + t], c.y, dHx_z);
+          const float g0 = __fmul_rn(dHy_z, c.w), g1 = __fmul_rn(dHx_z, c.w);
+          const float p0 = psi_next(c.x, psE[2][t], c.y, g0), p1 = psi_next(c.x, psE[2][NC + t], c.y, g1);
           psE[2][t] = p0;
           psE[2][NC + t] = p1;
-          ex = res_add(ex, -ce, p0, c.z, dHy_z);
-          ey = res_add(ey, ce, p1, c.z, dHx_z);
+          ex = psi_add(ex, -ce, p0, c.z, g0);
+          ey = psi_add(ey, ce, p1, c.z, g1);
         }
       }
       if (v & (63u << RES_PEC)) {
