@@ -434,12 +434,15 @@ int rfxb_plan_set_launch_config(RfxbPlan* plan, const RfxbLaunchConfig* config);
 int rfxb_batch_launch_config(const RfxbBatch* batch, RfxbLaunchConfig* current, RfxbLaunchConfig* limits);
 int rfxb_batch_set_launch_config(RfxbBatch* batch, const RfxbLaunchConfig* config);
 
-/* Test hooks of the persistent step kernels (no counterpart in the
- * reference).  debug_fault: from the next launch on, the CTA with block
- * index `cta` (-1: none) does not load plane xa of its first work item, and
- * every pipeline wait gives up after `wait_limit` polls, so that CTA's wait
- * runs out and rfxb_*_device_status reports RFXB_E_TIMEOUT (no box is left
- * in flight: the CTA drains the others before leaving).  debug_poison
+/* Test hooks (no counterpart in the reference).  debug_fault: from the next
+ * launch on, the CTA with block index `cta` (-1: none) of the persistent and the
+ * two-step kernels does not load plane xa of its first work item, and their
+ * pipeline waits and the grid barrier of the one-launch advance give up after
+ * `wait_limit` polls, so that CTA's wait runs out and rfxb_*_device_status
+ * reports RFXB_E_TIMEOUT (no box is left in flight: the CTA drains the others
+ * before leaving).  The other launches run the persistent kernels' item code
+ * with limits fixed at compile time (as launch arguments they cost the step
+ * 0.6 to 1 %).  debug_poison
  * replaces entry `index` of a work list (0/1 forward CPML/CPML-free, 2/3/4
  * reverse y-slab/other CPML/CPML-free) with an empty x range, which the
  * persistent kernels skip and report as RFXB_E_WORK.  Both leave the batch's

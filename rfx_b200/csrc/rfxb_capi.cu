@@ -58,7 +58,7 @@ size_t fwdv_smem_bytes(int tile, bool cp);
 __global__ void fwd_resident_kernel(const RfxbInst*, ResidentShape, int, int, int, int, unsigned*, int);
 size_t resident_smem_bytes(const ResidentShape&, int n_axes);
 size_t adj_step_smem_bytes();
-__global__ void fwd2_step_kernel(const RfxbInst*, const RfxbWork2*, const CUtensorMap*, int, int);
+__global__ void fwd2_step_kernel(const RfxbInst*, const RfxbWork2*, const CUtensorMap*, int, int, StepFault);
 size_t fwd2_step_smem_bytes();
 }  // namespace rfxb
 
@@ -247,7 +247,7 @@ struct RfxbBatch {
   int* d_qctr = nullptr;           // [8]: fetch counters of the forward (3) and reverse (4) queues
   int fwd_persist = 0;             // 0: off; k >= 1: on, k-1 CTAs per SM try the CPML-free list first
   int adj_persist = 0;             // 0: off; 1: on
-  int fault_cta = -1;              // test-only fault injection of the persistent kernels
+  int fault_cta = -1;              // test-only fault injection (persistent and two-step kernels)
   int wait_limit = rfxb::kWaitLimit;
   int adj_persist_grid = 0;        // CTAs of the persistent reverse launch (resident at once)
   int fwd_mode = 0;                // forward step kernel variant (see rfxb_fwd.cu)
@@ -860,7 +860,7 @@ int pick_fwd_tile(const RfxbBatch* g) {
 
 // The two-step kernel with its dynamic shared memory enabled.
 constexpr int kFwd2Threads = RFXB_D2ROWS * RFXB_D2COLS / 4;
-using Fwd2Kernel = void (*)(const RfxbInst*, const RfxbWork2*, const CUtensorMap*, int, int);
+using Fwd2Kernel = void (*)(const RfxbInst*, const RfxbWork2*, const CUtensorMap*, int, int, StepFault);
 Fwd2Kernel fwd2_kernel() {
   Fwd2Kernel k = fwd2_step_kernel;
   allow_smem(reinterpret_cast<const void*>(k), fwd2_step_smem_bytes());
@@ -1517,7 +1517,8 @@ int launch_pass(RfxbBatch* g, int n, int par, int pp, cudaStream_t st) {
   RFXB_CUDA(cudaEventRecord(g->ev_fork, st));
   RFXB_CUDA(cudaStreamWaitEvent(g->side_stream, g->ev_fork, 0));
   RFXB_CUDA(cudaStreamWaitEvent(g->side2, g->ev_fork, 0));
-  fwd2_kernel()<<<g->n_wd, kFwd2Threads, fwd2_step_smem_bytes(), g->side2>>>(g->d_inst, g->d_wd, g->d_maps, n, par);
+  fwd2_kernel()<<<g->n_wd, kFwd2Threads, fwd2_step_smem_bytes(), g->side2>>>(g->d_inst, g->d_wd, g->d_maps, n, par,
+                                                                               StepFault{g->fault_cta, g->wait_limit});
   if (g->n_wd1 > 0)
     launch_fwd(1, false, g, g->d_wd1, g->n_wd1, n, step_sel(par, 2, pp), g->side_stream);
   if (g->n_wd2 > 0) launch_fwd(1, true, g, g->d_wd2, g->n_wd2, n, step_sel(par, 2, pp), st);

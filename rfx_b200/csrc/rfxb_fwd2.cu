@@ -77,7 +77,7 @@ __device__ __forceinline__ void pec_faces(unsigned pec, int i, int j, int k, int
 // interior cell and those checks are compiled out.
 template <bool EDGE>
 __device__ __forceinline__ void fwd2_item(Fwd2Smem& S, const RfxbWork2& w, const CUtensorMap* __restrict__ maps,
-                                          int par) {
+                                          int par, const StepFault& fault) {
   constexpr int C = Fwd2Smem::C, R = Fwd2Smem::R, CE = Fwd2Smem::CE, CH = Fwd2Smem::CH, NT = R * C / 4, ZQ = C / 4;
   const int tid = threadIdx.x, r = tid / ZQ, zq = tid % ZQ;
   const RfxbInst& P = S.P;
@@ -86,7 +86,7 @@ __device__ __forceinline__ void fwd2_item(Fwd2Smem& S, const RfxbWork2& w, const
   const long long ps = P.ps, cs = P.cs;
   const unsigned pec = P.pec_axes;
   const CUtensorMap* tm = maps + (size_t)w.inst * RFXB_NMAPS;
-  const int wlim = kWaitLimit;
+  const int wlim = fault.wait_limit;
   // The boxes: E of planes xa-2 .. xb+1, H of xa-2 .. xb, coefficients of xa-1 .. xb
   // (map coordinates: z, j + 1, i + 1, component)
   const bool producer = tid == NT - 1;
@@ -113,7 +113,7 @@ __device__ __forceinline__ void fwd2_item(Fwd2Smem& S, const RfxbWork2& w, const
     issue_e(xa - 1);
     issue_h(xa - 2);
     issue_h(xa - 1);
-    issue_e(xa);
+    if ((int)blockIdx.x != fault.cta) issue_e(xa);
     issue_c(xa - 1);
     issue_c(xa);
   }
@@ -311,7 +311,7 @@ __device__ __forceinline__ void fwd2_item(Fwd2Smem& S, const RfxbWork2& w, const
 
 __global__ void __launch_bounds__(RFXB_D2ROWS * RFXB_D2COLS / 4, 2)
 fwd2_step_kernel(const RfxbInst* __restrict__ insts, const RfxbWork2* __restrict__ work,
-                 const CUtensorMap* __restrict__ maps, int n, int par) {
+                 const CUtensorMap* __restrict__ maps, int n, int par, StepFault fault) {
   extern __shared__ __align__(128) unsigned char fwd2_smem_raw[];
   Fwd2Smem& S = *reinterpret_cast<Fwd2Smem*>(fwd2_smem_raw);
   const int tid = threadIdx.x;
@@ -323,8 +323,8 @@ fwd2_step_kernel(const RfxbInst* __restrict__ insts, const RfxbWork2* __restrict
   }
   load_inst(S.P, insts + w.inst, tid, blockDim.x);
   __syncthreads();
-  if (w.mid & RFXB_MID_EDGE) fwd2_item<true>(S, w, maps, par);
-  else fwd2_item<false>(S, w, maps, par);
+  if (w.mid & RFXB_MID_EDGE) fwd2_item<true>(S, w, maps, par, fault);
+  else fwd2_item<false>(S, w, maps, par, fault);
 }
 
 }  // namespace rfxb
