@@ -943,7 +943,14 @@ int resident_ctas(int tile, bool cp) {
 
 // Block partition of the resident forward kernel for one plan: at most one
 // block per SM, the cheapest one (cells computed per step, shell cells read at
-// half weight) whose state fits the shared memory of an SM.
+// half weight) whose state fits the shared memory of an SM.  Below 140 cells per
+// SM a plan takes a half, a third .. of the SMs and leaves the rest to plans on
+// other streams: more blocks gain it little there, while many plans at once would
+// run one after another (us per step of one plan / of each of 32 on streams of
+// their own: 24x22x20 148 blocks 3.15 / 3.26, 74 blocks 3.34 / 1.71, launches per
+// step 23.7 / 2.58; 27^3 3.32 / 3.45, 3.61 / 1.88, 25.7 / 2.97).  Larger grids
+// need every SM (43x37x33: 148 blocks 4.08 / 4.22, 74 blocks 5.16 / 2.58, launches
+// per step 27 / 4.76).
 ResidentShape resident_shape(const RfxbPlan& p, int sms, size_t smem_max, size_t* smem) {
   ResidentShape best{};
   const int n[3] = {p.nx, p.ny, p.nz};
@@ -952,7 +959,10 @@ ResidentShape resident_shape(const RfxbPlan& p, int sms, size_t smem_max, size_t
   int dev = 0, coop = 0;
   cudaGetDevice(&dev);
   if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) != cudaSuccess || !coop) return best;
-  if ((long long)n[0] * n[1] * n[2] > (long long)sms * 4096) return best;
+  const long long cells = (long long)n[0] * n[1] * n[2];
+  if (cells > (long long)sms * 4096) return best;
+  const int share = (int)((sms * 140LL + cells - 1) / cells);   // plans that fit side by side
+  sms = std::max(1, sms / share);
   double best_cost = 1e300;
   for (int c0 = 1; c0 <= std::min(sms, n[0]); ++c0) {
     const int b0 = (n[0] + c0 - 1) / c0;

@@ -3,7 +3,7 @@ memory; it gives the results of one launch per step, bit for bit.
 
 Advances of one step each take the step kernels, so the two are compared on
 grids whose blocks end on, before and after the grid's faces, from a few cells
-to the largest that fits, thin axes (generic step kernels), CPML on some axes,
+to the largest that fits, axes so thin that tiles reach both slabs, CPML on some axes,
 odd and even step counts, chunks, graded spacing, a PEC sheet, and more sources
 and probes than one mask word holds.
 """
@@ -21,7 +21,8 @@ from tests.test_gpu_fullsize import _advance, _random_fields
 pytestmark = pytest.mark.gpu
 
 CASES = [((87, 47, 42), 8, "xyz", "", 1), ((33, 29, 31), 6, "yz", "x", 40), ((5, 4, 3), 0, "", "xyz", 1),
-         ((61, 1 + 52, 49), 8, "x", "yz", 3), ((97, 77, 75), 0, "", "xyz", 2), ((40, 21, 150), 5, "xyz", "", 2)]
+         ((61, 1 + 52, 49), 8, "x", "yz", 3), ((97, 77, 75), 0, "", "xyz", 2), ((40, 21, 150), 5, "xyz", "", 2), ((24, 22, 20), 4, "xyz", "", 2),
+         ((2, 2, 2), 0, "", "xyz", 1), ((19, 31, 11), 3, "xz", "y", 3)]
 
 
 def _compare(r, shape, n):
@@ -29,6 +30,7 @@ def _compare(r, shape, n):
     runs = []
     for chunks in (n, 1, 3):
         ts, _ = _advance(r, n, init=init, chunks=chunks)
+        assert r.plan.forward_route()[0] == (1 if chunks == n else 2)
         runs.append([ts] + [f.cpu().numpy().copy() for f in r.plan.store_fields()] +
                     [r.plan.save_state()])
     for other in runs[1:]:
