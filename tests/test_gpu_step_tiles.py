@@ -58,6 +58,7 @@ def test_forward_lists_agree_bit_for_bit(cuda, shape, ncp, axes, mu):
     try:
         lim = r.plan.launch_config()[1]
         single = run(fwd_split=0)
+        assert r.plan.forward_route() == (1, 24)
         assert np.abs(single[0]).max() > 0
         others = ([dict(fwd_split=1)] if lim["fwd_split"] else []) + \
                  ([dict(fwd_split=0, fwd_persist=2)] if lim["fwd_persist"] else [])
@@ -91,6 +92,7 @@ def test_reverse_lists_agree_bit_for_bit(cuda, shape, ncp, axes):
     try:
         lim = sw.batch.launch_config()[1]
         J0, g0 = run(adj_lite=0)
+        assert sw.batch.forward_route() == (1, 24)
         assert np.abs(g0).max() > 0
         others = ([dict(adj_lite=1)] if lim["adj_lite"] else []) + \
                  ([dict(adj_lite=0, adj_persist=1)] if lim["adj_persist"] else [])
