@@ -107,6 +107,7 @@ struct RfxbPlan {
   int nx = 0, ny = 0, nz = 0;
   double dt = 0.0;
   long long elems = 0;         // floats per padded per-cell array
+  bool x_inner_identity = true;   // the low x slab's innermost layer has no CPML terms (c = 0, kappa = 1)
   int par = 0;                 // parity of the field buffers holding the current state
   int ppar = 0;                // parity of the CPML psi buffers holding the current state (a
                                // two-step pass flips the fields once and the psi twice)
@@ -543,11 +544,12 @@ int depth2_column(const RfxbPlan& p, int y0, int z0) {
 
 // The x range of a plan's two-step segments: all planes without x CPML (the
 // items at the x faces take the guarded path), else the planes whose x-1 ..
-// x+1 neighbours are off the x slabs.
+// x+1 neighbours are off the x slabs, and one less at the low end where the
+// innermost layer, whose H the first plane's item recomputes, has CPML terms.
 void depth2_xrange(const RfxbPlan& p, int& dlo, int& dhi) {
   const int n = p.inst.ncp;
   const int ncpx = (n > 0 && (p.inst.cpml_axes & 1u)) ? n : 0;
-  dlo = ncpx > 0 ? ncpx + 1 : 0;
+  dlo = ncpx > 0 ? ncpx + (p.x_inner_identity ? 1 : 2) : 0;
   dhi = ncpx > 0 ? p.nx - ncpx - 1 : p.nx;
 }
 
@@ -2126,6 +2128,7 @@ int rfxb_plan_create(const RfxbDesc* d, RfxbPlan** out) {
     if (int rc = p->alloc(&dct, t4.size())) return bail(rc);
     if (cudaMemcpy(dct, t4.data(), t4.size() * sizeof(float4), cudaMemcpyHostToDevice) != cudaSuccess)
       return bail(fail(RFXB_E_LAUNCH, "cudaMemcpy"));
+    p->x_inner_identity = t4[6 * ncp + ncp - 1].y == 0.f && t4[6 * ncp + ncp - 1].z == 0.f;
     I.cpt = dct;
     I.cpu = dct + 6 * ncp;
     p->psi_elems[0] = 4LL * ncp * d->ny * I.zs;

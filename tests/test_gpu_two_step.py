@@ -3,7 +3,7 @@
 
 A two-step pass advances the CPML-free interior tiles from step n to n+2 on
 the two-step kernel (one read of E^n, H^{n-1/2}, ca/cb with a two-cell halo,
-the intermediate state in shared memory) while the CPML tiles and the tiles
+the intermediate state on chip) while the CPML tiles and the tiles
 near sources, probes, faces and the gradient region take two one-step
 launches through an intermediate field buffer.  Every cell is computed with
 the same rounding sequence either way, so the fields, probe traces, DFT
@@ -16,6 +16,8 @@ identical, not merely close:
 * the reference's own PEC benchmark (no CPML, PEC faces) at 129^3, and grids
   mixing CPML, PEC and open faces by axis (the guarded path of the tiles
   whose cells reach a face);
+* one and two CPML layers (a single layer absorbs; the innermost of several has no
+  CPML terms, and a pass recomputes the low one's H along x);
 * a graded-z grid with CPML and a PEC sheet (the spacing tables of the
   non-uniform lane, the PEC edge mask in both steps of a pass);
 * a DFT plane, a flux monitor and an NTFF box through two-step tiles (the
@@ -109,6 +111,25 @@ def test_two_step_mixed_faces_equal_one_step(cuda, cpml_axes, pec_axes):
         _check_two_step_available(r)
         init = _random_fields(g.shape, 10)
         _same(_run(r, n, init, 1), _run(r, n, init, 2), f"cpml {cpml_axes!r}, pec {pec_axes!r}")
+    finally:
+        r.plan.close()
+
+
+@pytest.mark.parametrize("ncp,cpml_axes,kappa_max", [(1, "x", 1.0), (1, "xyz", 4.0), (2, "x", 4.0)])
+def test_two_step_few_layers_equal_one_step(cuda, ncp, cpml_axes, kappa_max):
+    from rfx_b200.grid import Grid
+    from rfx_b200.simulation import MaterialArrays, prepare_device_run
+    shape, n = (70, 88, 128), 12
+    g = Grid(freq_max=20e9, domain=tuple((s - 2 * ncp - 1) * 1e-3 for s in shape), dx=1e-3, cpml_layers=ncp,
+             kappa_max=kappa_max)
+    assert g.shape == shape
+    ones = np.ones(shape, np.float32)
+    r = prepare_device_run(g, MaterialArrays(ones, 0 * ones, ones), n, cpml_axes=cpml_axes, pec_axes="", sources=[],
+                           probes=[(30, 4, 4, "ez")], dft_planes=[], pec_mask=None, dft_time_offset=1)
+    try:
+        _check_two_step_available(r)
+        init = _random_fields(shape, 6)
+        _same(_run(r, n, init, 1), _run(r, n, init, 2), f"{ncp} layers on {cpml_axes}")
     finally:
         r.plan.close()
 
