@@ -1,7 +1,8 @@
 // Generic fused reverse step of the adjoint (per-thread copies): the tiling, x
 // march, staged plane pipeline and halo recomputation of the generic forward
-// kernel (rfxb_fwd.cu), used with RFXB_STAGING=cpasync and by plans whose psi
-// offsets pass 32 bits; every other plan's reverse step is in rfxb_adjv.cu.
+// kernel (rfxb_fwd.cu), used with RFXB_STAGING=cpasync and by groups with a plan
+// whose psi offsets pass 32 bits or whose z slabs meet; every other plan's
+// reverse step is in rfxb_adjv.cu.
 //
 // The transpose of one forward step (see rfxb_adj.cu for the derivation)
 // has the forward's dependency shape with the roles swapped:

@@ -406,18 +406,17 @@ bool tile_reaches_yz(const RfxbPlan& p, int y0, int z0, int ty = kTY, int tz = 3
          ((ax & 4u) && (z0 - 1 < n || z0 + tz - 1 >= p.nz - n));
 }
 
-// Segments of every tile's full x line.
+// Segments of every 8 x 32 tile's full x line.
 void all_segments(const std::vector<RfxbPlan*>& plans, double slab, std::vector<WorkSeg>& segs) {
-  const int ty = kTY, tz = 32;
   for (size_t q = 0; q < plans.size(); ++q) {
     const RfxbPlan& p = *plans[q];
     const int n = p.inst.ncp;
     const unsigned ax = n > 0 ? p.inst.cpml_axes : 0u;
-    for (int y0 = 0; y0 < p.ny; y0 += ty)
-      for (int z0 = 0; z0 < p.nz; z0 += tz) {
+    for (int y0 = 0; y0 < p.ny; y0 += kTY)
+      for (int z0 = 0; z0 < p.nz; z0 += 32) {
         double c = 1.0;
-        if ((ax & 2u) && (y0 - 1 < n || y0 + ty - 1 >= p.ny - n)) c += slab;
-        if ((ax & 4u) && (z0 - 1 < n || z0 + tz - 1 >= p.nz - n)) c += slab;
+        if ((ax & 2u) && (y0 - 1 < n || y0 + kTY - 1 >= p.ny - n)) c += slab;
+        if ((ax & 4u) && (z0 - 1 < n || z0 + 31 >= p.nz - n)) c += slab;
         const int ncpx = (ax & 1u) ? n : 0;
         segs.push_back(WorkSeg{(int)q, y0, z0, 0, p.nx, p.nx, ncpx, c, (ax & 1u) ? slab : 0.0});
       }
@@ -711,7 +710,6 @@ void make_balanced_work(const std::vector<RfxbPlan*>& plans, int resident, doubl
   balance_segments(segs, resident, prologue, out);
 }
 
-// RFXB_WORK=uniform selects the plain split (one x chunk count for the group).
 // Modelled extra cost of a tile-plane per CPML slab it lies in, relative to
 // a plain tile-plane (RFXB_SLAB_WEIGHT, default 0.4).
 double slab_weight() {
@@ -767,12 +765,14 @@ bool adj_lite_enabled() {
   return v == 1;
 }
 
-// Work-list builder: 1 cost-balanced (default), 0 RFXB_WORK=uniform (one x
-// chunk count for the group), 2 RFXB_WORK=stream (x pieces of at most
-// RFXB_WORK_PLANES planes, default 24, listed piece-major and then in raster
-// order of instance, y, z, so that tiles which share halo rows are dispatched
-// together and stay within a few planes of each other: their halo reads then
-// come from L2).
+// Work-list builder of the generic and two-pass kernels: 1 cost-balanced
+// (default), 0 RFXB_WORK=uniform (one x chunk count for the group), 2
+// RFXB_WORK=stream (x pieces of at most RFXB_WORK_PLANES planes, default 24,
+// listed piece-major and then in raster order of instance, y, z, so that tiles
+// which share halo rows are dispatched together and stay within a few planes of
+// each other: their halo reads then come from L2).  The single-launch lists are
+// always cost-balanced; the split, persistent and two-step forms exist only
+// with 1.
 int work_mode() {
   static int v = -1;
   if (v < 0) {
@@ -842,7 +842,7 @@ void launch_fwd(int tile, bool cp, const RfxbBatch* g, const RfxbWork* list, int
 }
 
 // The generic per-thread-copy forward kernel (RFXB_STAGING=cpasync, and plans
-// whose psi offsets pass 32 bits).
+// whose psi offsets pass 32 bits or whose z slabs meet).
 void launch_fwd_generic(const RfxbBatch* g, int n, int sel, cudaStream_t st) {
   allow_smem(reinterpret_cast<const void*>(fwd_step_kernel), fwd_step_smem_bytes());
   fwd_step_kernel<<<g->n_work, dim3(32, kTY), fwd_step_smem_bytes(), st>>>(g->d_inst, g->d_work, n, sel);
@@ -1072,7 +1072,6 @@ int encode_block_map(CUtensorMap* m, const RfxbPlan& p, float* block, int ncomp,
 }
 
 int encode_forward_maps(RfxbPlan* p) {
-  const unsigned ty = kTY;
   for (int t = 0; t < 2; ++t) {
     const unsigned tz = kFwdTile[t].tz, tyt = kFwdTile[t].ty;
     CUtensorMap* m = &p->tmaps[RFXB_MAP_V0 + 7 * t];
@@ -1098,6 +1097,29 @@ bool vec_kernels_ok(const RfxbPlan& p) {
   for (int a = 0; a < 3; ++a)
     if (p.psi_elems[a] >= (1LL << 31)) return false;
   return !(p.inst.ncp > 0 && (p.inst.cpml_axes & 4u) && p.nz - 2 * p.inst.ncp < 3);
+}
+
+// Whether a plan's forward CPML terms take the profile's own coefficients and the
+// difference over the cell, instead of coefficients divided by the cell, which
+// rounds each of them once more, alike in every step.  Plans with more than 16
+// layers or with an 8 x 32 tile that reaches both slabs of an axis do: their
+// results are those of the kernel with one cell per thread, bit for bit without
+// kappa grading, which ran them before there were four cells per thread (divided
+// coefficients: 1.07 times its error against a float64 march on average, up to
+// 1.13).  The other plans' results have always been those of divided coefficients
+// (0.97 to 1.13 times that error, 1.015 on average); the time is the same.
+bool own_profile(const RfxbPlan& p) {
+  const RfxbInst& I = p.inst;
+  const int n = I.ncp;
+  if (n == 0 || I.cpml_axes == 0u) return false;
+  if (I.ncp4 > 16) return true;
+  if (I.cpml_axes & 2u)
+    for (int y0 = 0; y0 < p.ny; y0 += kTY)
+      if (y0 - 1 < n && y0 + kTY - 1 >= p.ny - n) return true;
+  if (I.cpml_axes & 4u)
+    for (int z0 = 0; z0 < p.nz; z0 += 32)
+      if (z0 - 1 < n && z0 + 31 >= p.nz - n) return true;
+  return false;
 }
 
 // Forward kernel variant of a group: 0 with RFXB_STAGING=cpasync or when a
@@ -2117,12 +2139,16 @@ int rfxb_plan_create(const RfxbDesc* d, RfxbPlan** out) {
       I.ib[f] = (float)(1.0 / d->cpml_cell[f]);
     }
     // per face and layer: the reverse kernels' table, then the forward kernels'
+    const bool own = own_profile(*p);
+    for (int q = 0; q < 2; ++q) I.zw[q] = own ? I.ib[4 + q] : 1.f;
     std::vector<float4> t4(12 * ncp);
     for (int f = 0; f < 6; ++f)
       for (int s = 0; s < ncp; ++s) {
         const float b = tb[(f * 3 + 0) * ncp + s], c = tb[(f * 3 + 1) * ncp + s], km = tb[(f * 3 + 2) * ncp + s];
         t4[f * ncp + s] = make_float4(b, (float)((double)c * I.ib[f]), (float)((double)km * I.ib[f]), 0.f);
-        t4[(6 + f) * ncp + s] = make_float4(b, c, km, I.ib[f]);
+        t4[(6 + f) * ncp + s] = t4[f * ncp + s];
+        t4[(6 + f) * ncp + s].w = 1.f;
+        if (own) t4[(6 + f) * ncp + s] = make_float4(b, c, km, I.ib[f]);
       }
     float4* dct = nullptr;
     if (int rc = p->alloc(&dct, t4.size())) return bail(rc);

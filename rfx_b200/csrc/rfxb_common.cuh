@@ -59,12 +59,10 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint32_t addr, uint32_t parity
   return false;
 }
 // Mbarrier phases carried from one work item to the next by a CTA that
-// processes several (the persistent kernels): bit s of `stage` is the parity
-// of the next completion of plane stage s, bit s of `ring` that of psi ring
-// slot s.  A CTA that runs one item starts from zero.
+// processes several (the persistent kernels): bit b of `stage` is the parity
+// of the next completion of barrier b.  A CTA that runs one item starts from zero.
 struct StepPhases {
   uint32_t stage = 0u;
-  uint32_t ring = 0u;
 };
 
 // Fault injection of the bounded-wait test (the defaults in every other
@@ -92,10 +90,8 @@ __device__ __forceinline__ float yee_e(float ca, float e, float cb, float curl) 
 }
 
 // CPML of the forward step, from a field difference over a cell, g = difference *
-// (1 / cell):  psi' = b psi + c g,  f + s (psi' + km g).  c and km are the tables'
-// own values: with 1 / cell folded into them each coefficient is rounded once
-// more, alike in every step (error against float64 up to 1.13 times this one's
-// over grids of 43x37x33 to 72x70x75), and the operations are as many.
+// w with the profile's (b, c, km, w) of RfxbInst::cpu:  psi' = b psi + c g,
+// f + s (psi' + km g).
 __device__ __forceinline__ float psi_next(float b, float psi, float c, float g) {
   return __fmaf_rn(c, g, __fmul_rn(b, psi));
 }

@@ -1,7 +1,8 @@
 // Generic forward time step of the Yee/CPML leapfrog (per-thread copies): one
 // fused kernel per step, used with RFXB_STAGING=cpasync, by the entry point
-// that allocates nothing, and by plans whose psi offsets pass 32 bits.  The
-// step kernel of every other plan is in rfxb_fwdv.cu; this file also holds the
+// that allocates nothing, and by groups with a plan whose psi offsets pass 32
+// bits or whose z slabs meet (fewer than three cells between them).  The step
+// kernel of every other plan is in rfxb_fwdv.cu; this file also holds the
 // running DFT, the layout conversions and the coefficient kernel.
 //
 // One CTA owns a (TY x 32) tile of the (y, z) plane and marches along x over

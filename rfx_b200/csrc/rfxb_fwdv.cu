@@ -29,8 +29,8 @@
 // 360 (CPML-free) and 525 instructions per cell against 130 and 250 here and read
 // psi 4 bytes at a time.  24 x 32 tiles take two CTAs per SM (seven warps, 128
 // registers, up to 110 KB); taller ones leave one, lower ones reread more halo.
-// Measured, one cell per thread -> here: 217x217x121 with CPML 12 182 -> 129 us a
-// step, 131x147x103 with CPML 8 96 -> 61, 277^3 with CPML 10 about 325 -> 316 (of
+// Measured, one cell per thread -> here: 217x217x121 with CPML 12 182 -> 122 us a
+// step, 131x147x103 with CPML 8 96 -> 62, 277^3 with CPML 10 about 325 -> 312 (of
 // which CPML-free items 160).  H and the coefficients loaded into registers one
 // plane ahead instead of staged: 263 us instead of 183 on 257^3.
 #include "rfxb_common.cuh"
@@ -64,7 +64,7 @@ struct __align__(128) VSmem {
   float h[2][2][TY][D::TZ];               // hx, hz of plane i in slot i & 1: rows y0-1 .. y0+TY-2
   float hc[2][2][TY];                     // hx, hy of column z0-1
   float zt[2][D::TZ];                     // zh, ze of the tile's columns
-  float zp[3][D::TZ];                     // z profile of the columns (b, c, 1/kappa-1)
+  float zp[3][D::TZ];                     // z profile of the columns (b, c, km)
   float ps[CP ? RFXB_PSLOTS : 1][CP ? D::MAIN : 1][4];
   RfxbInst P;
   unsigned long long mbar[RFXB_VBARS];    // E stages, H stages, coefficient stages
@@ -74,7 +74,7 @@ struct __align__(128) VSmem {
 struct VSlab {
   bool y = false;              // in a y slab
   unsigned z = 0u;             // cells in a z slab (zslab_of)
-  float4 cy;                   // y profile (b, c, 1/kappa-1, 1/cell)
+  float4 cy;                   // y profile (b, c, km, w)
   int oy = 0;                  // y psi element of (q 0, plane 0): + i * ncp * zs
   int oz = 0;                  // z psi element of the first cell's (q 0, plane 0): + i * ny * ncp4
 };
@@ -100,14 +100,14 @@ __device__ __forceinline__ void psi_xy(Vec<L>& f, const Vec<L>& s, Vec<L> p, flo
   }
   if (WRITE) vst<L>(out, p);
 }
-// The same for a z slab: profile per column, psi at the columns' layers, ib = 1/cell.
+// The same for a z slab: profile per column, psi at the columns' layers.
 template <int L, int SGN, bool WRITE, bool K>
 __device__ __forceinline__ void psi_z(Vec<L>& f, const Vec<L>& s, Vec<L> p, float* out, unsigned m, const float* zp,
-                                      int zstride, float ib, const Vec<L>& d, Vec<L>& k, bool rec = false) {
+                                      int zstride, float w, const Vec<L>& d, Vec<L>& k, bool rec = false) {
   const Vec<L> b = vld<L>(zp), c = vld<L>(zp + zstride), km = vld<L>(zp + 2 * zstride);
 #pragma unroll
   for (int l = 0; l < L; ++l) {
-    const float g = __fmul_rn(d[l], ib);
+    const float g = __fmul_rn(d[l], w);
     p[l] = psi_next(b[l], p[l], c[l], g);
     if ((m >> l) & 1u) f[l] = psi_add(f[l], SGN > 0 ? s[l] : -s[l], p[l], km[l], g);
   }
@@ -115,7 +115,7 @@ __device__ __forceinline__ void psi_z(Vec<L>& f, const Vec<L>& s, Vec<L> p, floa
 #pragma unroll
     for (int l = 0; l < L; ++l) {
       if (!((m >> l) & 1u)) continue;
-      const float t = __fmaf_rn(km[l], __fmul_rn(d[l], ib), p[l]);
+      const float t = __fmaf_rn(km[l], __fmul_rn(d[l], w), p[l]);
       k[l] = SGN > 0 ? __fadd_rn(k[l], t) : __fsub_rn(k[l], t);
     }
   }
@@ -131,7 +131,7 @@ template <int L, int MASK, bool CP, bool WRITE, int EW, int CE, class Hold, clas
 __device__ __forceinline__ void h_vec(const float* A, const float* B, int o, const Vec<L>* e0, float exz, float eyz,
                                       Hold&& hold, Old&& old, float xh, float yh, const Vec<L>& zh, const Vec<L>& ch,
                                       const RfxbInst& P, int par, bool xon, const float4& cx, int ox, const VSlab& S,
-                                      const float* zp, float ibz, int i, int qx, int qy, int qz, int ncp, Vec<L>& hx, Vec<L>& hy,
+                                      const float* zp, float wz, int i, int qx, int qy, int qz, int ncp, Vec<L>& hx, Vec<L>& hy,
                                       Vec<L>& hz) {
   constexpr int ZS = EW - 8;
   const int iy = S.oy + i * ncp * P.zs, iz = S.oz + i * P.ny * P.ncp4;
@@ -147,7 +147,7 @@ __device__ __forceinline__ void h_vec(const float* A, const float* B, int o, con
     }
     if (CP && S.y) psi_xy<L, -1, WRITE, false>(hx, ch, old(1, 0), P.psH[par ^ 1][1] + iy, S.cy, gy, none);
     if (CP && S.z)
-      psi_z<L, +1, WRITE, false>(hx, ch, old(2, 0), P.psH[par ^ 1][2] + iz, S.z, zp, ZS, ibz, gz, none);
+      psi_z<L, +1, WRITE, false>(hx, ch, old(2, 0), P.psH[par ^ 1][2] + iz, S.z, zp, ZS, wz, gz, none);
   }
   if (MASK & 2) {   // Hy += ch psi(dEz/dx) [x q0], Hy -= ch psi(dEx/dz) [z q1]
     Vec<L> gx = vld<L>(B + o + 2 * CE), gz;
@@ -160,7 +160,7 @@ __device__ __forceinline__ void h_vec(const float* A, const float* B, int o, con
     }
     if (CP && xon) psi_xy<L, +1, WRITE, false>(hy, ch, old(0, 0), P.psH[par ^ 1][0] + ox, cx, gx, none);
     if (CP && S.z)
-      psi_z<L, -1, WRITE, false>(hy, ch, old(2, 1), P.psH[par ^ 1][2] + iz + qz, S.z, zp, ZS, ibz, gz, none);
+      psi_z<L, -1, WRITE, false>(hy, ch, old(2, 1), P.psH[par ^ 1][2] + iz + qz, S.z, zp, ZS, wz, gz, none);
   }
   if (MASK & 4) {   // Hz -= ch psi(dEy/dx) [x q1], Hz += ch psi(dEx/dy) [y q1]
     Vec<L> gx = vld<L>(B + o + CE), gy = vld<L>(A + o + EW);
@@ -352,7 +352,7 @@ __device__ __forceinline__ bool fwdv_item(VSmem<TY, ZQ, CP>& S, const RfxbInst* 
     const int jk = j * zs + k;
     const float yh = own ? __ldg(P.yh + j) : 0.f, ye = own ? __ldg(P.ye + j) : 0.f;
     const float* zp = &S.zp[0][4 * zq];
-    const float ibz = CP ? P.ib[4 + (k >= ncp)] : 0.f;
+    const float wz = CP ? P.zw[k >= ncp] : 0.f;
     const bool last_q = zq == ZQ - 1, first_q = zq == 0;
     // sources and probes in this thread's columns
     unsigned smask = 0u, pmask = 0u;
@@ -409,7 +409,7 @@ __device__ __forceinline__ bool fwdv_item(VSmem<TY, ZQ, CP>& S, const RfxbInst* 
               if (a == 1) return vld<4>(p + B.oy + (xa - 1) * ncp * zs + q * qy);
               return zpsi_load<4>(p + B.oz + (xa - 1) * ny * n4 + q * qz, B.z);
             },
-            __ldg(xh_tab + xa - 1), yh, vld<4>(&S.zt[0][4 * zq]), ch, P, par, xon, cx, xbase + jk, B, zp, ibz, xa - 1, qx, qy, qz,
+            __ldg(xh_tab + xa - 1), yh, vld<4>(&S.zt[0][4 * zq]), ch, P, par, xon, cx, xbase + jk, B, zp, wz, xa - 1, qx, qy, qz,
             ncp, t, hyp, hzp);
       }
 #pragma unroll
@@ -459,7 +459,7 @@ __device__ __forceinline__ bool fwdv_item(VSmem<TY, ZQ, CP>& S, const RfxbInst* 
                 if (a == 0 && B.y) return vld<4>(P.psH[par][0] + xbase + jk + q * qx);
                 return vld<4>(slot + (a == 2 ? 4 + q : q) * SS);
               },
-              xh, yh, vld<4>(&S.zt[0][4 * zq]), ch, P, par, xon, cx, xbase + jk, B, zp, ibz, i, qx, qy, qz, ncp, hx, hy, hz);
+              xh, yh, vld<4>(&S.zt[0][4 * zq]), ch, P, par, xon, cx, xbase + jk, B, zp, wz, i, qx, qy, qz, ncp, hx, hy, hz);
           if (kv < 4) {
 #pragma unroll
             for (int l = 1; l < 4; ++l)
@@ -512,7 +512,7 @@ __device__ __forceinline__ bool fwdv_item(VSmem<TY, ZQ, CP>& S, const RfxbInst* 
           }
           if (CP && B.y) psi_xy<4, +1, true, true>(ex, ce, vld<4>(slot + 2 * SS), P.psE[par ^ 1][1] + iy, B.cy, gy, kk, hist_i);
           if (CP && B.z)
-            psi_z<4, -1, true, true>(ex, ce, vld<4>(slot + 6 * SS), P.psE[par ^ 1][2] + iz, B.z, zp, 4 * ZQ, ibz, gz, kk, hist_i);
+            psi_z<4, -1, true, true>(ex, ce, vld<4>(slot + 6 * SS), P.psE[par ^ 1][2] + iz, B.z, zp, 4 * ZQ, wz, gz, kk, hist_i);
           if (hist_i) keep(0, cu);
         }
         {   // Ey -= ce psi(dHz/dx) [x q0], Ey += ce psi(dHx/dz) [z q1]
@@ -526,7 +526,7 @@ __device__ __forceinline__ bool fwdv_item(VSmem<TY, ZQ, CP>& S, const RfxbInst* 
           }
           if (CP && xon) psi_xy<4, -1, true, true>(ey, ce, vld<4>(B.y ? P.psE[par][0] + ix : slot + 2 * SS), P.psE[par ^ 1][0] + ix, cx, gx, kk, hist_i);
           if (CP && B.z)
-            psi_z<4, +1, true, true>(ey, ce, vld<4>(slot + 7 * SS), P.psE[par ^ 1][2] + iz + qz, B.z, zp, 4 * ZQ, ibz, gz, kk, hist_i);
+            psi_z<4, +1, true, true>(ey, ce, vld<4>(slot + 7 * SS), P.psE[par ^ 1][2] + iz + qz, B.z, zp, 4 * ZQ, wz, gz, kk, hist_i);
           if (hist_i) keep(1, cu);
         }
         {   // Ez += ce psi(dHy/dx) [x q1], Ez -= ce psi(dHx/dy) [y q1]
@@ -732,7 +732,7 @@ __device__ __forceinline__ bool fwdv_item(VSmem<TY, ZQ, CP>& S, const RfxbInst* 
           h_vec<4, 5, CP, false, EW, CE>(
               A, Bp, o, e0, A[o + 4], A[o + 4 + CE], [&](int c) { return vld<4>(H + c * D::CH + 4 * lane); },
               [&](int a, int q) { return a == 0 ? pr[0] : a == 2 ? pr[3] : q == 0 ? pr[1] : pr[2]; }, xh, yh,
-              vld<4>(&S.zt[0][4 * lane]), ch, P, par, xon, cx, xbase + jk, B, &S.zp[0][4 * lane], P.ib[4 + (k >= ncp)], i, qx, qy, qz, ncp, hx, hy,
+              vld<4>(&S.zt[0][4 * lane]), ch, P, par, xon, cx, xbase + jk, B, &S.zp[0][4 * lane], P.zw[k >= ncp], i, qx, qy, qz, ncp, hx, hy,
               hz);
         }
         vst<4>(&S.h[sl][0][0][4 * lane], hx);

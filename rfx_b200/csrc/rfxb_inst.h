@@ -60,7 +60,10 @@ struct RfxbInst {
   unsigned cpml_axes;      // bit a set -> axis a absorbs
   const float* cpb;        // [face][3][ncp]: b, c, (1/kappa - 1); face = 2*axis + side
   const float4* cpt;       // [face][ncp]: (b, c / cell, (1/kappa - 1) / cell, 0), reverse step
-  const float4* cpu;       // [face][ncp]: (b, c, 1/kappa - 1, 1 / cell), forward step
+  const float4* cpu;       // [face][ncp]: (b, c, km, w), forward step: g = difference * w with
+                           // w = 1 / cell and the tables' own c and km = 1/kappa - 1, or
+                           // w = 1 and both divided by the cell (own_profile in rfxb_capi.cu)
+  float zw[2];             // w of the low and the high z face
   float ib[6];             // 1 / boundary cell size per face
   float* psH[2][3];        // H-side psi per axis, ping-pong
   float* psE[2][3];        // E-side psi per axis, ping-pong

@@ -310,13 +310,14 @@ class Plan:
         return out
 
     def forward_variant(self) -> int:
-        """0 generic step kernel, 1 TMA staging without CPML, 2 TMA staging
-        with TMA-staged CPML psi."""
+        """0 generic step kernel, 1 TMA staging and four cells per thread without
+        CPML, 2 the same with the CPML psi prefetched one plane ahead."""
         return int(self._lib.rfxb_plan_forward_variant(self._h))
 
     def adjoint_variant(self) -> int:
-        """0 cp.async staging, 1 TMA staging, 2 TMA staging with TMA-staged
-        adjoint psi; -1 before the first adjoint advance."""
+        """0 cp.async staging, 2 TMA staging and four cells per thread with the
+        adjoint psi prefetched one plane ahead, 3 the same without CPML; -1
+        before the first adjoint advance."""
         return int(self._lib.rfxb_plan_adjoint_variant(self._h))
 
     def step_launches(self):

@@ -1,12 +1,12 @@
 """Rounding of the forward step's CPML terms.
 
-The kernels with four cells per thread and the one-launch advance of small grids
-take a psi term from g = difference * (1 / cell) and the profile's own b, c and
-1/kappa - 1, as the kernel with one cell per thread (RFXB_STAGING=cpasync) does;
-without kappa grading the results are its results bit for bit, on grids whose
-tiles reach both slabs of an axis and on others.  (With 1 / cell folded into c,
-every c was rounded once more and the fields were up to 1.13 times as far from a
-float64 march.)
+Grids with an 8 x 32 tile that reaches both slabs of an axis, or with more than 16
+layers, take a psi term from g = difference * (1 / cell) and the profile's own b, c
+and 1/kappa - 1, as the kernel with one cell per thread (RFXB_STAGING=cpasync)
+does; without kappa grading the results are its results bit for bit, from the
+kernels with four cells per thread and the one-launch advance alike.  (With 1 / cell
+divided into c, every c is rounded once more and the fields were up to 1.13 times
+as far from a float64 march.)  Other grids take the divided coefficients.
 
 kappa_max > 1 adds the curl's own term: forward and reverse step against the
 float64 oracle.  Per step a cell takes some twenty roundings of 2^-24, which add
@@ -29,8 +29,10 @@ from tests.test_gpu_fullsize import COMPONENTS, _advance, _random_fields
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 # cells, CPML layers, CPML axes, per-cell mu_r
-SCENES = [((43, 37, 33), 6, "xyz", False), ((36, 52, 40), 8, "xyz", False), ((64, 52, 49), 8, "xyz", False),
-          ((60, 33, 36), 6, "yz", True), ((47, 21, 70), 7, "y", False), ((50, 30, 21), 5, "z", True)]
+SCENES = [((43, 37, 33), 6, "xyz", False), ((36, 52, 39), 8, "xyz", False), ((60, 33, 36), 6, "yz", True),
+          ((47, 22, 70), 8, "y", False), ((50, 30, 21), 5, "z", True), ((60, 45, 77), 18, "xyz", False),
+          ((80, 200, 38), 7, "xz", False)]
+OTHER = ((64, 52, 49), 8, "xyz", False)   # divided coefficients
 STEPS = 24
 
 
@@ -63,7 +65,7 @@ def _march(r, init, n, chunks):
 
 def _main(path):
     out = {}
-    for q, scene in enumerate(SCENES):
+    for q, scene in enumerate(SCENES + [OTHER]):
         r, init, _, _ = _run(scene)
         for c, f in zip(COMPONENTS, _march(r, init, STEPS, 1)):
             out[f"{c}{q}"] = f
@@ -80,21 +82,24 @@ def test_forward_step_rounds_as_one_cell_per_thread(cuda, tmp_path):
     p = subprocess.run([sys.executable, "-c", code], cwd=ROOT, env=env, capture_output=True, text=True, timeout=300)
     assert p.returncode == 0, p.stderr[-2000:]
     one = np.load(path)
-    for q, scene in enumerate(SCENES):
+    for q, scene in enumerate(SCENES + [OTHER]):
         r, init, _, _ = _run(scene)
         try:
             assert r.plan.forward_variant() == 2
             for chunks, route in ((1, 1 if scene[3] else 2), (STEPS, 1)):
                 got = _march(r, init, STEPS, chunks)
-                assert r.plan.forward_route()[0] == route
+                assert np.prod(scene[0]) > 606208 or r.plan.forward_route()[0] == route
                 for c, f in zip(COMPONENTS, got):
-                    assert np.array_equal(f, one[f"{c}{q}"]), (scene, chunks, c)
+                    if scene is OTHER:
+                        assert np.linalg.norm(f - one[f"{c}{q}"]) < 2e-6 * np.linalg.norm(f)
+                    else:
+                        assert np.array_equal(f, one[f"{c}{q}"]), (scene, chunks, c)
         finally:
             r.plan.close()
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("scene", SCENES[:2] + SCENES[3:4])
+@pytest.mark.parametrize("scene", SCENES[:3] + [OTHER])
 def test_forward_with_kappa_grading_matches_float64(cuda, scene):
     n, kappa = 60, 5.0
     r, init, mats, src = _run(scene, n, kappa)
