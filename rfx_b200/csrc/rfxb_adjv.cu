@@ -15,14 +15,6 @@
 // its psi) and travels inside the flux: to the next lane in z, to the next
 // plane in registers, and in y through shared memory (K) or, for the one row
 // above, by evaluating that row's G again, so a plane needs one barrier.
-// A flux that travels, s q + r, is rounded once, and the difference to it has its
-// own product fused, fma(s, q, -other), with r added by itself: without CPML these
-// are the operations of the kernel with one cell per thread (rfxb_adj_fused.cu),
-// in the slabs as many roundings.  The differences of phase B that need no other
-// row are formed before the barrier, so that nothing but p crosses it.  With every
-// product rounded by itself the adjoint fields were 1.04 to 1.17 times as far from
-// a float64 march, at 97x83x109 46.5 against 49.4 us a step now, 221x141x69 96.6 /
-// 97.5, a 131^3 closed box 41.5 / 42.1, the sweep below 1417 / 1411.
 // The probe cotangent of y_{n-1}, the source adjoint and the PEC / edge mask
 // follow; adjoint fields and psi are ping-ponged like the forward state.  The
 // eps_r gradient over the recorded region is accumulated in phase A from the
@@ -31,12 +23,10 @@
 // What bounds it: instructions and, in the slabs, instruction fetch (the CPML
 // path is 98 KB of code; the rare work -- probes, sources, gradient, failure --
 // therefore sits behind single sites over indexed copies: the step of 20 grids
-// of 64-160 cells a side 1477 -> 1380 us), and registers: E and cb of the own
-// cells are read from their stage where they are used (221x141x69 103 -> 98 us a
-// step with them held in registers and 212 instead of 96 bytes spilled).  One cell per
-// thread with the relations of the neighbours evaluated again in place -> here,
-// reverse steps alone: that sweep 1629 -> 1411 us (three launches against one),
-// 221x141x69 with CPML 10 131 -> 97.5, 97x83x109 with CPML 8 58.5 -> 49.4.
+// of 64-160 cells a side 1477 -> 1380 us).  One cell per thread with the
+// relations of the neighbours evaluated again in place -> here: that step
+// 1810 -> 1375 us (three launches against one), 221x141x69 with CPML 10
+// 157 -> 100, 97x83x109 with CPML 8 103 -> 43.
 #include "rfxb_common.cuh"
 #include "rfxb_vec.cuh"
 
@@ -90,70 +80,51 @@ template <int SGN>
 __device__ __forceinline__ float rel_r(float nu, float s, float t, float c, float km) {
   return __fmaf_rn(SGN > 0 ? s : -s, __fmul_rn(km, t), __fmul_rn(c, nu));
 }
-// r of a relation of an x or y slab, from its old psi p
-template <int L, int SGN, bool WRITE>
-__device__ __forceinline__ Vec<L> rel_xy(Vec<L> p, float* out, const float4& c, const Vec<L>& s, const Vec<L>& t,
-                                         bool write = true) {
-  Vec<L> r;
+// f += ADD * r of a relation of an x or y slab, from its old psi p
+template <int L, int SGN, int ADD, bool WRITE>
+__device__ __forceinline__ void rel_xy(Vec<L>& f, Vec<L> p, float* out, const float4& c, const Vec<L>& s,
+                                       const Vec<L>& t, bool write = true) {
 #pragma unroll
   for (int l = 0; l < L; ++l) {
     const float nu = rel_nu<SGN>(p[l], s[l], t[l]);
-    r[l] = rel_r<SGN>(nu, s[l], t[l], c.y, c.z);
+    const float r = rel_r<SGN>(nu, s[l], t[l], c.y, c.z);
+    f[l] = ADD > 0 ? __fadd_rn(f[l], r) : __fsub_rn(f[l], r);
     p[l] = __fmul_rn(c.x, nu);
   }
   if (WRITE && write) vst<L>(out, p);
-  return r;
 }
-// the same for a z slab (zero off it): profile per column, psi at the columns' layers
-template <int L, int SGN, bool WRITE>
-__device__ __forceinline__ Vec<L> rel_z(Vec<L> p, float* out, unsigned m, const Vec<L>& b, const Vec<L>& c,
-                                        const Vec<L>& km, const Vec<L>& s, const Vec<L>& t) {
-  Vec<L> r;
+// the same for a z slab: profile per column, psi at the columns' layers
+template <int L, int SGN, int ADD, bool WRITE>
+__device__ __forceinline__ void rel_z(Vec<L>& f, Vec<L> p, float* out, unsigned m, const Vec<L>& b,
+                                      const Vec<L>& c, const Vec<L>& km, const Vec<L>& s, const Vec<L>& t) {
 #pragma unroll
   for (int l = 0; l < L; ++l) {
     const float nu = rel_nu<SGN>(p[l], s[l], t[l]);
-    r[l] = (m >> l) & 1u ? rel_r<SGN>(nu, s[l], t[l], c[l], km[l]) : 0.f;
+    const float r = rel_r<SGN>(nu, s[l], t[l], c[l], km[l]);
+    if ((m >> l) & 1u) f[l] = ADD > 0 ? __fadd_rn(f[l], r) : __fsub_rn(f[l], r);
     p[l] = __fmul_rn(b[l], nu);
   }
   if (WRITE) zpsi_store<L>(out, m, p);
-  return r;
 }
 
 template <int L>
-__device__ __forceinline__ Vec<L> vsplat(float a) {
+__device__ __forceinline__ Vec<L> vscale(float a, const Vec<L>& b, const Vec<L>& c) {   // a (b c)
   Vec<L> r;
 #pragma unroll
-  for (int l = 0; l < L; ++l) r[l] = a;
+  for (int l = 0; l < L; ++l) r[l] = __fmul_rn(a, __fmul_rn(b[l], c[l]));
   return r;
 }
 template <int L>
-__device__ __forceinline__ Vec<L> vmul(const Vec<L>& a, const Vec<L>& b) {
+__device__ __forceinline__ Vec<L> vscale(const Vec<L>& a, const Vec<L>& b, const Vec<L>& c) {
   Vec<L> r;
 #pragma unroll
-  for (int l = 0; l < L; ++l) r[l] = __fmul_rn(a[l], b[l]);
+  for (int l = 0; l < L; ++l) r[l] = __fmul_rn(a[l], __fmul_rn(b[l], c[l]));
   return r;
 }
-// s q + SGN r, rounded once
-template <int SGN, int L>
-__device__ __forceinline__ Vec<L> vfma(const Vec<L>& s, const Vec<L>& q, const Vec<L>& r) {
-  Vec<L> f;
-#pragma unroll
-  for (int l = 0; l < L; ++l) f[l] = __fmaf_rn(s[l], q[l], SGN > 0 ? r[l] : -r[l]);
-  return f;
+// a + ((b - bn) - (c - cn))
+__device__ __forceinline__ float curl_t(float a, float b, float bn, float c, float cn) {
+  return __fadd_rn(a, __fsub_rn(__fsub_rn(b, bn), __fsub_rn(c, cn)));
 }
-// a flux: with R, r is zero off the slabs; without, no cell has one
-template <bool R, int SGN, int L>
-__device__ __forceinline__ Vec<L> vflux(const Vec<L>& s, const Vec<L>& q, const Vec<L>& r) {
-  return R ? vfma<SGN>(s, q, r) : vmul(s, q);
-}
-// f += SGN r
-template <int SGN, int L>
-__device__ __forceinline__ void vacc(Vec<L>& f, const Vec<L>& r) {
-#pragma unroll
-  for (int l = 0; l < L; ++l) f[l] = SGN > 0 ? __fadd_rn(f[l], r[l]) : __fsub_rn(f[l], r[l]);
-}
-// a + (b - c), b and c two differences of fluxes
-__device__ __forceinline__ float curl_t(float a, float b, float c) { return __fadd_rn(a, __fsub_rn(b, c)); }
 
 // One work item (see fwdv_item): returns false when a bounded wait ran out.
 template <int TY, int ZQ, bool CP>
@@ -292,90 +263,52 @@ __device__ __forceinline__ bool adjv_item(AVSmem<TY, ZQ, CP>& S, const RfxbInst*
     bad_end = bar_or<NT>(!(ok0 && ok1 && ok2));
   }
 
-  // Fluxes of L columns with fields ex ey ez and coefficient cb; in a slab, ld(q)
-  // gives the old psi and ld(2) the cells' ce.  A flux s q + r is rounded once; in a
-  // difference of two the own product is not rounded before it, fma(s, q, -other),
-  // and r goes to H by itself.
+  // fluxes of L columns with fields ex ey ez and coefficient cb; in a slab, ld(q)
+  // gives the old psi and ld(2) the cells' ce.
   // G of the y direction: Gyx = ye q_x + r_y0, Gyz = ye q_z - r_y1.
-  auto gy_flux = [&](auto LL, const Vec<decltype(LL)::v>& ex, const Vec<decltype(LL)::v>& ez,
-                     const Vec<decltype(LL)::v>& cb, float ye, bool on, const float4& c, auto&& ld,
+  auto gy_flux = [&](auto LL, auto WR, const Vec<decltype(LL)::v>& ex, const Vec<decltype(LL)::v>& ez,
+                     const Vec<decltype(LL)::v>& cb, float ye, bool on, const float4& c, int iy, auto&& ld,
                      Vec<decltype(LL)::v>& gyx, Vec<decltype(LL)::v>& gyz) {
     constexpr int L = decltype(LL)::v;
-    const Vec<L> s = vsplat<L>(ye);
-    Vec<L> r0 = vzero<L>(), r1 = vzero<L>();
-    if (CP && on) {
-      const Vec<L> ce = ld(2);
-      r0 = rel_xy<L, +1, false>(ld(0), nullptr, c, ce, ex);
-      r1 = rel_xy<L, -1, false>(ld(1), nullptr, c, ce, ez);
-    }
-    gyx = vflux<CP, +1>(s, vmul(cb, ex), r0);
-    gyz = vflux<CP, -1>(s, vmul(cb, ez), r1);
-  };
-  // Gyx - nyx and Gyz - nyz, nyx and nyz the fluxes of the row above: the products
-  // in dyx and dyz, the relations added to hz and hx
-  auto gy_diff = [&](auto LL, auto WR, const Vec<decltype(LL)::v>& ex, const Vec<decltype(LL)::v>& ez,
-                     const Vec<decltype(LL)::v>& cb, float ye, bool on, const float4& c, int iy, auto&& ld,
-                     const Vec<decltype(LL)::v>& nyx, const Vec<decltype(LL)::v>& nyz, Vec<decltype(LL)::v>& dyx,
-                     Vec<decltype(LL)::v>& dyz, Vec<decltype(LL)::v>& hx, Vec<decltype(LL)::v>& hz) {
-    constexpr int L = decltype(LL)::v;
     constexpr bool W = decltype(WR)::v != 0;
-    const Vec<L> s = vsplat<L>(ye);
-    dyx = vfma<-1>(s, vmul(cb, ex), nyx);
-    dyz = vfma<-1>(s, vmul(cb, ez), nyz);
+    gyx = vscale<L>(ye, cb, ex);
+    gyz = vscale<L>(ye, cb, ez);
     if (CP && on) {
       const Vec<L> ce = ld(2);
       float* out = AD.aPsiE[par ^ 1][1];
-      vacc<+1>(hz, rel_xy<L, +1, W>(ld(0), out + iy, c, ce, ex));
-      vacc<+1>(hx, rel_xy<L, -1, W>(ld(1), out + iy + qy, c, ce, ez));
+      rel_xy<L, +1, +1, W>(gyx, ld(0), out + iy, c, ce, ex);
+      rel_xy<L, -1, -1, W>(gyz, ld(1), out + iy + qy, c, ce, ez);
     }
   };
-  // G of the z direction, Gzx = ze q_x - r_z0, Gzy = ze q_y + r_z1; with H the relations are added to hx and hy
-  auto gz_flux = [&](auto LL, auto WR, auto HH, const Vec<decltype(LL)::v>& ex, const Vec<decltype(LL)::v>& ey,
+  // G of the z direction: Gzx = ze q_x - r_z0, Gzy = ze q_y + r_z1.
+  auto gz_flux = [&](auto LL, auto WR, const Vec<decltype(LL)::v>& ex, const Vec<decltype(LL)::v>& ey,
                      const Vec<decltype(LL)::v>& cb, const Vec<decltype(LL)::v>& ze, unsigned on, const float* zp, int iz,
-                     auto&& ld, Vec<decltype(LL)::v>& gzx, Vec<decltype(LL)::v>& gzy, Vec<decltype(LL)::v>& hx,
-                     Vec<decltype(LL)::v>& hy) {
+                     auto&& ld, Vec<decltype(LL)::v>& gzx, Vec<decltype(LL)::v>& gzy) {
     constexpr int L = decltype(LL)::v;
-    constexpr bool W = decltype(WR)::v != 0, H = decltype(HH)::v != 0;
-    Vec<L> r0 = vzero<L>(), r1 = vzero<L>();
+    constexpr bool W = decltype(WR)::v != 0;
+    gzx = vscale<L>(ze, cb, ex);
+    gzy = vscale<L>(ze, cb, ey);
     if (CP && on) {
       const Vec<L> ce = ld(2);
       const Vec<L> b = vld<L>(zp), c = vld<L>(zp + ZPS), km = vld<L>(zp + 2 * ZPS);
       float* out = AD.aPsiE[par ^ 1][2];
-      r0 = rel_z<L, -1, W>(ld(0), out + iz, on, b, c, km, ce, ex);
-      r1 = rel_z<L, +1, W>(ld(1), out + iz + qz, on, b, c, km, ce, ey);
-      if (H) {
-        vacc<+1>(hy, r0);
-        vacc<+1>(hx, r1);
-      }
-    }
-    gzx = vflux<CP, -1>(ze, vmul(cb, ex), r0);
-    gzy = vflux<CP, +1>(ze, vmul(cb, ey), r1);
-  };
-  // the products of Gzx - Gzx|z+1 and Gzy - Gzy|z+1 of four columns, nx_ and ny_ the fluxes of the column after them
-  auto gz_diff = [&](const Vec<4>& ex, const Vec<4>& ey, const Vec<4>& cb, const Vec<4>& ze, const Vec<4>& gzx,
-                     const Vec<4>& gzy, float nx_, float ny_, Vec<4>& dzx, Vec<4>& dzy) {
-#pragma unroll
-    for (int l = 0; l < 4; ++l) {
-      dzx[l] = __fmaf_rn(ze[l], __fmul_rn(cb[l], ex[l]), -(l < 3 ? gzx[l < 3 ? l + 1 : l] : nx_));
-      dzy[l] = __fmaf_rn(ze[l], __fmul_rn(cb[l], ey[l]), -(l < 3 ? gzy[l < 3 ? l + 1 : l] : ny_));
+      rel_z<L, -1, -1, W>(gzx, ld(0), out + iz, on, b, c, km, ce, ex);
+      rel_z<L, +1, +1, W>(gzy, ld(1), out + iz + qz, on, b, c, km, ce, ey);
     }
   };
-  // G of the x direction, Gxy = xe q_y - r_x0, Gxz = xe q_z + r_x1, and its relations (zero off the slabs)
+  // G of the x direction: Gxy = xe q_y - r_x0, Gxz = xe q_z + r_x1.
   auto gx_flux = [&](auto LL, const Vec<decltype(LL)::v>& ey, const Vec<decltype(LL)::v>& ez,
                      const Vec<decltype(LL)::v>& cb, float xe, bool on, bool write, const float4& c, int ix, auto&& ld,
-                     Vec<decltype(LL)::v>& gxy, Vec<decltype(LL)::v>& gxz, Vec<decltype(LL)::v>& r0,
-                     Vec<decltype(LL)::v>& r1) {
+                     Vec<decltype(LL)::v>& gxy, Vec<decltype(LL)::v>& gxz) {
     constexpr int L = decltype(LL)::v;
-    const Vec<L> s = vsplat<L>(xe);
-    r0 = r1 = vzero<L>();
+    gxy = vscale<L>(xe, cb, ey);
+    gxz = vscale<L>(xe, cb, ez);
     if (CP && on) {
       const Vec<L> ce = ld(2);
       float* out = AD.aPsiE[par ^ 1][0];
-      r0 = rel_xy<L, -1, L == 4>(ld(0), out + ix, c, ce, ey, write);
-      r1 = rel_xy<L, +1, L == 4>(ld(1), out + ix + qx, c, ce, ez, write);
+      rel_xy<L, -1, -1, L == 4>(gxy, ld(0), out + ix, c, ce, ey, write);
+      rel_xy<L, +1, +1, L == 4>(gxz, ld(1), out + ix + qx, c, ce, ez, write);
     }
-    gxy = vflux<CP, -1>(s, vmul(cb, ey), r0);
-    gxz = vflux<CP, +1>(s, vmul(cb, ez), r1);
   };
   // loaders from global memory: psi at p (q stride qs), ce at cell e
   auto glob = [&](auto LL, const float* p, int qs, long long e) {
@@ -392,15 +325,6 @@ __device__ __forceinline__ bool adjv_item(AVSmem<TY, ZQ, CP>& S, const RfxbInst*
   using L1 = IntC<1>;
   using NoW = IntC<0>;
   using Wr = IntC<1>;
-  auto ch_at = [&](long long e) {
-    Vec<4> c;
-    if (ch_arr) c = vld<4>(ch_arr + e);
-    else {
-#pragma unroll
-      for (int l = 0; l < 4; ++l) c[l] = ch0;
-    }
-    return c;
-  };
   // Gzx, Gzy of column z0 + TZ (the one after the tile) at a row's position
   auto gz_after = [&](const float* St, int o, int irow, long long e, float& gx, float& gy) {
     const int k = z0 + TZ;
@@ -409,7 +333,7 @@ __device__ __forceinline__ bool adjv_item(AVSmem<TY, ZQ, CP>& S, const RfxbInst*
     ze[0] = S.zt[0][TZ];
     int off = 0;
     const unsigned m = cpz ? zslab_of<1>(k, ncp, kb, nz, 2 * qz, off) : 0u;
-    gz_flux(L1{}, NoW{}, NoW{}, ex, ey, cb, ze, m, &S.zp[0][TZ], irow + off, glob(L1{}, psEz + irow + off, qz, e), a, b, a, b);
+    gz_flux(L1{}, NoW{}, ex, ey, cb, ze, m, &S.zp[0][TZ], irow + off, glob(L1{}, psEz + irow + off, qz, e), a, b);
     gx = a[0];
     gy = b[0];
   };
@@ -469,8 +393,9 @@ __device__ __forceinline__ bool adjv_item(AVSmem<TY, ZQ, CP>& S, const RfxbInst*
                         (n - P.hist_step0) >= 0 && (n - P.hist_step0) < P.hist_nsteps;
     const unsigned char* emask = P.emask;
 
+    Vec<4> a0[3], cb0;
     const int oh = (r + 1) * TZ + 4 * zq, oc = r * TZ + 4 * zq;   // this thread's place in an H / ca stage
-    Vec<4> rx0 = vzero<4>(), rx1 = vzero<4>(), kxyp = vzero<4>(), kxzp = vzero<4>();   // x relations of phase A, x fluxes K
+    Vec<4> gxy = vzero<4>(), gxz = vzero<4>(), kxyp = vzero<4>(), kxzp = vzero<4>();
     // prefetch of plane p's psi (and ce) into this thread's slots
     float* const slot = &S.ps[0][CP ? tid : 0][0];
     auto sl = [&](int q) { return vld<4>(slot + q * SS); };
@@ -522,6 +447,15 @@ __device__ __forceinline__ bool adjv_item(AVSmem<TY, ZQ, CP>& S, const RfxbInst*
         get(6, psEy + iyn + qy);
       }
     };
+    auto ch_at = [&](long long e) {
+      Vec<4> c;
+      if (ch_arr) c = vld<4>(ch_arr + e);
+      else {
+#pragma unroll
+        for (int l = 0; l < 4; ++l) c[l] = ch0;
+      }
+      return c;
+    };
     // fluxes of column k+4 from the next lane (the last one evaluates them)
     auto z_next = [&](const float* St, const Vec<4>& gzx, const Vec<4>& gzy, int i, float& nx_, float& ny_) {
       nx_ = __shfl_down_sync(0xffffffffu, gzx[0], 1, ZQ);
@@ -533,7 +467,7 @@ __device__ __forceinline__ bool adjv_item(AVSmem<TY, ZQ, CP>& S, const RfxbInst*
     {
       const float* St = &S.e[0][0];
       const float* S1 = &S.e[1][0];
-      Vec<4> a0[3], cb0, dxy, dxz, dzx, dzy, dyx, dyz;
+      Vec<4> pxy = vzero<4>(), pxz = vzero<4>();
       const int im = xa - 1;
       float4 cx;
       int xbase = 0;
@@ -541,44 +475,40 @@ __device__ __forceinline__ bool adjv_item(AVSmem<TY, ZQ, CP>& S, const RfxbInst*
       for (int c = 0; c < 3; ++c) a0[c] = vld<4>(St + o + c * CE);
       cb0 = vld<4>(St + o + CB);
       Vec<4> gzx = vzero<4>(), gzy = vzero<4>();
-      const Vec<4> ze = vld<4>(&S.zt[0][4 * zq]);
       const bool pro = own && xa > 0;
-      Vec<4> hx, hy = vld<4>(&S.ho[0][oh + D::CH]), hz = vld<4>(&S.ho[0][oh + 2 * D::CH]), nxy, nxz, nyx, nyz, px0, px1;
-      float nzx, nzy;
       if (pro) {
         const bool on = xslab(im, cx, xbase);
         gx_flux(L4{}, a0[1], a0[2], cb0, __ldg(xe_tab + im), on, false, cx, xbase + jk,
-                glob(L4{}, psEx + xbase + jk, qx, col + (long long)im * ps), nxy, nxz, px0, px1);
-        if (CP && on) {
-          vacc<+1>(hy, px1);
-          vacc<+1>(hz, px0);
-        }
-        gz_flux(L4{}, NoW{}, Wr{}, a0[0], a0[1], cb0, ze, zon, zp, oz + im * ny * n4,
-                globz(L4{}, psEz + oz + im * ny * n4, qz, col + (long long)im * ps, zon), gzx, gzy, hx, hy);
+                glob(L4{}, psEx + xbase + jk, qx, col + (long long)im * ps), pxy, pxz);
+        gz_flux(L4{}, NoW{}, a0[0], a0[1], cb0, vld<4>(&S.zt[0][4 * zq]), zon, zp, oz + im * ny * n4,
+                globz(L4{}, psEz + oz + im * ny * n4, qz, col + (long long)im * ps, zon), gzx, gzy);
       }
+      float nzx, nzy;
       z_next(St, gzx, gzy, max(im, 0), nzx, nzy);
+      Vec<4> gyx = vzero<4>(), gyz, nyx = vzero<4>(), nyz;
       if (pro) {
-        gz_diff(a0[0], a0[1], cb0, ze, gzx, gzy, nzx, nzy, dzx, dzy);
-        gy_flux(L4{}, vld<4>(St + o + EW), vld<4>(St + o + EW + 2 * CE), vld<4>(St + o + EW + CB), ye1, ynon, cyn,
-                glob(L4{}, psEy + oyn + im * ncp * zs, qy, col + zs + (long long)im * ps), nyx, nyz);
-        gy_diff(L4{}, NoW{}, a0[0], a0[2], cb0, ye, yon, cy, oy + im * ncp * zs,
-                glob(L4{}, psEy + oy + im * ncp * zs, qy, col + (long long)im * ps), nyx, nyz, dyx, dyz, hx, hz);
+        gy_flux(L4{}, NoW{}, a0[0], a0[2], cb0, ye, yon, cy, oy + im * ncp * zs,
+                glob(L4{}, psEy + oy + im * ncp * zs, qy, col + (long long)im * ps), gyx, gyz);
+        gy_flux(L4{}, NoW{}, vld<4>(St + o + EW), vld<4>(St + o + EW + 2 * CE), vld<4>(St + o + EW + CB), ye1, ynon, cyn,
+                oyn + im * ncp * zs, glob(L4{}, psEy + oyn + im * ncp * zs, qy, col + zs + (long long)im * ps), nyx, nyz);
       }
+#pragma unroll
+      for (int c = 0; c < 3; ++c) a0[c] = vld<4>(S1 + o + c * CE);
+      cb0 = vld<4>(S1 + o + CB);
       if (own) {
         xbase = 0;
         const bool on = xslab(xa, cx, xbase);
-        gx_flux(L4{}, vld<4>(S1 + o + CE), vld<4>(S1 + o + 2 * CE), vld<4>(S1 + o + CB), __ldg(xe_tab + xa), on, true, cx,
-                xbase + jk, glob(L4{}, psEx + xbase + jk, qx, col + (long long)xa * ps), nxy, nxz, rx0, rx1);
+        gx_flux(L4{}, a0[1], a0[2], cb0, __ldg(xe_tab + xa), on, true, cx, xbase + jk,
+                glob(L4{}, psEx + xbase + jk, qx, col + (long long)xa * ps), gxy, gxz);
       }
       if (pro) {
         const long long e = col + (long long)im * ps;
-        const Vec<4> ch = ch_at(e), xe = vsplat<4>(__ldg(xe_tab + im));
-        dxy = vfma<-1>(xe, vmul(cb0, a0[1]), nxy);
-        dxz = vfma<-1>(xe, vmul(cb0, a0[2]), nxz);
+        const Vec<4> h1 = vld<4>(&S.ho[0][oh + D::CH]), h2 = vld<4>(&S.ho[0][oh + 2 * D::CH]), ch = ch_at(e);
+        Vec<4> hy, hz;
 #pragma unroll
         for (int l = 0; l < 4; ++l) {
-          hy[l] = curl_t(hy[l], dxz[l], dzx[l]);
-          hz[l] = curl_t(hz[l], dyx[l], dxy[l]);
+          hy[l] = curl_t(h1[l], pxz[l], gxz[l], gzx[l], l < 3 ? gzx[l < 3 ? l + 1 : l] : nzx);
+          hz[l] = curl_t(h2[l], gyx[l], nyx[l], pxy[l], gxy[l]);
         }
         h_cot(pmask, ptail, im, j, k, [&](int l, int c, float g) {
 #pragma unroll
@@ -588,16 +518,22 @@ __device__ __forceinline__ bool adjv_item(AVSmem<TY, ZQ, CP>& S, const RfxbInst*
               else if (c == 2) hz[t] = hz[t] + g;
             }
         });
-        const Vec<4> py = vmul(ch, hy), pz = vmul(ch, hz), xh = vsplat<4>(__ldg(xh_tab + im));
+        const float xh = __ldg(xh_tab + im);
+        Vec<4> py, pz, one;
+#pragma unroll
+        for (int l = 0; l < 4; ++l) {
+          one[l] = 1.f;
+          py[l] = __fmul_rn(ch[l], hy[l]);
+          pz[l] = __fmul_rn(ch[l], hz[l]);
+          kxyp[l] = __fmul_rn(xh, py[l]);
+          kxzp[l] = __fmul_rn(xh, pz[l]);
+        }
         xbase = 0;
         if (CP && xslab(im, cx, xbase)) {
           const float* q = AD.aPsiH[par][0] + xbase + jk;
-          const Vec<4> one = vsplat<4>(1.f);
-          kxyp = vfma<+1>(xh, py, rel_xy<4, +1, false>(vld<4>(q), nullptr, cx, one, py));
-          kxzp = vfma<-1>(xh, pz, rel_xy<4, -1, false>(vld<4>(q + qx), nullptr, cx, one, pz));
-        } else {
-          kxyp = vmul(xh, py);
-          kxzp = vmul(xh, pz);
+          float* u = AD.aPsiH[par ^ 1][0];
+          rel_xy<4, +1, +1, false>(kxyp, vld<4>(q), u, cx, one, py);
+          rel_xy<4, -1, -1, false>(kxzp, vld<4>(q + qx), u, cx, one, pz);
         }
       }
     }
@@ -605,7 +541,7 @@ __device__ __forceinline__ bool adjv_item(AVSmem<TY, ZQ, CP>& S, const RfxbInst*
     if (CP && own) fetch(xa);
     if (CP) cp_async_commit();
     bool bad = false;
-    float xe1_n = __ldg(xe_tab + xa + 1), xh_n = __ldg(xh_tab + xa), xe = __ldg(xe_tab + xa);
+    float xe1_n = __ldg(xe_tab + xa + 1), xh_n = __ldg(xh_tab + xa);
     int sA = 1, sB = 2;
 #pragma unroll 1
     for (int i = xa; i < xb; ++i) {
@@ -623,53 +559,40 @@ __device__ __forceinline__ bool adjv_item(AVSmem<TY, ZQ, CP>& S, const RfxbInst*
       const float* St = &S.e[sA][0];
       const float* S1 = &S.e[sB][0];
       const float* Ho = &S.ho[sH(i)][oh];
-      const float* Sa = St + o;
       // ---- phase A ----
       Vec<4> gzx = vzero<4>(), gzy = vzero<4>();
       const int iz = oz + i * ny * n4;
-      Vec<4> hx, hy, hz;   // H, then p = ch aH1
-      if (own) {
-        hx = vld<4>(Ho);
-        hy = vld<4>(Ho + D::CH);
-        hz = vld<4>(Ho + 2 * D::CH);
-        if (CP && xon) {
-          vacc<+1>(hy, rx1);
-          vacc<+1>(hz, rx0);
-        }
-        gz_flux(L4{}, Wr{}, Wr{}, vld<4>(Sa), vld<4>(Sa + CE), vld<4>(Sa + CB), vld<4>(&S.zt[0][4 * zq]), zon, zp, iz,
-                [&](int q) { return q == 2 ? sl(4) : sl(q); }, gzx, gzy, hx, hy);
-      }
+      if (own)
+        gz_flux(L4{}, Wr{}, a0[0], a0[1], cb0, vld<4>(&S.zt[0][4 * zq]), zon, zp, iz,
+                [&](int q) { return q == 2 ? sl(4) : sl(q); }, gzx, gzy);
       float nzx, nzy;
       z_next(St, gzx, gzy, i, nzx, nzy);
-      Vec<4> kzx = vzero<4>(), kzy = vzero<4>(), rz0 = vzero<4>(), rz1 = vzero<4>();
-      Vec<4> sx, sy, sz;   // what phase B adds to ca aEm before the terms of the row below
+      Vec<4> kyx = vzero<4>(), kyz = vzero<4>(), kzx = vzero<4>(), kzy = vzero<4>(), kxy = vzero<4>(), kxz = vzero<4>();
       if (own) {
-        Vec<4> nyx, nyz, dyx, dyz, nxy, nxz, dzx, dzy;
-        gz_diff(vld<4>(Sa), vld<4>(Sa + CE), vld<4>(Sa + CB), vld<4>(&S.zt[0][4 * zq]), gzx, gzy, nzx, nzy, dzx, dzy);
-        gy_flux(L4{}, vld<4>(St + o + EW), vld<4>(St + o + EW + 2 * CE), vld<4>(St + o + EW + CB), ye1, ynon, cyn,
+        Vec<4> gyx, gyz, nyx, nyz, g1xy, g1xz;
+        gy_flux(L4{}, Wr{}, a0[0], a0[2], cb0, ye, yon, cy, oy + i * ncp * zs,
+                [&](int q) { return q == 2 ? sl(4) : sl(zon ? 5 + q : q); }, gyx, gyz);
+        gy_flux(L4{}, NoW{}, vld<4>(St + o + EW), vld<4>(St + o + EW + 2 * CE), vld<4>(St + o + EW + CB), ye1, ynon, cyn,
+                oyn + i * ncp * zs,
                 [&](int q) {
                   if (q == 2) return vld<4>(P.ce + e + zs);
                   return vld<4>(zon ? psEy + oyn + i * ncp * zs + q * qy : slot + (5 + q) * SS);
                 }, nyx, nyz);
-        gy_diff(L4{}, Wr{}, vld<4>(Sa), vld<4>(Sa + 2 * CE), vld<4>(Sa + CB), ye, yon, cy, oy + i * ncp * zs,
-                [&](int q) { return q == 2 ? sl(4) : sl(zon ? 5 + q : q); }, nyx, nyz, dyx, dyz, hx, hz);
-#pragma unroll
-        for (int l = 0; l < 4; ++l) hx[l] = curl_t(hx[l], dzy[l], dyz[l]);
         gx_flux(L4{}, vld<4>(S1 + o + CE), vld<4>(S1 + o + 2 * CE), vld<4>(S1 + o + CB), xe1, x1on, i + 1 < xb, cx1,
                 xbase1 + jk,
                 [&](int q) {
                   if (q == 2) return vld<4>((zon || yon) ? P.ce + e + ps : slot + 4 * SS);
                   return vld<4>((zon || yon) ? psEx + xbase1 + jk + q * qx : slot + q * SS);
-                }, nxy, nxz, rx0, rx1);
-        {
-          const Vec<4> s = vsplat<4>(xe), cb = vld<4>(Sa + CB);
-          const Vec<4> dxy = vfma<-1>(s, vmul(cb, vld<4>(Sa + CE)), nxy), dxz = vfma<-1>(s, vmul(cb, vld<4>(Sa + 2 * CE)), nxz);
+                }, g1xy, g1xz);
+        Vec<4> hx = vld<4>(Ho), hy = vld<4>(Ho + D::CH), hz = vld<4>(Ho + 2 * D::CH);
 #pragma unroll
-          for (int l = 0; l < 4; ++l) {
-            hy[l] = curl_t(hy[l], dxz[l], dzx[l]);
-            hz[l] = curl_t(hz[l], dyx[l], dxy[l]);
-          }
+        for (int l = 0; l < 4; ++l) {
+          hx[l] = curl_t(hx[l], gzy[l], l < 3 ? gzy[l < 3 ? l + 1 : l] : nzy, gyz[l], nyz[l]);
+          hy[l] = curl_t(hy[l], gxz[l], g1xz[l], gzx[l], l < 3 ? gzx[l < 3 ? l + 1 : l] : nzx);
+          hz[l] = curl_t(hz[l], gyx[l], nyx[l], gxy[l], g1xy[l]);
         }
+        gxy = g1xy;
+        gxz = g1xz;
         if (pmask || ptail)
           h_cot(pmask, ptail, i, j, k, [&](int l, int c, float g) {
 #pragma unroll
@@ -696,9 +619,9 @@ __device__ __forceinline__ bool adjv_item(AVSmem<TY, ZQ, CP>& S, const RfxbInst*
           float al[3][4];
 #pragma unroll
           for (int l = 0; l < 4; ++l) {
-            al[0][l] = Sa[l];
-            al[1][l] = Sa[CE + l];
-            al[2][l] = Sa[2 * CE + l];
+            al[0][l] = a0[0][l];
+            al[1][l] = a0[1][l];
+            al[2][l] = a0[2][l];
           }
 #pragma unroll 1
           for (int l = max(0, P.hb[4] - k); l < min(4, P.hb[5] - k); ++l) {
@@ -710,92 +633,64 @@ __device__ __forceinline__ bool adjv_item(AVSmem<TY, ZQ, CP>& S, const RfxbInst*
             P.grad[c0 + l] += acc;
           }
         }
-        // p = ch aH1 and its fluxes in z
+        // p = ch aH1 and its fluxes
         const Vec<4> ch = ch_at(e), zh = vld<4>(&S.zt[1][4 * zq]);
-        hx = vmul(ch, hx);
-        hy = vmul(ch, hy);
-        hz = vmul(ch, hz);
-        if (CP && zon) {   // (hx <- ey, +1, q0), (hy <- ex, -1, q1)
-          float* u = AD.aPsiH[par ^ 1][2] + iz;
-          const Vec<4> b = vld<4>(zp), c = vld<4>(zp + ZPS), km = vld<4>(zp + 2 * ZPS), one = vsplat<4>(1.f);
-          rz0 = rel_z<4, +1, true>(sl(2), u, zon, b, c, km, one, hx);
-          rz1 = rel_z<4, -1, true>(sl(3), u + qz, zon, b, c, km, one, hy);
-        }
-        kzx = vflux<CP, +1>(zh, hx, rz0);
-        kzy = vflux<CP, -1>(zh, hy, rz1);
-      }
-      const int ks = i & 1;
-      const float zmx = __shfl_up_sync(0xffffffffu, kzx[3], 1, ZQ), zmy = __shfl_up_sync(0xffffffffu, kzy[3], 1, ZQ);
-      if (own) {
-        // their differences, but for the first column of the tile (its neighbour's come from the halo warp)
-        const Vec<4> zh = vld<4>(&S.zt[1][4 * zq]), one = vsplat<4>(1.f);
+        Vec<4> one;
 #pragma unroll
         for (int l = 0; l < 4; ++l) {
-          const bool far = l == 0 && first_q;
-          sy[l] = far ? 0.f : __fmaf_rn(zh[l], hx[l], -(l ? kzx[l ? l - 1 : 0] : zmx));
-          sx[l] = far ? 0.f : __fmaf_rn(zh[l], hy[l], -(l ? kzy[l ? l - 1 : 0] : zmy));
+          one[l] = 1.f;
+          hx[l] = __fmul_rn(ch[l], hx[l]);
+          hy[l] = __fmul_rn(ch[l], hy[l]);
+          hz[l] = __fmul_rn(ch[l], hz[l]);
+          kyx[l] = __fmul_rn(yh, hx[l]);
+          kzx[l] = __fmul_rn(zh[l], hx[l]);
+          kxy[l] = __fmul_rn(xh, hy[l]);
+          kzy[l] = __fmul_rn(zh[l], hy[l]);
+          kyz[l] = __fmul_rn(yh, hz[l]);
+          kxz[l] = __fmul_rn(xh, hz[l]);
         }
-        if (CP && zon) {
-          vacc<+1>(sy, rz0);
-          vacc<-1>(sx, rz1);
-        }
-        // the differences in x
-        const Vec<4> s = vsplat<4>(xh);
-        Vec<4> dz = vfma<-1>(s, hz, kxzp), r0 = vzero<4>(), r1 = vzero<4>();
-        sz = vfma<-1>(s, hy, kxyp);
         if (CP && xon) {   // (hy <- ez, +1, q0), (hz <- ey, -1, q1)
           const float* q = AD.aPsiH[par][0] + xbase + jk;
           float* u = AD.aPsiH[par ^ 1][0] + xbase + jk;
           const bool far = zon || yon;
-          r0 = rel_xy<4, +1, true>(vld<4>(far ? q : slot + 2 * SS), u, cx, one, hy);
-          r1 = rel_xy<4, -1, true>(vld<4>(far ? q + qx : slot + 3 * SS), u + qx, cx, one, hz);
-          vacc<+1>(sz, r0);
-          vacc<-1>(dz, r1);
+          rel_xy<4, +1, +1, true>(kxy, vld<4>(far ? q : slot + 2 * SS), u, cx, one, hy);
+          rel_xy<4, -1, -1, true>(kxz, vld<4>(far ? q + qx : slot + 3 * SS), u + qx, cx, one, hz);
         }
-        kxyp = vflux<CP, +1>(s, hy, r0);
-        kxzp = vflux<CP, -1>(s, hz, r1);
-#pragma unroll
-        for (int l = 0; l < 4; ++l) sy[l] = __fsub_rn(dz[l], sy[l]);
-        // the fluxes in y, to the row above
-        Vec<4> ry0 = vzero<4>(), ry1 = vzero<4>();
         if (CP && yon) {   // (hx <- ez, -1, q0), (hz <- ex, +1, q1)
           const int iy = oy + i * ncp * zs;
           const float* q = AD.aPsiH[par][1] + iy;
           float* u = AD.aPsiH[par ^ 1][1] + iy;
-          ry0 = rel_xy<4, -1, true>(vld<4>(zon ? q : slot + 2 * SS), u, cy, one, hx);
-          ry1 = rel_xy<4, +1, true>(vld<4>(zon ? q + qy : slot + 3 * SS), u + qy, cy, one, hz);
-          vacc<+1>(sz, ry0);
-          vacc<-1>(sx, ry1);
+          rel_xy<4, -1, -1, true>(kyx, vld<4>(zon ? q : slot + 2 * SS), u, cy, one, hx);
+          rel_xy<4, +1, +1, true>(kyz, vld<4>(zon ? q + qy : slot + 3 * SS), u + qy, cy, one, hz);
         }
-        if (r + 1 < TY) {
-          const Vec<4> s = vsplat<4>(yh);
-          vst<4>(&S.k[ks][0][r + 1][4 * zq], vflux<CP, -1>(s, hx, ry0));
-          vst<4>(&S.k[ks][1][r + 1][4 * zq], vflux<CP, +1>(s, hz, ry1));
+        if (CP && zon) {   // (hx <- ey, +1, q0), (hy <- ex, -1, q1)
+          float* u = AD.aPsiH[par ^ 1][2] + iz;
+          const Vec<4> b = vld<4>(zp), c = vld<4>(zp + ZPS), km = vld<4>(zp + 2 * ZPS);
+          rel_z<4, +1, +1, true>(kzx, sl(2), u, zon, b, c, km, one, hx);
+          rel_z<4, -1, -1, true>(kzy, sl(3), u + qz, zon, b, c, km, one, hy);
         }
       }
       if (CP && own && i + 1 < xb) fetch(i + 1);
       if (CP) cp_async_commit();
-      // the cells' own E: its stage is refilled after the barrier
-      Vec<4> a0[3];
-#pragma unroll
-      for (int c = 0; c < 3; ++c) a0[c] = vld<4>(Sa + c * CE);
+      const int ks = i & 1;
+      if (r + 1 < TY) {
+        vst<4>(&S.k[ks][0][r + 1][4 * zq], kyx);
+        vst<4>(&S.k[ks][1][r + 1][4 * zq], kyz);
+      }
       if (bar_or<NT>(bad)) { bad = true; break; }
       bad = !wait(5 + sC(i));
       // ---- phase B ----
+      float zmx = __shfl_up_sync(0xffffffffu, kzx[3], 1, ZQ), zmy = __shfl_up_sync(0xffffffffu, kzy[3], 1, ZQ);
       if (own) {
-        if (first_q) {
-          const float zh0 = S.zt[1][4 * zq];
-          sx[0] = __fadd_rn(sx[0], __fmaf_rn(zh0, hy[0], -S.kc[ks][1][r]));
-          sy[0] = __fsub_rn(sy[0], __fmaf_rn(zh0, hx[0], -S.kc[ks][0][r]));
-        }
+        if (first_q) { zmx = S.kc[ks][0][r]; zmy = S.kc[ks][1][r]; }
         const Vec<4> myx = vld<4>(&S.k[ks][0][r][4 * zq]), myz = vld<4>(&S.k[ks][1][r][4 * zq]);
         const Vec<4> cav = vld<4>(&S.ca[sC(i)][oc]);
         Vec<4> ex, ey, ez;
 #pragma unroll
         for (int l = 0; l < 4; ++l) {
-          ex[l] = __fmaf_rn(cav[l], a0[0][l], __fsub_rn(sx[l], __fmaf_rn(yh, hz[l], -myz[l])));
-          ey[l] = __fmaf_rn(cav[l], a0[1][l], sy[l]);
-          ez[l] = __fmaf_rn(cav[l], a0[2][l], __fsub_rn(__fmaf_rn(yh, hx[l], -myx[l]), sz[l]));
+          ex[l] = curl_t(__fmul_rn(cav[l], a0[0][l]), kzy[l], l ? kzy[l ? l - 1 : 0] : zmy, kyz[l], myz[l]);
+          ey[l] = curl_t(__fmul_rn(cav[l], a0[1][l]), kxz[l], kxzp[l], kzx[l], l ? kzx[l ? l - 1 : 0] : zmx);
+          ez[l] = curl_t(__fmul_rn(cav[l], a0[2][l]), kyx[l], myx[l], kxy[l], kxyp[l]);
         }
         if (n >= 1 && (pmask | smask | (unsigned)ptail | (unsigned)stail)) {
           // over an indexed copy: the E-probe cotangents of y_{n-1}, then the source adjoints
@@ -849,7 +744,11 @@ __device__ __forceinline__ bool adjv_item(AVSmem<TY, ZQ, CP>& S, const RfxbInst*
         vst<4>(Fo + cs + e, ey);
         vst<4>(Fo + 2 * cs + e, ez);
       }
-      xe = xe1;
+      kxyp = kxy;
+      kxzp = kxz;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) a0[c] = vld<4>(S1 + o + c * CE);
+      cb0 = vld<4>(S1 + o + CB);
       sA = sB;
       sB = sB == 2 ? 0 : sB + 1;
     }
@@ -895,25 +794,26 @@ __device__ __forceinline__ bool adjv_item(AVSmem<TY, ZQ, CP>& S, const RfxbInst*
         if (c.y == j && (row ? (c.z >= k && c.z < k + 4) : c.z == k)) pmask |= 1u << q;
       }
     const bool ptail = P.nprb > 32;
-    // G of the x direction (row Gxy, column Gxz) of plane p and its relation
-    auto gx_halo = [&](const float* St, int p, float xe, Vec<4>& gr, Vec<1>& gc, Vec<4>& rr, Vec<1>& rc) {
+    // G of the x direction on plane i: row Gxy, column Gxz
+    Vec<4> gxr = vzero<4>();
+    float gxc = 0.f;
+    auto gx_halo = [&](const float* St, int p, float xe, Vec<4>& gr, float& gc) {
       float4 cx;
       int xbase = 0;
       const bool xs = xslab(p, cx, xbase);
       const long long e = col + (long long)p * ps;
       if (row) {
-        Vec<4> g, d;
+        Vec<4> dummy;
         gx_flux(L4{}, vld<4>(St + o + CE), vld<4>(St + o + 2 * CE), vld<4>(St + o + CB), xe, xs, false, cx, xbase + jk,
-                glob(L4{}, psEx + xbase + jk, qx, e), gr, g, rr, d);
+                glob(L4{}, psEx + xbase + jk, qx, e), gr, dummy);
       } else if (colm) {
         Vec<1> g, d;
         gx_flux(L1{}, vld<1>(St + o + CE), vld<1>(St + o + 2 * CE), vld<1>(St + o + CB), xe, xs, false, cx, xbase + jk,
-                glob(L1{}, psEx + xbase + jk, qx, e), g, gc, d, rc);
+                glob(L1{}, psEx + xbase + jk, qx, e), d, g);
+        gc = g[0];
       }
     };
-    Vec<4> rxr, g0r;
-    Vec<1> rxc, g0c;
-    gx_halo(&S.e[1][0], xa, __ldg(xe_tab + xa), g0r, g0c, rxr, rxc);
+    gx_halo(&S.e[1][0], xa, __ldg(xe_tab + xa), gxr, gxc);
     float hc0 = 0.f, hc1 = 0.f;   // the column's adjoint hx, hy, one plane ahead
     auto load_old = [&](int i) {
       if (!colm) return;
@@ -930,7 +830,7 @@ __device__ __forceinline__ bool adjv_item(AVSmem<TY, ZQ, CP>& S, const RfxbInst*
     last_e = min(xa + 2, xb);
     last_h = min(xa + 1, xb - 1);
     bool bad = false;
-    float xe1_n = __ldg(xe_tab + xa + 1), xe = __ldg(xe_tab + xa);
+    float xe1_n = __ldg(xe_tab + xa + 1);
     int sA = 1, sB = 2;
 #pragma unroll 1
     for (int i = xa; i < xb; ++i) {
@@ -944,21 +844,17 @@ __device__ __forceinline__ bool adjv_item(AVSmem<TY, ZQ, CP>& S, const RfxbInst*
       const float* Ho = &S.ho[sH(i)][0];
       const int ks = i & 1;
       const int irow = orow + i * ny * n4, iz = irow + zoff;
-      Vec<4> nxr, nrr;   // flux and relation of plane i+1
-      Vec<1> nxc, nrc;
-      gx_halo(S1, i + 1, xe1, nxr, nxc, nrr, nrc);
-      const bool xon = in_xslab(i);
+      Vec<4> g1r = vzero<4>();
+      float g1c = 0.f;
+      gx_halo(S1, i + 1, xe1, g1r, g1c);
       if (is_row) {
-        Vec<4> kyx = vzero<4>(), kyz = vzero<4>(), gzx, gzy = vzero<4>(), ex, ez, cb, hx, hz, dz;
+        Vec<4> kyx = vzero<4>(), kyz = vzero<4>(), gzx, gzy = vzero<4>(), ex, ez, cb;
         if (row) {
           ex = vld<4>(St + o);
           ez = vld<4>(St + o + 2 * CE);
           cb = vld<4>(St + o + CB);
-          hx = vld<4>(Ho + 4 * lane);
-          hz = vld<4>(Ho + 2 * D::CH + 4 * lane);
-          if (xon) vacc<+1>(hz, rxr);
-          gz_flux(L4{}, NoW{}, Wr{}, ex, vld<4>(St + o + CE), cb, vld<4>(&S.zt[0][4 * lane]), zon_r, &S.zp[0][4 * lane], iz,
-                  globz(L4{}, psEz + iz, qz, e, zon_r), gzx, gzy, hx, dz);
+          gz_flux(L4{}, NoW{}, ex, vld<4>(St + o + CE), cb, vld<4>(&S.zt[0][4 * lane]), zon_r, &S.zp[0][4 * lane], iz,
+                  globz(L4{}, psEz + iz, qz, e, zon_r), gzx, gzy);
         }
         float nzy = __shfl_down_sync((1u << ZQ) - 1u, gzy[0], 1, ZQ);
         if (row) {
@@ -966,17 +862,15 @@ __device__ __forceinline__ bool adjv_item(AVSmem<TY, ZQ, CP>& S, const RfxbInst*
             float d;
             gz_after(St, o + 4, irow, e + 4, d, nzy);
           }
-          Vec<4> nyx, nyz, dyx, dyz, dzx, dzy;
-          gz_diff(ex, vld<4>(St + o + CE), cb, vld<4>(&S.zt[0][4 * lane]), gzx, gzy, 0.f, nzy, dzx, dzy);
-          gy_flux(L4{}, vld<4>(St + o + EW), vld<4>(St + o + EW + 2 * CE), vld<4>(St + o + EW + CB), ye1, ynon, cyn,
-                  glob(L4{}, psEy + oyn + i * ncp * zs, qy, e + zs), nyx, nyz);
-          gy_diff(L4{}, NoW{}, ex, ez, cb, ye, yon, cy, oy + i * ncp * zs, glob(L4{}, psEy + oy + i * ncp * zs, qy, e), nyx,
-                  nyz, dyx, dyz, hx, hz);
-          const Vec<4> dxr = vfma<-1>(vsplat<4>(xe), vmul(cb, vld<4>(St + o + CE)), nxr);
+          Vec<4> gyx, gyz, nyx, nyz;
+          gy_flux(L4{}, NoW{}, ex, ez, cb, ye, yon, cy, oy + i * ncp * zs, glob(L4{}, psEy + oy + i * ncp * zs, qy, e), gyx, gyz);
+          gy_flux(L4{}, NoW{}, vld<4>(St + o + EW), vld<4>(St + o + EW + 2 * CE), vld<4>(St + o + EW + CB), ye1, ynon, cyn,
+                  oyn + i * ncp * zs, glob(L4{}, psEy + oyn + i * ncp * zs, qy, e + zs), nyx, nyz);
+          Vec<4> hx = vld<4>(Ho + 4 * lane), hz = vld<4>(Ho + 2 * D::CH + 4 * lane);
 #pragma unroll
           for (int l = 0; l < 4; ++l) {
-            hx[l] = curl_t(hx[l], dzy[l], dyz[l]);
-            hz[l] = curl_t(hz[l], dyx[l], dxr[l]);
+            hx[l] = curl_t(hx[l], gzy[l], l < 3 ? gzy[l < 3 ? l + 1 : l] : nzy, gyz[l], nyz[l]);
+            hz[l] = curl_t(hz[l], gyx[l], nyx[l], gxr[l], g1r[l]);
           }
           if (pmask || ptail)
             h_cot(pmask, ptail, i, j, k, [&](int l, int c, float g) {
@@ -987,16 +881,20 @@ __device__ __forceinline__ bool adjv_item(AVSmem<TY, ZQ, CP>& S, const RfxbInst*
                   else if (c == 2) hz[t] = hz[t] + g;
                 }
             });
-          const Vec<4> ch = ch_at(e), s = vsplat<4>(yh), one = vsplat<4>(1.f);
-          hx = vmul(ch, hx);
-          hz = vmul(ch, hz);
+          Vec<4> one;
+#pragma unroll
+          for (int l = 0; l < 4; ++l) {
+            const float ch = ch_arr ? ch_arr[e + l] : ch0;
+            one[l] = 1.f;
+            hx[l] = __fmul_rn(ch, hx[l]);
+            hz[l] = __fmul_rn(ch, hz[l]);
+            kyx[l] = __fmul_rn(yh, hx[l]);
+            kyz[l] = __fmul_rn(yh, hz[l]);
+          }
           if (CP && yon) {
             const float* q = AD.aPsiH[par][1] + oy + i * ncp * zs;
-            kyx = vfma<-1>(s, hx, rel_xy<4, -1, false>(vld<4>(q), nullptr, cy, one, hx));
-            kyz = vfma<+1>(s, hz, rel_xy<4, +1, false>(vld<4>(q + qy), nullptr, cy, one, hz));
-          } else {
-            kyx = vmul(s, hx);
-            kyz = vmul(s, hz);
+            rel_xy<4, -1, -1, false>(kyx, vld<4>(q), nullptr, cy, one, hx);
+            rel_xy<4, +1, +1, false>(kyz, vld<4>(q + qy), nullptr, cy, one, hz);
           }
         }
         vst<4>(&S.k[ks][0][0][4 * lane], kyx);
@@ -1007,43 +905,41 @@ __device__ __forceinline__ bool adjv_item(AVSmem<TY, ZQ, CP>& S, const RfxbInst*
         if (colm) {
           const Vec<1> ex = vld<1>(St + o), ey = vld<1>(St + o + CE), ez = vld<1>(St + o + 2 * CE), cb = vld<1>(St + o + CB);
           // z fluxes of this column and of column z0
-          Vec<1> ze, nzx, nzy, nyx, nyz, dzx, dzy, dyx, dyz, dxz, hz, hx = vsplat<1>(hc0), hy = vsplat<1>(hc1);
-          if (xon) vacc<+1>(hy, rxc);
-          ze[0] = S.zt[0][0];
-          gz_flux(L1{}, NoW{}, NoW{}, vld<1>(St + o + 1), vld<1>(St + o + 1 + CE), vld<1>(St + o + 1 + CB), ze, zon_0, &S.zp[0][0],
-                  irow + zoff0, glob(L1{}, psEz + irow + zoff0, qz, e + 1), nzx, nzy, hx, hy);
+          Vec<1> ze, gzx, gzy, nzx, nzy, gyx, gyz, nyx, nyz;
           ze[0] = ze_c;
-          dzx = vfma<-1>(ze, vmul(cb, ex), nzx);
-          dzy = vfma<-1>(ze, vmul(cb, ey), nzy);
+          gzx = vscale<1>(ze, cb, ex);
+          gzy = vscale<1>(ze, cb, ey);
           if (CP && zon_c) {
-            const Vec<1> ce = vld<1>(P.ce + e);
-            vacc<+1>(hy, rel_xy<1, -1, false>(vld<1>(psEz + iz), nullptr, czc, ce, ex));
-            vacc<+1>(hx, rel_xy<1, +1, false>(vld<1>(psEz + iz + qz), nullptr, czc, ce, ey));
+            Vec<1> ce = vld<1>(P.ce + e);
+            rel_xy<1, -1, -1, false>(gzx, vld<1>(psEz + iz), nullptr, czc, ce, ex);
+            rel_xy<1, +1, +1, false>(gzy, vld<1>(psEz + iz + qz), nullptr, czc, ce, ey);
           }
-          gy_flux(L1{}, vld<1>(St + o + EW), vld<1>(St + o + EW + 2 * CE), vld<1>(St + o + EW + CB), ye1, ynon, cyn,
-                  glob(L1{}, psEy + oyn + i * ncp * zs, qy, e + zs), nyx, nyz);
-          gy_diff(L1{}, NoW{}, ex, ez, cb, ye, yon, cy, oy + i * ncp * zs, glob(L1{}, psEy + oy + i * ncp * zs, qy, e), nyx,
-                  nyz, dyx, dyz, hx, hz);
-          dxz = vfma<-1>(vsplat<1>(xe), vmul(cb, ez), nxc);
-          hx[0] = curl_t(hx[0], dzy[0], dyz[0]);
-          hy[0] = curl_t(hy[0], dxz[0], dzx[0]);
+          ze[0] = S.zt[0][0];
+          gz_flux(L1{}, NoW{}, vld<1>(St + o + 1), vld<1>(St + o + 1 + CE), vld<1>(St + o + 1 + CB), ze, zon_0, &S.zp[0][0],
+                  irow + zoff0, glob(L1{}, psEz + irow + zoff0, qz, e + 1), nzx, nzy);
+          gy_flux(L1{}, NoW{}, ex, ez, cb, ye, yon, cy, oy + i * ncp * zs, glob(L1{}, psEy + oy + i * ncp * zs, qy, e), gyx, gyz);
+          gy_flux(L1{}, NoW{}, vld<1>(St + o + EW), vld<1>(St + o + EW + 2 * CE), vld<1>(St + o + EW + CB), ye1, ynon, cyn,
+                  oyn + i * ncp * zs, glob(L1{}, psEy + oyn + i * ncp * zs, qy, e + zs), nyx, nyz);
+          Vec<1> hx, hy, one;
+          hx[0] = curl_t(hc0, gzy[0], nzy[0], gyz[0], nyz[0]);
+          hy[0] = curl_t(hc1, gxc, g1c, gzx[0], nzx[0]);
           if (pmask || ptail)
             h_cot(pmask, ptail, i, j, k, [&](int l, int c, float g) {
               if (l != 0) return;
               if (c == 0) hx[0] = hx[0] + g;
               else if (c == 1) hy[0] = hy[0] + g;
             });
-          const Vec<1> ch = vsplat<1>(ch_arr ? ch_arr[e] : ch0), zh = vsplat<1>(zh_c), one = vsplat<1>(1.f);
-          hx = vmul(ch, hx);
-          hy = vmul(ch, hy);
+          const float ch = ch_arr ? ch_arr[e] : ch0;
+          one[0] = 1.f;
+          hx[0] = __fmul_rn(ch, hx[0]);
+          hy[0] = __fmul_rn(ch, hy[0]);
           Vec<1> vx, vy;
+          vx[0] = __fmul_rn(zh_c, hx[0]);
+          vy[0] = __fmul_rn(zh_c, hy[0]);
           if (CP && zon_c) {
             const float* q = AD.aPsiH[par][2] + iz;
-            vx = vfma<+1>(zh, hx, rel_xy<1, +1, false>(vld<1>(q), nullptr, czc, one, hx));
-            vy = vfma<-1>(zh, hy, rel_xy<1, -1, false>(vld<1>(q + qz), nullptr, czc, one, hy));
-          } else {
-            vx = vmul(zh, hx);
-            vy = vmul(zh, hy);
+            rel_xy<1, +1, +1, false>(vx, vld<1>(q), nullptr, czc, one, hx);
+            rel_xy<1, -1, -1, false>(vy, vld<1>(q + qz), nullptr, czc, one, hy);
           }
           kzx = vx[0];
           kzy = vy[0];
@@ -1051,9 +947,8 @@ __device__ __forceinline__ bool adjv_item(AVSmem<TY, ZQ, CP>& S, const RfxbInst*
         S.kc[ks][0][lane - ZQ] = kzx;
         S.kc[ks][1][lane - ZQ] = kzy;
       }
-      rxr = nrr;
-      rxc = nrc;
-      xe = xe1;
+      gxr = g1r;
+      gxc = g1c;
       if (i + 1 < xb) load_old(i + 1);
       if (bar_or<NT>(bad)) { bad = true; break; }
       // phase A of plane i is done: its H stage takes plane i+2 and its E stage
